@@ -15,11 +15,10 @@
 //                  N = 64 heads, K = 128 in four steps, accumulator in tensor memory; the raw e4m3 products are
 //                  exact, so the token's scale is applied once, after the sum over K.  Each thread then owns a
 //                  token: relu, times the head weight, summed over the 64 heads in head order.
-//   select kernels: items (order-preserving key of the score, position) are distinct, so the cut is one exact item:
-//                  an 8-pass radix select, compaction of the winners, bitonic sort of 2048 items in shared memory
-//                  (best first, ties by position).  Two levels: a CTA per 16384 positions keeps its best 2048 (a
-//                  sequence of one chunk is finished there), a CTA per longer sequence merges the chunks' candidates.
+//   select kernel: a counting sort by value over a cluster of CTAs per sequence (best first, ties by position), with an
+//                  exact radix select and bitonic sort for score distributions that it does not separate.
 // Every wait is bounded; a failure is recorded in the status word the host entry point reads back.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -35,6 +34,8 @@ namespace syfi {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kHeads = 64;
 constexpr int kDim = 128;
 constexpr int kPage = 64;
@@ -42,7 +43,7 @@ constexpr int kPageRows = 66;                 // 128-byte rows per cache page: 6
 constexpr int kPageBytes = kPageRows * 128;   // 8448
 constexpr int kKeep = SYFI_DSA_TOPK;          // tokens kept per sequence
 constexpr int kTokTile = 128;                 // tokens per MMA: two cache pages
-constexpr int kTilesPerCta = 8;               // a score CTA walks 1024 tokens of one sequence
+constexpr int kMaxTilesPerCta = 8;            // a score CTA walks up to 1024 tokens of one sequence
 constexpr int kScoreThreads = 160;            // four epilogue warps (one tensor-memory lane quarter each) + a producer / MMA warp
 constexpr int kScoreStages = 2;
 constexpr int kScoreSmem = 1024 + kScoreStages * kTokTile * kDim + kHeads * kDim;   // slack + key tiles + query tile
@@ -50,18 +51,26 @@ constexpr int kSelectThreads = 1024;
 constexpr long long kWaitLimit = 1ll << 31;   // SM clocks (about a second)
 constexpr int kStatusScoreTimeout = 201;
 
-// Score kernel: CTA (x, b) scores tokens [1024 x, 1024 x + 1024) of sequence b, 128 at a time, through a two-deep
+// larger float <-> larger key (NaN aside); key 0 is below every score
+__device__ __forceinline__ uint32_t score_key(float s) {
+  const uint32_t u = __float_as_uint(s);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// Score kernel: CTA (x, b) scores the x-th run of tiles_per_cta * 128 tokens of sequence b, 128 at a time, through a two-deep
 // ring of key tiles in shared memory and two accumulators in tensor memory: while the four epilogue warps turn
 // tile i into scores, the tensor core works on tile i + 1 and TMA fetches tile i + 2.
 __global__ void __launch_bounds__(kScoreThreads)
 dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const uint8_t* __restrict__ cache, const float* __restrict__ weights,
                  const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ block_table, int max_pages,
-                 float* __restrict__ scores, int max_ls, int* __restrict__ status) {
-  const int b = blockIdx.y, t_begin = blockIdx.x * kTilesPerCta * kTokTile;
+                 float* __restrict__ scores, int max_ls, int tiles_per_cta, uint2* __restrict__ ranges, int* __restrict__ status) {
+  const int b = blockIdx.y, t_begin = blockIdx.x * tiles_per_cta * kTokTile;
+  pdl_wait();                                  // the selection of the call before reads the scores written here
+  pdl_trigger();
   const int n = min(seq_lens[b], max_ls);
   if (t_begin >= n) return;                    // the whole CTA leaves before any barrier or allocation
-  const int tiles = min(kTilesPerCta, (n - t_begin + kTokTile - 1) / kTokTile);
+  const int tiles = min(tiles_per_cta, (n - t_begin + kTokTile - 1) / kTokTile);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -70,12 +79,13 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __shared__ uint64_t full[kScoreStages], empty[kScoreStages], tfull[kScoreStages], tempty[kScoreStages], qfull;
   __shared__ uint32_t s_tmem;
   __shared__ float s_w[kHeads];
-  __shared__ int s_page[2 * kTilesPerCta];
+  __shared__ int s_page[2 * kMaxTilesPerCta];
   __shared__ volatile int s_abort;
+  __shared__ uint2 s_range[4];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < kHeads) s_w[tid] = weights[b * kHeads + tid];
-  if (tid < 2 * kTilesPerCta)
+  if (tid < 2 * tiles)
     s_page[tid] = (t_begin + tid * kPage < n) ? block_table[b * max_pages + t_begin / kPage + tid] : -1;
   if (tid == 0) {
     for (int i = 0; i < kScoreStages; ++i) {
@@ -137,6 +147,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // ------------------------------------------------------------ epilogue: thread = token lane of the tile
     const int tl = tid;                        // 0..127
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    uint32_t low = 0xffffffffu, high = 0u;     // range of this thread's scores, for the selection's bins
     for (int i = 0; i < tiles; ++i) {
       const int st = i % kScoreStages;
       const uint32_t ph = (i / kScoreStages) & 1u;
@@ -163,11 +174,23 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc = fmaf(s_w[c * 16 + j], fmaxf(__uint_as_float(r[j]) * scale, 0.0f), acc);
       }
-      if (valid) scores[static_cast<size_t>(b) * max_ls + t] = acc;
+      if (valid) {
+        scores[static_cast<size_t>(b) * max_ls + t] = acc;
+        low = min(low, score_key(acc));
+        high = max(high, score_key(acc));
+      }
     }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    if (lane == 0) s_range[warp] = make_uint2(low, high);
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) {
+    uint2 r = s_range[0];
+    for (int w = 1; w < 4; ++w) r = make_uint2(min(r.x, s_range[w].x), max(r.y, s_range[w].y));
+    ranges[static_cast<size_t>(b) * gridDim.x + blockIdx.x] = r;
+  }
   if (warp == 4) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kScoreStages * kHeads);
@@ -175,23 +198,14 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (tid == 0 && s_abort != 0) atomicExch(status, s_abort);
 }
 
-// larger float <-> larger key (NaN aside); key 0 is below every score
-__device__ __forceinline__ uint32_t score_key(float s) {
-  const uint32_t u = __float_as_uint(s);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-constexpr int kSelectChunk = 16 * kSelectThreads;   // 16384 positions per select CTA of the first level
-
-// The best min(2048, n) of n items, best first, left in s_item[0 .. 2047] (zeros behind them).  An item is
+// The best min(2048, n) of n items, best first, left in s_item[0 .. 2047] (zeros behind them); one CTA.  An item is
 // (order-preserving key of the score << 32) | ~position, so items are distinct, "larger" means "better score, then
 // lower position", and the cut is one exact item value: an 8-pass radix select over the 64 bits (one byte per
 // pass, a histogram in shared memory filled through warp-aggregated increments, since most scores of a sequence
 // share their top bytes), a compaction of the items at or above the cut, and a bitonic sort.
-// get(j) returns the calling thread's j-th item (j < per_thread), 0 where it has none; without `sorted` the winners
-// are left in arbitrary order.
+// get(j) returns the calling thread's j-th item (j < per_thread), 0 where it has none.
 template <typename Get>
-__device__ __forceinline__ void select_best(Get get, int per_thread, int k, bool sorted, unsigned long long* s_item,
+__device__ __forceinline__ void select_best(Get get, int per_thread, int k, unsigned long long* s_item,
                                             unsigned long long* s_swap, int* s_hist, int* s_misc) {
   const int tid = threadIdx.x, lane = tid & 31;
   for (int i = tid; i < kKeep; i += kSelectThreads) s_item[i] = 0ull;
@@ -254,129 +268,268 @@ __device__ __forceinline__ void select_best(Get get, int per_thread, int k, bool
     if (win) s_item[base + __popc(winners & ((1u << lane) - 1u))] = it;
   }
   __syncthreads();
-  if (sorted) {
-    // Bitonic sort, descending, two adjacent items per thread in registers.  A compare-exchange at distance d pairs
-    // item i with item i ^ d: d = 1 is inside the thread, d = 2 .. 32 pairs this thread with lane ^ (d / 2) of its
-    // warp (shuffles, no barrier), d >= 64 goes through shared memory (two buffers in turn: one barrier per stage,
-    // 15 stages instead of 66 barriers).  The first of a pair keeps the larger item where the block of `size`
-    // items it lies in is sorted downwards ((i & size) == 0), the smaller one otherwise.
-    unsigned long long e0 = s_item[2 * tid], e1 = s_item[2 * tid + 1];
-    unsigned long long* buf = s_swap;
-    unsigned long long* other = s_item;
-    auto pick = [](unsigned long long a, unsigned long long c, bool keep_max) {
-      return keep_max ? (a > c ? a : c) : (a < c ? a : c);
-    };
-    for (int size = 2; size <= kKeep; size <<= 1) {
-      const bool desc = ((2 * tid) & size) == 0;
-      for (int stride = size >> 1; stride >= 64; stride >>= 1) {
-        buf[2 * tid] = e0;
-        buf[2 * tid + 1] = e1;
-        __syncthreads();
-        const int half = stride >> 1;
-        const int pt = tid ^ half;
-        const bool keep_max = ((tid & half) == 0) == desc;
-        e0 = pick(e0, buf[2 * pt], keep_max);
-        e1 = pick(e1, buf[2 * pt + 1], keep_max);
-        unsigned long long* t = buf; buf = other; other = t;
-      }
-      for (int stride = (size >> 1) < 32 ? (size >> 1) : 32; stride >= 2; stride >>= 1) {
-        const int half = stride >> 1;
-        const bool keep_max = ((tid & half) == 0) == desc;
-        e0 = pick(e0, __shfl_xor_sync(0xffffffffu, e0, half), keep_max);
-        e1 = pick(e1, __shfl_xor_sync(0xffffffffu, e1, half), keep_max);
-      }
-      const unsigned long long hi = e0 > e1 ? e0 : e1, lo = e0 > e1 ? e1 : e0;
-      e0 = desc ? hi : lo;
-      e1 = desc ? lo : hi;
+  // Bitonic sort, descending, two adjacent items per thread in registers.  A compare-exchange at distance d pairs
+  // item i with item i ^ d: d = 1 is inside the thread, d = 2 .. 32 pairs this thread with lane ^ (d / 2) of its
+  // warp (shuffles, no barrier), d >= 64 goes through shared memory (two buffers in turn: one barrier per stage,
+  // 15 stages instead of 66 barriers).  The first of a pair keeps the larger item where the block of `size`
+  // items it lies in is sorted downwards ((i & size) == 0), the smaller one otherwise.
+  unsigned long long e0 = s_item[2 * tid], e1 = s_item[2 * tid + 1];
+  unsigned long long* buf = s_swap;
+  unsigned long long* other = s_item;
+  auto pick = [](unsigned long long a, unsigned long long c, bool keep_max) {
+    return keep_max ? (a > c ? a : c) : (a < c ? a : c);
+  };
+  for (int size = 2; size <= kKeep; size <<= 1) {
+    const bool desc = ((2 * tid) & size) == 0;
+    for (int stride = size >> 1; stride >= 64; stride >>= 1) {
+      buf[2 * tid] = e0;
+      buf[2 * tid + 1] = e1;
+      __syncthreads();
+      const int half = stride >> 1;
+      const int pt = tid ^ half;
+      const bool keep_max = ((tid & half) == 0) == desc;
+      e0 = pick(e0, buf[2 * pt], keep_max);
+      e1 = pick(e1, buf[2 * pt + 1], keep_max);
+      unsigned long long* t = buf; buf = other; other = t;
     }
-    __syncthreads();                             // every reader of either buffer is through
-    s_item[2 * tid] = e0;
-    s_item[2 * tid + 1] = e1;
+    for (int stride = (size >> 1) < 32 ? (size >> 1) : 32; stride >= 2; stride >>= 1) {
+      const int half = stride >> 1;
+      const bool keep_max = ((tid & half) == 0) == desc;
+      e0 = pick(e0, __shfl_xor_sync(0xffffffffu, e0, half), keep_max);
+      e1 = pick(e1, __shfl_xor_sync(0xffffffffu, e1, half), keep_max);
+    }
+    const unsigned long long hi = e0 > e1 ? e0 : e1, lo = e0 > e1 ? e1 : e0;
+    e0 = desc ? hi : lo;
+    e1 = desc ? lo : hi;
   }
+  __syncthreads();                             // every reader of either buffer is through
+  s_item[2 * tid] = e0;
+  s_item[2 * tid + 1] = e1;
   __syncthreads();
 }
 
-__device__ __forceinline__ void write_tokens(const unsigned long long* s_item, int k, const int32_t* table_row,
-                                             int32_t* o) {
-  for (int i = threadIdx.x; i < kKeep; i += kSelectThreads) {
-    int32_t tok = -1;
-    if (i < k) {
-      const int pos = static_cast<int>(~static_cast<uint32_t>(s_item[i] & 0xffffffffull));
-      tok = table_row[pos / kPage] * kPage + pos % kPage;
-    }
-    o[i] = tok;
-  }
+constexpr int kBins = 4096;        // value bins of one sequence: a score's bin is linear in the score
+constexpr int kMaxInBin = 512;     // most items a bin at or above the cut may hold, see dsa_select_kernel
+constexpr int kMaxCluster = 8;     // CTAs that share a sequence
+constexpr int kMaxListed = kKeep + kMaxInBin;
+constexpr int kTablePages = 2048;  // block-table entries kept in shared memory
+constexpr int kSelectSmem = 2 * kMaxListed * 8 + kBins * 4 + kTablePages * 4;
+static_assert(kMaxListed * 8 >= kBins * 4 && kKeep * 8 <= kBins * 4, "aliases of the selection's buffers");
+
+__device__ __forceinline__ float key_score(uint32_t key) {   // inverse of score_key
+  return __uint_as_float((key & 0x80000000u) ? (key ^ 0x80000000u) : ~key);
+}
+// rounding is monotone, so a larger score never has a smaller bin
+__device__ __forceinline__ int score_bin(float s, float lowest, float scale) {
+  return min(kBins - 1, static_cast<int>((s - lowest) * scale));
 }
 
-// First level: CTA (c, b) takes positions [16384 c, 16384 c + 16384) of sequence b, 16 per thread in registers.
-// A sequence of one chunk is finished here; of a longer one, each chunk's best 2048 items go to `cand` (every token
-// of the sequence's best 2048 is among the best 2048 of its chunk).
+// Selection and sort in one pass over the scores: a counting sort by value.  A cluster of CTAs shares a sequence, CTA r
+// takes every gridDim.x-th block of 1024 positions (PER blocks at most, kept in registers; PER = 0: any number, read
+// again in both sweeps).
+//   1. the range of the sequence's scores (the score kernel left one per run of tokens) is cut into 4096 equal bins;
+//   2. histogram of the bins per CTA, summed over the cluster slice by slice (each CTA a share of the bins: distributed
+//      shared memory moves about 16 bytes per clock and CTA, and the first CTA fetching all of it took 3.7 us) into the
+//      first CTA;
+//   3. the first CTA sums the counts from the top: every bin gets the rank of its first item, and the bin in which the
+//      count reaches 2048 is the cut;
+//   4. every item of the cut bin or a higher one goes to the first CTA (the others collect theirs and send them in one
+//      piece: an atomic on a remote cursor per item took 3 us), which groups them by bin, each at its bin's cursor;
+//   5. an item's final rank is its bin's first rank plus the number of larger items in the bin (a handful), so the
+//      2048 best are written best first without a sorting network.
+// The kernel is a chain of short steps between barriers, so what counts is their number: an eight-pass radix select and
+// a 66-stage bitonic sort per 16384 positions, then the same again over the chunks' candidates, took 25 us for three
+// short sequences and 22 + 32 us for 32 sequences of 65536 tokens; this one takes 6 and 12 us.
+// Where the bins do not separate the scores (a bin at or above the cut holds more than kMaxInBin items: ties, or
+// outliers that stretch the range; infinities and NaNs), the first CTA runs that radix select and sort over the whole
+// sequence instead.  Both orders are exact: by score key, then by position.
+template <int PER, bool CLUSTER>
 __global__ void __launch_bounds__(kSelectThreads)
-dsa_select_kernel(const float* __restrict__ scores, int max_ls, const int32_t* __restrict__ seq_lens,
-                  const int32_t* __restrict__ block_table, int max_pages, unsigned long long* __restrict__ cand,
+dsa_select_kernel(const float* __restrict__ scores, const uint2* __restrict__ ranges, int runs, int run_len, int max_ls,
+                  const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ block_table, int max_pages,
                   int32_t* __restrict__ out) {
-  __shared__ unsigned long long s_item[kKeep];
-  __shared__ unsigned long long s_swap[kKeep];   // second buffer of the sort
-  __shared__ int s_hist[256];
-  __shared__ int s_misc[12];
-  const int b = blockIdx.y, c = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ int4 s_dyn[];
+  int4* s_hist4 = s_dyn;                                            // [kBins] counts; later the items that arrive
+  int* s_hist = reinterpret_cast<int*>(s_hist4);
+  unsigned long long* s_in = reinterpret_cast<unsigned long long*>(s_hist4);
+  unsigned long long* s_item = s_in + kMaxListed;                   // [kMaxListed] items grouped by bin
+  int4* s_cursor4 = reinterpret_cast<int4*>(s_item + kMaxListed);   // [kBins] counts of the sequence, then cursors
+  int* s_cursor = reinterpret_cast<int*>(s_cursor4);
+  int* s_table = s_cursor + kBins;                                  // [kTablePages] start of the sequence's block table
+  __shared__ int s_scan[32];
+  __shared__ int s_cut[3];              // cut bin (-1: the bins do not separate the scores), candidate, items at or above it
+  __shared__ int s_own, s_base;         // items this CTA has collected, their place in the first CTA's s_in
+  __shared__ int s_arrived;             // first CTA: items in s_in
+  __shared__ int s_radix[256], s_misc[12];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = CLUSTER ? static_cast<int>(blockIdx.x) : 0;
+  s_hist4[tid] = make_int4(0, 0, 0, 0);
+  if (tid == 0) { s_own = 0; s_arrived = 0; }
+  pdl_wait();
+  pdl_trigger();
   const int n = min(seq_lens[b], max_ls);
-  const int chunks = (n + kSelectChunk - 1) / kSelectChunk;
-  if (c >= max(chunks, 1)) return;
   int32_t* o = out + static_cast<size_t>(b) * kKeep;
-  if (n == 0) {
-    for (int i = tid; i < kKeep; i += kSelectThreads) o[i] = -1;
+  if (n <= 0) {                         // the same for every CTA of the cluster
+    if (rank == 0)
+      for (int i = tid; i < kKeep; i += kSelectThreads) o[i] = -1;
     return;
   }
-  const int begin = c * kSelectChunk, len = min(kSelectChunk, n - begin);
+  // a sequence that fits one CTA's registers is finished by the first CTA, without the cluster's barriers
+  const bool joint = CLUSTER && n > (PER > 0 ? PER : 8) * kSelectThreads;
+  const int ctas = joint ? static_cast<int>(gridDim.x) : 1;
+  if (rank >= ctas) return;
+  const int k = min(kKeep, n);
   const float* sc = scores + static_cast<size_t>(b) * max_ls;
-  unsigned long long mine[16];
+  const int32_t* table = block_table + static_cast<size_t>(b) * max_pages;
+  const int first = rank * kSelectThreads + tid, step = ctas * kSelectThreads;
+  float mine[PER > 0 ? PER : 1];
+  // f(score, position) for each of this thread's positions
+  auto sweep = [&](auto f) {
+    if constexpr (PER > 0) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int i = begin + j * kSelectThreads + tid;
-    mine[j] = (j * kSelectThreads + tid < len)
-                  ? (static_cast<unsigned long long>(score_key(sc[i])) << 32) | (~static_cast<uint32_t>(i))
-                  : 0ull;
-  }
-  const int k = min(kKeep, len);
-  select_best([&](int j) { return mine[j]; }, 16, k, chunks == 1, s_item, s_swap, s_hist, s_misc);
-  if (chunks == 1) {
-    write_tokens(s_item, k, block_table + static_cast<size_t>(b) * max_pages, o);
-  } else {
-    unsigned long long* dst = cand + (static_cast<size_t>(b) * gridDim.x + c) * kKeep;
-    for (int i = tid; i < kKeep; i += kSelectThreads) dst[i] = s_item[i];
-  }
-}
-
-// Second level, sequences of more than one chunk: the best 2048 of the chunks' candidates.
-__global__ void __launch_bounds__(kSelectThreads)
-dsa_merge_kernel(const unsigned long long* __restrict__ cand, int max_chunks, int max_ls,
-                 const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ block_table, int max_pages,
-                 int32_t* __restrict__ out) {
-  __shared__ unsigned long long s_item[kKeep];
-  __shared__ unsigned long long s_swap[kKeep];   // second buffer of the sort
-  __shared__ int s_hist[256];
-  __shared__ int s_misc[12];
-  const int b = blockIdx.x, tid = threadIdx.x;
-  const int n = min(seq_lens[b], max_ls);
-  const int chunks = (n + kSelectChunk - 1) / kSelectChunk;
-  if (chunks <= 1) return;                     // finished by the first level
-  const unsigned long long* src = cand + static_cast<size_t>(b) * max_chunks * kKeep;
-  const int total = chunks * kKeep;
-  const int per_thread = (total + kSelectThreads - 1) / kSelectThreads;
-  if (per_thread <= 16) {   // up to 8 chunks (131072 tokens): the candidates stay in registers over the eight passes
-    unsigned long long mine[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int i = j * kSelectThreads + tid;
-      mine[j] = i < total ? src[i] : 0ull;
+      for (int j = 0; j < PER; ++j)
+        if (first + j * step < n) f(mine[j], first + j * step);
+    } else {
+      for (int i = first; i < n; i += step) f(__ldg(sc + i), i);
     }
-    select_best([&](int j) { return mine[j]; }, 16, kKeep, true, s_item, s_swap, s_hist, s_misc);
-  } else {
-    select_best([&](int j) { const int i = j * kSelectThreads + tid; return i < total ? src[i] : 0ull; }, per_thread,
-                kKeep, true, s_item, s_swap, s_hist, s_misc);
+  };
+  if constexpr (PER > 0) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) mine[j] = first + j * step < n ? __ldg(sc + first + j * step) : 0.0f;
   }
-  write_tokens(s_item, kKeep, block_table + static_cast<size_t>(b) * max_pages, out + static_cast<size_t>(b) * kKeep);
+
+  if (rank == 0)
+    for (int i = tid; i < kTablePages && i * kPage < n; i += kSelectThreads) s_table[i] = table[i];
+
+  // 1. range (every warp for itself: no barrier)
+  uint32_t low = 0xffffffffu, high = 0u;
+  for (int i = lane; i * run_len < n; i += 32) {
+    const uint2 r = ranges[static_cast<size_t>(b) * runs + i];
+    low = min(low, r.x);
+    high = max(high, r.y);
+  }
+  const float lowest = key_score(__reduce_min_sync(0xffffffffu, low));
+  const float range = key_score(__reduce_max_sync(0xffffffffu, high)) - lowest;
+  const float scale = static_cast<float>(kBins - 1) / range;
+  // NaNs and infinities make the range, ties and tiny ranges the scale useless
+  const bool binned = range > 0.0f && range <= 3.0e38f && scale <= 3.0e38f;
+  __syncthreads();
+
+  // 2. histogram
+  if (binned) sweep([&](float s, int) { atomicAdd(&s_hist[score_bin(s, lowest, scale)], 1); });
+  if (joint) {
+    cluster.sync();
+    const int quads = kBins / 4 / ctas;   // cluster sizes are powers of two
+    if (tid < quads) {
+      const int i = rank * quads + tid;
+      int4 r[kMaxCluster];
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c)
+        r[c] = c < ctas ? cluster.map_shared_rank(s_hist4, c)[i] : make_int4(0, 0, 0, 0);
+#pragma unroll
+      for (int c = 1; c < kMaxCluster; ++c) {
+        r[0].x += r[c].x; r[0].y += r[c].y; r[0].z += r[c].z; r[0].w += r[c].w;
+      }
+      cluster.map_shared_rank(s_cursor4, 0)[i] = r[0];
+    }
+    cluster.sync();
+  } else {
+    __syncthreads();
+  }
+
+  // 3. first rank of every bin, and the cut; thread t has bins 4 t .. 4 t + 3 counted from the top
+  if (rank == 0) {
+    static_assert(kBins == 4 * kSelectThreads, "four bins per thread");
+    const int quad = kSelectThreads - 1 - tid;
+    const int4 q = joint ? s_cursor4[quad] : s_hist4[quad];
+    const int h[4] = {q.w, q.z, q.y, q.x}, sum = q.x + q.y + q.z + q.w;
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += up;
+    }
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    int at = __reduce_add_sync(0xffffffffu, lane < warp ? s_scan[lane] : 0) + incl - sum;   // items above this thread's bins
+    bool crowded = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int bin = 4 * quad + 3 - j;
+      s_cursor[bin] = at;
+      crowded |= at < k && h[j] > kMaxInBin;
+      if (at < k && at + h[j] >= k) { s_cut[1] = bin; s_cut[2] = at + h[j]; }
+      at += h[j];
+    }
+    crowded = __syncthreads_or(crowded);
+    if (tid == 0) s_cut[0] = binned && !crowded ? s_cut[1] : -1;
+  }
+  int cut;
+  if (joint) {
+    cluster.sync();
+    cut = cluster.map_shared_rank(s_cut, 0)[0];
+  } else {
+    __syncthreads();
+    cut = s_cut[0];
+  }
+
+  // 4. the items at or above the cut bin, grouped by bin
+  auto item_of = [](float s, int i) {
+    return (static_cast<unsigned long long>(score_key(s)) << 32) | static_cast<uint32_t>(~i);
+  };
+  auto bin_of = [&](unsigned long long it) { return score_bin(key_score(static_cast<uint32_t>(it >> 32)), lowest, scale); };
+  if (cut >= 0) {
+    if (rank == 0) {
+      sweep([&](float s, int i) {
+        const int bin = score_bin(s, lowest, scale);
+        if (bin >= cut) s_item[atomicAdd(&s_cursor[bin], 1)] = item_of(s, i);
+      });
+    } else {
+      sweep([&](float s, int i) {
+        if (score_bin(s, lowest, scale) >= cut) s_item[atomicAdd(&s_own, 1)] = item_of(s, i);
+      });
+      __syncthreads();
+      if (tid == 0 && s_own > 0) s_base = atomicAdd(cluster.map_shared_rank(&s_arrived, 0), s_own);
+      __syncthreads();
+      unsigned long long* in = cluster.map_shared_rank(s_in, 0) + s_base;
+      for (int i = tid; i < s_own; i += kSelectThreads) in[i] = s_item[i];
+    }
+  }
+  if (joint) cluster.sync();     // also keeps the first CTA's shared memory until the others are through with it
+  else __syncthreads();
+  if (rank != 0) return;
+
+  auto token = [&](unsigned long long item) {
+    const int pos = static_cast<int>(~static_cast<uint32_t>(item)), page = pos / kPage;
+    return (page < kTablePages ? s_table[page] : table[page]) * kPage + pos % kPage;
+  };
+  if (cut >= 0) {
+    if (joint) {
+      for (int i = tid; i < s_arrived; i += kSelectThreads) {
+        const unsigned long long it = s_in[i];
+        s_item[atomicAdd(&s_cursor[bin_of(it)], 1)] = it;
+      }
+      __syncthreads();
+    }
+    // 5. a bin's cursor now stands at the first rank of the next lower bin
+    for (int i = tid; i < s_cut[2]; i += kSelectThreads) {
+      const unsigned long long it = s_item[i];
+      const int bin = bin_of(it), end = s_cursor[bin];
+      int at = bin == kBins - 1 ? 0 : s_cursor[bin + 1];
+      int final_rank = at;
+#pragma unroll 4
+      for (; at < end; ++at) final_rank += s_item[at] > it;
+      if (final_rank < k) o[final_rank] = token(it);
+    }
+  } else {
+    select_best([&](int j) {
+      const int i = j * kSelectThreads + tid;
+      return i < n ? item_of(__ldg(sc + i), i) : 0ull;
+    }, (n + kSelectThreads - 1) / kSelectThreads, k, s_item, reinterpret_cast<unsigned long long*>(s_cursor), s_radix, s_misc);
+    for (int i = tid; i < k; i += kSelectThreads) o[i] = token(s_item[i]);
+  }
+  for (int i = k + tid; i < kKeep; i += kSelectThreads) o[i] = -1;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -409,14 +562,60 @@ bool rows128_map(CUtensorMap* m, const void* base, uint64_t rows) {
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// per-device scratch: the scores of every token of every sequence, and a status word
+template <int PER, bool CLUSTER>
+cudaError_t launch_select_as(int ctas, const float* scores, const uint2* ranges, int runs, int run_len,
+                             int max_ls, const int32_t* seq_lens, const int32_t* block_table, int batch, int max_pages,
+                             int32_t* out, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas, batch);
+  cfg.blockDim = dim3(kSelectThreads);
+  cfg.dynamicSmemBytes = kSelectSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ctas;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CLUSTER ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, dsa_select_kernel<PER, CLUSTER>, scores, ranges, runs, run_len, max_ls, seq_lens,
+                            block_table, max_pages, out);
+}
+
+// CTAs per sequence by the table's width and the batch.  8192 positions per CTA (eight per thread in registers) while
+// that gives at most one CTA per SM, else 16384: clusters of eight with two CTAs on every SM do not all find room at
+// once (32 sequences of 65536 tokens: 72 us per call with eight CTAs each, 63 us with four).  Beyond 131072
+// positions the scores are read again (from L2) in each sweep.
+cudaError_t launch_select(const float* scores, const uint2* ranges, int runs, int run_len, int max_ls,
+                          const int32_t* seq_lens, const int32_t* block_table, int batch, int max_pages, int32_t* out,
+                          int num_sms, cudaStream_t st) {
+  auto run = [&](auto* launch, int ctas) {
+    return launch(ctas, scores, ranges, runs, run_len, max_ls, seq_lens, block_table, batch, max_pages, out, st);
+  };
+  auto ctas_for = [&](int positions) {
+    int ctas = 1;
+    while (ctas < kMaxCluster && static_cast<int64_t>(ctas) * positions < max_ls) ctas *= 2;
+    return ctas;
+  };
+  const int c8 = ctas_for(8 * kSelectThreads), c16 = ctas_for(16 * kSelectThreads);
+  if (c8 == 1) return run(launch_select_as<8, false>, 1);
+  if (static_cast<int64_t>(c16) * 16 * kSelectThreads < max_ls) return run(launch_select_as<0, true>, kMaxCluster);
+  if (c8 * 8 * kSelectThreads >= max_ls && static_cast<int64_t>(batch) * c8 <= num_sms) return run(launch_select_as<8, true>, c8);
+  return c16 == 1 ? run(launch_select_as<16, false>, 1) : run(launch_select_as<16, true>, c16);
+}
+
+// per-device scratch: the scores of every token of every sequence with their ranges, and a status word
 struct Scratch {
   float* scores = nullptr;
   size_t floats = 0;
-  unsigned long long* cand = nullptr;   // [batch][chunks][2048] items of the first selection level
-  size_t cand_items = 0;
   int* status = nullptr;
+  // the last few tensor maps: they depend on an address and a row count only, which a serving loop repeats
+  struct Map { const void* base = nullptr; uint64_t rows = 0; CUtensorMap map; };
+  Map maps[8];
+  int next_map = 0;
   bool checked = false;
+  int num_sms = 0;
 };
 std::mutex g_mu;
 Scratch g_scratch[64];
@@ -447,11 +646,14 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   Scratch& s = g_scratch[dev];
   if (!s.checked) {     // once per device: the attribute queries cost more than the kernels
     int major = 0;
-    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess || major != 10)
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess || major != 10 ||
+        cudaDeviceGetAttribute(&s.num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return fail(SYFI_DSA_ERR_CUDA, "this library is built for sm_100a (B200) only");
     s.checked = true;
   }
-  const size_t need = static_cast<size_t>(batch) * max_ls;
+  // scores, and a score range per 128 tokens at most (a multiple of 64 floats before it)
+  const size_t n_scores = static_cast<size_t>(batch) * max_ls;
+  const size_t need = n_scores + 2 * static_cast<size_t>(batch) * ((max_ls + kTokTile - 1) / kTokTile);
   if (need > s.floats) {
     if (cudaDeviceSynchronize() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "device synchronisation failed");
     if (s.scores) cudaFree(s.scores);
@@ -460,43 +662,45 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
     if (cudaMalloc(&s.scores, need * sizeof(float)) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "out of device memory for the scores");
     s.floats = need;
   }
-  {
-    const size_t chunks_all = static_cast<size_t>((max_ls + kSelectChunk - 1) / kSelectChunk);
-    const size_t need_items = chunks_all > 1 ? static_cast<size_t>(batch) * chunks_all * kKeep : 0;
-    if (need_items > s.cand_items) {
-      if (cudaDeviceSynchronize() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "device synchronisation failed");
-      if (s.cand) cudaFree(s.cand);
-      s.cand = nullptr;
-      s.cand_items = 0;
-      if (cudaMalloc(&s.cand, need_items * sizeof(unsigned long long)) != cudaSuccess)
-        return fail(SYFI_DSA_ERR_CUDA, "out of device memory for the selection candidates");
-      s.cand_items = need_items;
-    }
-  }
   if (!s.status) {
     if (cudaMalloc(&s.status, 16) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "out of device memory");
     cudaMemset(s.status, 0, 16);
-    if (cudaFuncSetAttribute(dsa_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScoreSmem) != cudaSuccess)
-      return fail(SYFI_DSA_ERR_CUDA, "cannot raise the shared-memory limit of the score kernel");
+    auto raise = [](auto* kernel, int bytes) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    if (!raise(dsa_score_kernel, kScoreSmem) || !raise(dsa_select_kernel<8, false>, kSelectSmem) ||
+        !raise(dsa_select_kernel<8, true>, kSelectSmem) || !raise(dsa_select_kernel<16, true>, kSelectSmem) ||
+        !raise(dsa_select_kernel<16, false>, kSelectSmem) || !raise(dsa_select_kernel<0, true>, kSelectSmem))
+      return fail(SYFI_DSA_ERR_CUDA, "cannot raise the shared-memory limit of the indexer's kernels");
   }
-  CUtensorMap tm_q, tm_k;
-  if (!rows128_map(&tm_q, q_index_fp8, static_cast<uint64_t>(batch) * kHeads) ||
-      !rows128_map(&tm_k, k_index_cache_fp8, static_cast<uint64_t>(num_pages) * kPageRows))
+  auto map_of = [&s](const void* base, uint64_t rows) -> const CUtensorMap* {
+    for (const Scratch::Map& m : s.maps)
+      if (m.base == base && m.rows == rows) return &m.map;
+    Scratch::Map& m = s.maps[s.next_map];
+    m.base = nullptr;
+    if (!rows128_map(&m.map, base, rows)) return nullptr;
+    m.base = base;
+    m.rows = rows;
+    s.next_map = (s.next_map + 1) % 8;
+    return &m.map;
+  };
+  const CUtensorMap* tm_q = map_of(q_index_fp8, static_cast<uint64_t>(batch) * kHeads);
+  const CUtensorMap* tm_k = map_of(k_index_cache_fp8, static_cast<uint64_t>(num_pages) * kPageRows);
+  if (!tm_q || !tm_k)
     return fail(SYFI_DSA_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-  const int tiles = (max_ls + kTilesPerCta * kTokTile - 1) / (kTilesPerCta * kTokTile);
-  dsa_score_kernel<<<dim3(tiles, batch), kScoreThreads, kScoreSmem, st>>>(
-      tm_q, tm_k, static_cast<const uint8_t*>(k_index_cache_fp8), weights, seq_lens, block_table, max_pages, s.scores,
-      max_ls, s.status);
-  if (cudaGetLastError() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "score kernel launch failed");
-  const int chunks = (max_ls + kSelectChunk - 1) / kSelectChunk;
-  dsa_select_kernel<<<dim3(chunks, batch), kSelectThreads, 0, st>>>(s.scores, max_ls, seq_lens, block_table, max_pages,
-                                                                    s.cand, topk_indices);
-  if (cudaGetLastError() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "select kernel launch failed");
-  if (chunks > 1) {
-    dsa_merge_kernel<<<batch, kSelectThreads, 0, st>>>(s.cand, chunks, max_ls, seq_lens, block_table, max_pages,
-                                                       topk_indices);
-    if (cudaGetLastError() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "merge kernel launch failed");
-  }
+  // Tiles per score CTA: as few as keep a few waves of CTAs (four to five fit an SM) in flight by the table's width;
+  // a short table is a matter of latency, where each tile more in a CTA's chain is about half a microsecond.
+  const int64_t tiles = static_cast<int64_t>(batch) * ((max_ls + kTokTile - 1) / kTokTile);
+  const int per_cta = tiles <= 1024 ? 1 : tiles <= 4096 ? 2 : tiles <= 12288 ? 4 : kMaxTilesPerCta;
+  const int runs = (max_ls + per_cta * kTokTile - 1) / (per_cta * kTokTile);
+  uint2* ranges = reinterpret_cast<uint2*>(s.scores + n_scores);
+  if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, *tm_q, *tm_k,
+                       static_cast<const uint8_t*>(k_index_cache_fp8), weights, seq_lens, block_table, max_pages,
+                       s.scores, max_ls, per_cta, ranges, s.status) != cudaSuccess)
+    return fail(SYFI_DSA_ERR_CUDA, "score kernel launch failed");
+  if (launch_select(s.scores, ranges, runs, per_cta * kTokTile, max_ls, seq_lens, block_table, batch, max_pages,
+                    topk_indices, s.num_sms, st) != cudaSuccess)
+    return fail(SYFI_DSA_ERR_CUDA, "select kernel launch failed");
   return SYFI_DSA_OK;
 }
 

@@ -68,6 +68,64 @@ def test_indexer_ties_and_determinism(pkg):
     assert torch.equal(a[0].cpu(), want)
 
 
+@pytest.mark.parametrize("lens,table_pages,kind", [
+    ([8192, 2049, 2048, 1, 0], 128, "spread"),           # one CTA per sequence: its largest table
+    ([8193, 1024, 5000], 129, "spread"),                 # two CTAs
+    ([16385, 30000, 7], 512, "spread"),                  # four
+    ([65536, 2049], 1024, "spread"),                     # eight, eight positions per thread
+    ([65537, 131072], 2048, "spread"),                   # sixteen positions per thread
+    ([131073, 300], 2049, "spread"),                     # scores read again in every sweep
+    ([3000, 20000, 6000], 512, "zeros"),                 # the cut lies among equal scores: radix select and sort
+    ([140000, 9000], 2200, "zeros"),
+    ([9000, 4000], 256, "outlier"),                      # one score stretches the range
+    ([6000], 94, "nan"),
+])
+def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
+    """Every branch of the selection, with scores that both sides compute without a rounding difference: one head of
+    small integers carries weight 1, so a score is one exact integer times the token's scale.  The reference is a
+    stable descending sort (ties by position); indices must be equal."""
+    g = torch.Generator(device=DEV).manual_seed(len(lens) + table_pages)
+    B, need = len(lens), [(n + 63) // 64 for n in lens]
+    pages = sum(need) + 2
+    q = torch.randint(-4, 5, (B, 64, 128), generator=g, device=DEV).float()
+    keys = torch.randint(-4, 5, (pages, 64, 128), generator=g, device=DEV).float()
+    scale = 0.5 + torch.rand(pages, 64, generator=g, device=DEV)
+    if kind != "spread":
+        scale.fill_(1.0)
+    if kind == "zeros":          # three quarters of the keys repeat one key: scores of zero or one large tie
+        keys[:, 16:] = -q[0, 0]
+    if kind == "outlier":
+        scale[0, 0] = 1e7
+        keys[0, 0] = q[0, 0]
+    if kind == "nan":
+        scale[0, 0] = float("nan")
+    cache = torch.empty(pages, 64 * 132, dtype=torch.uint8, device=DEV)
+    cache[:, :8192] = keys.to(torch.float8_e4m3fn).view(torch.uint8).view(pages, -1)
+    cache[:, 8192:] = scale.view(torch.uint8)
+    w = torch.zeros(B, 64, device=DEV)
+    w[:, 0] = 1.0
+    perm = torch.arange(pages, device=DEV) if kind in ("outlier", "nan") else torch.randperm(pages, generator=g, device=DEV)
+    table = torch.zeros(B, table_pages, dtype=torch.int32, device=DEV)
+    at = 0
+    for b, n in enumerate(need):
+        table[b, :n] = perm[at: at + n].int()
+        at += n
+    sl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    out = torch.full((B, 2048), -7, dtype=torch.int32, device=DEV)
+    pkg.run_dsa_topk_indexer(q.to(torch.float8_e4m3fn), cache.view(torch.int8).view(pages, 64, 1, 132), w, sl, table, out)
+    pkg.dsa_check()
+    for b, n in enumerate(lens):
+        k = min(n, 2048)
+        assert bool((out[b, k:] == -1).all())
+        if n == 0:
+            continue
+        tb = table[b].long()
+        score = torch.relu((keys[tb[: need[b]]] @ q[b, 0]) * scale[tb[: need[b]]]).flatten()[:n]
+        score = torch.nan_to_num(score, nan=0.0)      # relu is a maximum with zero in the kernel: a NaN counts as zero
+        best = torch.sort(score, descending=True, stable=True).indices[:k]
+        assert torch.equal(out[b, :k].long(), tb[best // 64] * 64 + best % 64), (b, n)
+
+
 def test_indexer_argument_validation(pkg):
     from oracle import dsa_oracle
     q, cache, w, sl, table = (t.to(DEV) for t in dsa_oracle.make_inputs([100], seed=1))
