@@ -21,18 +21,19 @@ ABI = {
     "syfi_dsa_topk_indexer": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i64, _i32, _vp, _vp]),
     "syfi_dsa_check": (ctypes.c_int, [_vp]),
 }
-_bound = False
+_bound = None      # the library once this operator's functions are declared
 
 
 def _lib():
     global _bound
+    if _bound:
+        return _bound
     lib = load_library()
-    if not _bound:
-        for name, (res, args) in ABI.items():
-            fn = getattr(lib, name)
-            fn.restype = res
-            fn.argtypes = args
-        _bound = True
+    for name, (res, args) in ABI.items():
+        fn = getattr(lib, name)
+        fn.restype = res
+        fn.argtypes = args
+    _bound = lib
     return lib
 
 
@@ -49,11 +50,8 @@ def _expect(t, name, dtypes, shape, dev):
         raise ValueError(f"{name} must be contiguous")
 
 
-def run_dsa_topk_indexer(q_index_fp8, k_index_cache_fp8, weights, seq_lens, block_table, topk_indices, *,
-                         stream=None):
-    """Writes into ``topk_indices`` int32 [B, 2048] the cache token ids of each sequence's 2048 best-scoring
-    tokens, best first, -1 beyond the sequence's length.  Enqueues on the current CUDA stream, does not
-    synchronise."""
+def _validate(q_index_fp8, k_index_cache_fp8, weights, seq_lens, block_table, topk_indices):
+    """Raises ValueError with what is wrong; (device, batch, pages, max_pages) when nothing is."""
     if not isinstance(q_index_fp8, torch.Tensor) or q_index_fp8.device.type != "cuda":
         raise ValueError("q_index_fp8 must be a CUDA tensor: this library has no CPU path")
     dev = q_index_fp8.device
@@ -70,13 +68,47 @@ def run_dsa_topk_indexer(q_index_fp8, k_index_cache_fp8, weights, seq_lens, bloc
     max_pages = block_table.shape[1]
     _expect(block_table, "block_table", (torch.int32,), (B, max_pages), dev)
     _expect(topk_indices, "topk_indices", (torch.int32,), (B, TOPK), dev)
+    return dev, B, P, max_pages
+
+
+_f8, _u8, _i8, _f32, _int = torch.float8_e4m3fn, torch.uint8, torch.int8, torch.float32, torch.int32
+
+
+def run_dsa_topk_indexer(q_index_fp8, k_index_cache_fp8, weights, seq_lens, block_table, topk_indices, *,
+                         stream=None):
+    """Writes into ``topk_indices`` int32 [B, 2048] the cache token ids of each sequence's 2048 best-scoring
+    tokens, best first, -1 beyond the sequence's length.  Enqueues on the current CUDA stream, does not
+    synchronise."""
+    # One flat expression when everything is as it should be: the kernels take about ten microseconds on a short batch,
+    # the checks one by one as long.  Anything unexpected goes through the checks with a message for each.
+    try:
+        q, k, w, n, t, o = q_index_fp8, k_index_cache_fp8, weights, seq_lens, block_table, topk_indices
+        dev = q.device
+        B, P, max_pages = len(q), len(k), t.shape[1]
+        ok = (dev.type == "cuda" and q.shape == (B, HEADS, DIM) and (q.dtype is _f8 or q.dtype is _u8)
+              and k.shape == (P, PAGE, 1, DIM + 4) and (k.dtype is _i8 or k.dtype is _u8) and k.device == dev
+              and w.shape == (B, HEADS) and w.dtype is _f32 and w.device == dev
+              and n.shape == (B,) and n.dtype is _int and n.device == dev
+              and t.shape == (B, max_pages) and t.dtype is _int and t.device == dev
+              and o.shape == (B, TOPK) and o.dtype is _int and o.device == dev
+              and q.is_contiguous() and k.is_contiguous() and w.is_contiguous() and n.is_contiguous()
+              and t.is_contiguous() and o.is_contiguous())
+    except (AttributeError, TypeError, IndexError):
+        ok = False
+    if not ok:
+        dev, B, P, max_pages = _validate(q_index_fp8, k_index_cache_fp8, weights, seq_lens, block_table, topk_indices)
     if B == 0:
         return topk_indices
-    lib = _lib()
-    with torch.cuda.device(dev):
-        _check(lib.syfi_dsa_topk_indexer(q_index_fp8.data_ptr(), k_index_cache_fp8.data_ptr(), weights.data_ptr(),
-                                         seq_lens.data_ptr(), block_table.data_ptr(), B, P, max_pages,
-                                         topk_indices.data_ptr(), _stream_ptr(stream, dev.index)))
+    fn = _lib().syfi_dsa_topk_indexer
+    args = (q_index_fp8.data_ptr(), k_index_cache_fp8.data_ptr(), weights.data_ptr(), seq_lens.data_ptr(),
+            block_table.data_ptr(), B, P, max_pages, topk_indices.data_ptr(), _stream_ptr(stream, dev.index))
+    if dev.index == torch.cuda.current_device():
+        rc = fn(*args)
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args)
+    if rc:
+        _check(rc)
     return topk_indices
 
 
