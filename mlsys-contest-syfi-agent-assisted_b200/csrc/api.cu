@@ -131,9 +131,25 @@ int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uin
   return SYFI_MOE_OK;
 }
 
+// byte matrices [depth][rows][cols], box [box_depth][box_rows][128], 128-byte swizzle
+int make_map3(CUtensorMap* m, const void* base, uint64_t depth, uint64_t rows, uint64_t cols, uint32_t box_depth,
+              uint32_t box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return fail(SYFI_MOE_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  const cuuint64_t dims[3] = {cols, rows, depth};
+  const cuuint64_t strides[2] = {cols, cols * rows};
+  const cuuint32_t box[3] = {128, box_rows, box_depth};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(SYFI_MOE_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return SYFI_MOE_OK;
+}
+
 void free_workspace(Workspace& ws) {
   void* ptrs[] = {ws.topk_idx, ws.topk_w, ws.local_mask, ws.counts, ws.meta, ws.status, ws.trace, ws.row_token, ws.route_row,
-                  ws.work, ws.a_perm, ws.a_scale, ws.c_hi, ws.c_lo, ws.c_scale, ws.o_rows, ws.ep_ticket, ws.row_out};
+                  ws.parts_done, ws.work, ws.a_perm, ws.a_scale, ws.c_hi, ws.c_scale, ws.o_rows, ws.ep_ticket, ws.row_out};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   const int dev = ws.device;
@@ -177,12 +193,13 @@ int alloc_workspace(Workspace& ws, int64_t max_tokens, int64_t max_rows = 0) {
   CU_TRY(dev_alloc(&ws.trace, 8 * 4096, &total));
   CU_TRY(dev_alloc(&ws.row_token, row_cap, &total));
   CU_TRY(dev_alloc(&ws.route_row, T * kTopK, &total));
+  CU_TRY(dev_alloc(&ws.parts_done, (row_cap / kRowPad + kMaxLocalExperts) * kIBlocks, &total));
   CU_TRY(dev_alloc(&ws.work, kMaxLocalExperts, &total));
   CU_TRY(cudaMemset(ws.work, 0, kMaxLocalExperts * sizeof(ExpertWork)));
   CU_TRY(dev_alloc(&ws.a_perm, row_cap * kHidden, &total));
   CU_TRY(dev_alloc(&ws.a_scale, row_cap * kHBlocks, &total));
-  CU_TRY(dev_alloc(&ws.c_hi, row_cap * kInter, &total));
-  CU_TRY(dev_alloc(&ws.c_lo, row_cap * kInter, &total));
+  CU_TRY(dev_alloc(&ws.c_hi, 2 * row_cap * kInter, &total));
+  ws.c_lo = ws.c_hi + row_cap * kInter;
   CU_TRY(dev_alloc(&ws.c_scale, row_cap * kIBlocks, &total));
   CU_TRY(dev_alloc(&ws.o_rows, row_cap * kHidden, &total));
   CU_TRY(dev_alloc(&ws.ep_ticket, 4, &total));
@@ -289,16 +306,9 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   g1.token_tile = g2.token_tile = token_tile;
   g1.w_packed = packed ? static_cast<const uint8_t*>(w13) : nullptr;
   g2.w_packed = packed ? static_cast<const uint8_t*>(w2) : nullptr;
-  if (packed) {   // the producer fetches packed tiles with untiled copies: no weight tensor map
-    memset(&g1.tm_w, 0, sizeof(g1.tm_w));
-    memset(&g2.tm_w, 0, sizeof(g2.tm_w));
-  } else {
-    if ((rc = make_map(&g1.tm_w, w13, (uint64_t)e_local * 2 * kInter, kHidden, 128))) return rc;
-    if ((rc = make_map(&g2.tm_w, w2, (uint64_t)e_local * kHidden, kInter, 128))) return rc;
-  }
   if (pair) {
-    ctx->p1.tm_w = g1.tm_w;
-    ctx->p2.tm_w = g2.tm_w;
+    if ((rc = make_map(&ctx->p1.tm_w, w13, (uint64_t)e_local * 2 * kInter, kHidden, 128))) return rc;
+    if ((rc = make_map(&ctx->p2.tm_w, w2, (uint64_t)e_local * kHidden, kInter, 128))) return rc;
     if ((rc = make_map(&ctx->p1.tm_b0, ws.a_perm, ws.row_cap, kHidden, 32))) return rc;
     ctx->p1.tm_b1 = ctx->p1.tm_b0;
     if ((rc = make_map(&ctx->p2.tm_b0, ws.c_hi, ws.row_cap, kInter, 32))) return rc;
@@ -308,14 +318,19 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     if ((rc = make_map(&ctx->p2.tm_b0w, ws.c_hi, ws.row_cap, kInter, 128))) return rc;
     if ((rc = make_map(&ctx->p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128))) return rc;
   } else {
-  if ((rc = make_map(&g1.tm_b0, ws.a_perm, ws.row_cap, kHidden, token_tile))) return rc;
-  g1.tm_b1 = g1.tm_b0;
-  if ((rc = make_map(&g1.tm_b0s, ws.a_perm, ws.row_cap, kHidden, 16))) return rc;
-  g1.tm_b1s = g1.tm_b0s;
-  if ((rc = make_map(&g2.tm_b0, ws.c_hi, ws.row_cap, kInter, token_tile))) return rc;
-  if ((rc = make_map(&g2.tm_b1, ws.c_lo, ws.row_cap, kInter, token_tile))) return rc;
-  if ((rc = make_map(&g2.tm_b0s, ws.c_hi, ws.row_cap, kInter, 16))) return rc;
-  if ((rc = make_map(&g2.tm_b1s, ws.c_lo, ws.row_cap, kInter, 16))) return rc;
+  if (!packed) {   // (packed tiles are fetched with untiled copies)
+    const int n_boxes = token_tile == 32 ? 4 : 1;
+    for (int i = 0; i < n_boxes; ++i) {
+      CUtensorMap* m1 = i == 0 ? &g1.tm_w : &g1.tm_part.m[i - 1];
+      CUtensorMap* m2 = i == 0 ? &g2.tm_w : &g2.tm_part.m[i - 1];
+      if ((rc = make_map3(m1, w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128 >> i))) return rc;
+      if ((rc = make_map3(m2, w2, e_local, kHidden, kInter, 1, 128 >> i))) return rc;
+    }
+  }
+  if ((rc = make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, token_tile))) return rc;
+  if ((rc = make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16))) return rc;
+  if ((rc = make_map3(&g2.tm_b, ws.c_hi, 2, ws.row_cap, kInter, 2, token_tile))) return rc;
+  if ((rc = make_map3(&g2.tm_bs, ws.c_hi, 2, ws.row_cap, kInter, 2, 16))) return rc;
   if ((rc = make_scale_map(&g2.tm_sc, ws.c_scale, kIBlocks, ws.row_cap, token_tile))) return rc;
   g1.tm_sc = g2.tm_sc;
   }

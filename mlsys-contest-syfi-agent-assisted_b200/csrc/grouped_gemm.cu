@@ -27,9 +27,9 @@
 //     two accumulators (hi and lo) share the weight tile in shared memory.
 //
 // Pipeline per CTA (persistent over work items): warp 0 = TMA producer (weights with an
-// evict-first L2 policy when streamed once, token-side tiles evict-last), warp 1 = MMA issuer
-// and TMEM owner, then the promotion/epilogue warps (a warp reads one TMEM lane quarter; the
-// tile's columns are split between two or four warps per quarter), and a last warp that keeps
+// evict-first L2 policy when streamed once, token-side tiles evict-last), warp 1 and the last
+// warp = MMA issuers (warp 1 also owns the tensor memory), then the promotion/epilogue warps (a warp reads one TMEM lane quarter; the
+// tile's columns are split between two or four warps per quarter), and one warp that keeps
 // the cross-kernel bookkeeping off everybody else's path (mode 1: publishes finished items to
 // GEMM2; mode 2: waits for GEMM1 to finish an item's expert).  Shared-memory stages form a
 // ring guarded by full/empty mbarriers; the 512 TMEM columns form a ring of 512 / (2 NT)
@@ -39,6 +39,8 @@
 // Every wait is bounded: on expiry the CTA raises an abort flag, all roles leave their
 // loops, TMEM is released and the status word reports the failure to the host.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "moe_internal.h"
 #include "ptx.cuh"
@@ -53,7 +55,6 @@ constexpr int kTmemCols = 512;
 template <int MODE, int NT> struct Cfg {
   static constexpr int kKBlocks = MODE == 1 ? kHBlocks : kIBlocks;              // 56 / 16
   static constexpr int kFeatTiles = MODE == 1 ? kInter / 128 : kHidden / 128;   // 16 / 56
-  static constexpr int kRowsPerExpert = MODE == 1 ? 2 * kInter : kHidden;       // weight rows per expert
   static constexpr int kBTile = NT * 128;                                       // token-side tile bytes
   static constexpr int kStageBytes = MODE == 1 ? 2 * kATile + kBTile : kATile + 2 * kBTile;  // one K block
   // K blocks per pipeline step.  One thread issues every MMA (about 50 cycles each) and every
@@ -74,15 +75,17 @@ template <int MODE, int NT> struct Cfg {
   // promotion chain and of the SwiGLU / requantisation epilogue, which a single warp runs back to back:
   // measured 3-8 % faster per call than 32 columns per warp; 8 columns per warp was no better than 16.
   static constexpr int kColSplit = NT == 128 ? 4 : NT / 16;
-  static constexpr int kThreads = 64 + 128 * kColSplit + 32;   // producer, MMA, epilogue warps, publisher warp
+  static constexpr int kThreads = 64 + 128 * kColSplit + 64;   // producer, MMA, epilogue warps, publisher, second MMA warp
   static constexpr int kSmemBytes = 1024 /* alignment slack */ + kGroups * kGroupBytes +
                                     4 * (kScaleBufs * (kKBlocks * NT + 128) + 4 * NT + 2 * NT) +
                                     8 * (2 * kGroups + 2 * kPairs + 6) +
-                                    kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 32;
+                                    kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 24 + (MODE == 1 ? 256 : 8);
   static_assert(kSmemBytes <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
   static_assert(kKBlocks % kKps == 0 && kSlots % kTKps == 0 && kKps % kTKps == 0,
                 "steps must tile the K blocks and the slots");
   static_assert(kThreads <= 1024, "too many epilogue warps");
+  // The 32-row kernel cuts the items of a thin last round along the features (see Walker).
+  static constexpr bool kSplit = NT == 32;
 };
 
 struct GemmArgs {
@@ -97,10 +100,11 @@ struct GemmArgs {
   uint8_t* c_hi;            // mode 1 outputs
   uint8_t* c_lo;
   float* c_scale;           // [16][row_cap]
-  float* o_rows;            // mode 2 output [row_cap][7168]
+  float* o_rows;            // mode 2 output [row_cap][7168]; mode 1 of the 32-row kernel: accumulators of split items
   int row_cap;
   int e_local;
   int* ready;               // [32] GEMM1 items finished per expert: mode 1 increments, mode 2 waits on it
+  int* parts_done;          // [token tiles][16] mode 1: finished parts of a split item (zeroed by the gather kernel)
   int* status;
   long long* trace;         // [3][4096] timeline of CTA 0 when built with SYFI_TRACE, else unused
   long long* trace_cta;     // [grid][5] per-CTA start/end (globaltimer, clock64) and SM id, SYFI_TRACE only
@@ -123,61 +127,163 @@ struct GemmArgs {
 #define TRACE(role, tag) do { } while (0)
 #endif
 
+// A work item: 128 features (of W13: 128 up and 128 gate rows) of an expert times one token tile, or a part of it:
+// units of eight features [u0, u0 + nu) of the sixteen, nu = 8, 4 or 2.  Rows of a weight tile that a part does not load hold whatever
+// was there before; the accumulator lanes made of them are never read.
 struct Item {
   int expert, ft, row_start, n;
+  int tile;            // token tile, counted over all experts
+  int u0, nu;
 };
 
-// Work item w -> (expert, feature tile, token tile); see ExpertWork for the numbering.  A CTA's items
-// come in increasing order, so each role resumes the search at the expert of its previous item
-// (`e_hint`, start at 0): scanning the table from the front costs over a thousand cycles per item and
-// role once the later experts are reached, which the short GEMM2 items do not hide.
-template <int FT, int NT>
-__device__ __forceinline__ Item decode_item(const ExpertWork* s_work, int e_local, int w, int& e_hint) {
-  Item it{0, 0, 0, 0};
-  for (int e = e_hint; e < e_local; ++e) {
-    const ExpertWork ew = s_work[e];
-    const int base = ew.tile_off * FT;
-    if (w < base + ew.tiles * FT) {
-      const int local = w - base;
-      const int ti = local % ew.tiles;
-      it.expert = e;
-      it.ft = local / ew.tiles;
-      it.row_start = ew.row_off + ti * NT;
-      it.n = min(NT, ew.rows_pad - ti * NT);
-      e_hint = e;
-      return it;
-    }
-  }
-  return it;
+// How a ring entry holds an item's K blocks.
+//   whole items: two K blocks; mode 1 [up tile][gate tile][token tile] each, mode 2 the weight tiles of both first
+//     (adjacent, so pre-packed weights arrive as one copy), then [hi rows][lo rows] each;
+//   parts: four K blocks (two when the token tile has more than 16 rows), weights first, because the ring's depth in K
+//     blocks, not in bytes, is what covers the latency of HBM then.  In mode 1 a part's gate rows follow its up rows in
+//     ONE weight tile (lanes 0 .. F - 1 up, F .. 2 F - 1 gate of one accumulator), which halves the MMAs.
+// Everything here is a compile-time constant: with run-time pitches an MMA took 78 cycles to issue instead of 54, a TMA
+// load 150 instead of 75, and every size lost 5 to 10 %.
+enum Kind { kWhole = 0, kPartFew = 1, kPart = 2 };
+template <int MODE, int NT, Kind KIND>
+struct Layout {
+  using C = Cfg<MODE, NT>;
+  static constexpr int kKps = KIND == kPartFew ? 4 : C::kKps;                      // K blocks per ring entry
+  static constexpr int kWPitch = KIND == kWhole ? (MODE == 1 ? C::kStageBytes : kATile) : (MODE == 1 ? kATile : kATile / 2);
+  static constexpr int kBBase = KIND == kWhole ? (MODE == 1 ? 2 * kATile : kKps * kATile) : kKps * kWPitch;
+  static constexpr int kBRows = (KIND == kPartFew ? 16 : NT) * (MODE == 1 ? 1 : 2);
+  static constexpr int kBPitch = KIND == kWhole && MODE == 1 ? C::kStageBytes : kBRows * 128;
+  static_assert(KIND == kWhole || kBBase + kKps * kBRows * 128 <= C::kGroupBytes, "a part's K blocks fit the ring entry");
+  static_assert(KIND == kWhole || (kKps - 1) * kWPitch + kATile <= C::kGroupBytes, "and the tile an MMA reads lies inside it");
+  static_assert(C::kKBlocks % kKps == 0 && kKps % C::kTKps == 0, "whole steps");
+};
+template <int NT, bool SPLIT>
+__device__ __forceinline__ Kind kind_of(const Item& im) {
+  return !SPLIT || im.nu == 16 ? kWhole : im.n <= 16 ? kPartFew : kPart;
 }
 
-// Schedule: whole work items are dealt round-robin over the persistent grid (CTA b takes items b,
-// b + grid, ...).  With the item numbering above, the CTAs running side by side work on the token
-// tiles of the SAME weight tile, so all but one of them find it in L2.  Splitting items across CTAs
-// at K-step granularity (stream-K, static or with a dynamically claimed tail) was measured and
-// bought nothing at any batch size: the kernels are bound by aggregate HBM bandwidth, not by the
-// last wave, and the hand-off of partial sums costs what the better balance gains.
+// Where a role's walk stands.  A CTA's items come in increasing order, so each role resumes the search at the
+// expert of its previous item: scanning the table from the front costs over a thousand cycles per item and role
+// once the later experts are reached, which the short GEMM2 items do not hide.
+struct Place {
+  int expert = 0;
+};
+
+// Schedule: whole work items are dealt round-robin over the persistent grid (CTA b takes items b, b + grid, ...).
+// With the item numbering (see ExpertWork) the CTAs running side by side work on the token tiles of the SAME weight
+// tile, so all but one of them find it in L2.
+//
+// The last round.  Fewer CTAs with equally many items each, when that costs at most a fifth of the SMs, finish sooner
+// than a last round that keeps only some SMs busy: a single SM draws at most 57 GB/s from HBM, 1.3x its fair share.
+// Failing that, when the last round's items occupy at most half of the SMs (with three active experts, a token or two,
+// GEMM1 has 48 items for 148 SMs), the 32-row kernel cuts each of them along its features into two, four or eight parts,
+// as many as there are SMs for: each of the round's CTAs gets one part.  (Runs of equal length over all CTAs,
+// whatever item boundaries they cross, were slower: a part costs a pass over K of its own, whose MMAs take the same time
+// for 16 features as for 64.)  Cutting along K instead (stream-K) would change the order of the sums; cutting features
+// changes no arithmetic.  In mode 1 the requantisation needs all 128 features: parts store their accumulators and
+// whoever stores an item's last part finishes it; nobody waits.
+struct Schedule {
+  int grid, cta, rounds;        // whole items of this CTA: cta + i * grid, i < rounds
+  int tail_first, parts;        // split last round: its first item, parts per item
+  int n_items;
+  __device__ __forceinline__ int items() const { return n_items; }
+  template <int FT, int NT>
+  __device__ __forceinline__ Item item(const ExpertWork* s_work, int e_local, int i, Place& at) const {
+    Item it{0, 0, 0, 0, 0, 0, 16};
+    int w = cta + i * grid;
+    if (i >= rounds) {
+      w = tail_first + cta / parts;
+      const int part = cta % parts;
+      it.nu = 16 / parts;
+      it.u0 = part * it.nu;
+    }
+    for (int e = at.expert; e < e_local; ++e) {
+      const ExpertWork ew = s_work[e];
+      const int base = ew.tile_off * FT;
+      if (w < base + ew.tiles * FT) {
+        const int local = w - base;
+        const int ti = local % ew.tiles;
+        it.expert = e;
+        it.ft = local / ew.tiles;
+        it.row_start = ew.row_off + ti * NT;
+        it.n = min(NT, ew.rows_pad - ti * NT);
+        it.tile = ew.tile_off + ti;
+        at.expert = e;
+        break;
+      }
+    }
+    return it;
+  }
+};
+
+template <int FT, bool SPLIT>
+__device__ __forceinline__ Schedule make_schedule(int token_tiles) {
+  const int total = token_tiles * FT, cta = static_cast<int>(blockIdx.x);
+  Schedule s{static_cast<int>(gridDim.x), cta, 0, 0, 1, 0};
+  const int full = total / s.grid, rest = total - full * s.grid;
+  const int rounds = full + (rest > 0 ? 1 : 0);
+  const int even = rounds > 0 ? (total + rounds - 1) / rounds : s.grid;   // CTAs needed for `rounds` items each
+  if (even * 5 >= s.grid * 4) {
+    s.grid = even;
+  } else if (SPLIT && rest * 2 <= s.grid) {
+    s.rounds = full;
+    s.tail_first = full * s.grid;
+    s.parts = s.grid / rest >= 8 ? 8 : s.grid / rest >= 4 ? 4 : 2;
+    s.n_items = full + (cta < rest * s.parts ? 1 : 0);
+    return s;
+  }
+  s.rounds = (cta < s.grid && cta < total) ? (total - cta + s.grid - 1) / s.grid : 0;
+  s.n_items = s.rounds;
+  return s;
+}
+
+// Finishes row `row` of a split item from its stored accumulators, the same arithmetic as the epilogue of a whole
+// item; one warp, four features per lane.
+__device__ __forceinline__ void finish_row(const GemmArgs& p, int row, int ft, int lane) {
+  const float* src = p.o_rows + static_cast<size_t>(row) * kHidden + ft * 128 + lane * 4;
+  const float4 u4 = __ldcg(reinterpret_cast<const float4*>(src));
+  const float4 g4 = __ldcg(reinterpret_cast<const float4*>(src + kInter));
+  const float up[4] = {u4.x, u4.y, u4.z, u4.w}, gate[4] = {g4.x, g4.y, g4.z, g4.w};
+  float c[4], amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    c[j] = gate[j] * __fdividef(1.0f, 1.0f + __expf(-gate[j])) * up[j];
+    amax = fmaxf(amax, fabsf(c[j]));
+  }
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  const float sc = fmaxf(amax * (1.0f / 448.0f), 1e-12f), inv = 1.0f / sc;
+  uint32_t hp = 0, lp = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float v0 = c[2 * h], v1 = c[2 * h + 1];
+    const uint16_t hh = cvt_e4m3x2(v0 * inv, v1 * inv);
+    const float2 hb = e4m3x2_to_float2(hh);
+    const float r0 = fmaf(-hb.x, sc, v0), r1 = fmaf(-hb.y, sc, v1);
+    hp |= static_cast<uint32_t>(hh) << (16 * h);
+    lp |= static_cast<uint32_t>(cvt_e4m3x2(r0 * inv * kLoRatio, r1 * inv * kLoRatio)) << (16 * h);
+  }
+  const size_t off = static_cast<size_t>(row) * kInter + ft * 128 + lane * 4;
+  *reinterpret_cast<uint32_t*>(p.c_hi + off) = hp;
+  *reinterpret_cast<uint32_t*>(p.c_lo + off) = lp;
+  if (lane == 0) p.c_scale[static_cast<size_t>(ft) * p.row_cap + row] = sc;
+}
 
 template <int MODE, int NT>
 __global__ void __launch_bounds__((Cfg<MODE, NT>::kThreads), 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
-                    const __grid_constant__ CUtensorMap tm_b1, const __grid_constant__ CUtensorMap tm_b0s,
-                    const __grid_constant__ CUtensorMap tm_b1s, const __grid_constant__ CUtensorMap tm_sc,
-                    const GemmArgs p) {
+grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b,
+                    const __grid_constant__ CUtensorMap tm_bs, const __grid_constant__ CUtensorMap tm_sc,
+                    const __grid_constant__ PartMaps tm_part, const GemmArgs p) {
   using C = Cfg<MODE, NT>;
   constexpr int G = C::kGroups;           // smem ring entries, each kKps K blocks
   constexpr int KPS = C::kKps;
   constexpr int KB = C::kKBlocks;
-  constexpr int STEPS = KB / KPS;
   constexpr int FT = C::kFeatTiles;
   constexpr int TKPS = C::kTKps;
   constexpr int PAIRS = C::kPairs;        // TMEM ring entries, each kTKps accumulator-pair slots
-  constexpr int kBTile = C::kBTile;
-  // Layout of one ring entry (KPS K blocks).  Mode 1: per K block [up tile][gate tile][token tile].
-  // Mode 2: the weight tiles of all K blocks first (adjacent, so pre-packed weights arrive as one
-  // copy), then per K block [hi tile][lo tile].
-  auto w_off = [](int k) { return MODE == 1 ? k * C::kStageBytes : k * kATile; };
-  auto b_off = [](int k) { return MODE == 1 ? k * C::kStageBytes + 2 * kATile : KPS * kATile + k * 2 * kBTile; };
+  // Half of them for each MMA issuer (see mma_role).
+  constexpr int SUB = PAIRS / 2;
+  static_assert(PAIRS % 2 == 0, "two issuers");
+  constexpr bool SPLIT = C::kSplit;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -196,6 +302,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_work + kMaxLocalExperts);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   int* s_meta = reinterpret_cast<int*>(s_tmem + 3);   // [2] token tiles, active experts (copied from p.meta)
+  uint8_t* s_pub = reinterpret_cast<uint8_t*>(s_tmem + 6);   // mode 1, [256] ring: does this CTA publish its i-th item?
+  int* s_last = reinterpret_cast<int*>(s_tmem + 5);   // mode 1: this CTA finished the last part of a split item
   int* s_done = reinterpret_cast<int*>(s_tmem + 2);   // mode 1: epilogue warps that finished storing an item (running total); mode 2: items cleared for loading
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -220,10 +328,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     *s_done = 0;
     fence_barrier_init();
     if (p.w_packed == nullptr) tma_prefetch_desc(&tm_w);
-    tma_prefetch_desc(&tm_b0);
-    if (MODE == 2) tma_prefetch_desc(&tm_b1);
-    tma_prefetch_desc(&tm_b0s);
-    if (MODE == 2) tma_prefetch_desc(&tm_b1s);
+    tma_prefetch_desc(&tm_b);
+    tma_prefetch_desc(&tm_bs);
     if (MODE == 2) tma_prefetch_desc(&tm_sc);
   }
   if (warp == 1) {
@@ -237,7 +343,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // of GEMM2 overlap.  This cannot deadlock: a GEMM2 CTA only exists once every GEMM1 CTA has started
   // (that is when GEMM1 triggers its dependents), and GEMM1 CTAs wait for nothing.  The row tables and
   // counters GEMM2 reads here were complete before GEMM1 passed its own wait.
-  if (MODE == 1) pdl_wait();
+  // The 32-row GEMM1 also starts on its weights before the kernel in front of it is done: that kernel, the gather,
+  // lets this one start only after its own wait for the row lists, so the work table is complete here; only the
+  // gathered rows and their scales are waited for (by the producer and the epilogue warps).
+  if (MODE == 1 && !SPLIT) pdl_wait();
   pdl_trigger();
   // the work table and the two counters every role needs, fetched in one round trip
   if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxLocalExperts) {
@@ -251,20 +360,72 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
-  const int total = s_meta[0] * FT;                 // work items
-  // Effective grid: the launch always has one CTA per SM, but when the items do not fill the last
-  // round, fewer CTAs with equally many items each finish sooner than a last round that keeps only a
-  // handful of SMs busy (a single SM cannot pull more than about 1.4x its fair share of HBM).  Only
-  // taken when it costs at most a fifth of the SMs; the rest of the CTAs exit at once.
-  int eff_grid = static_cast<int>(gridDim.x);
-  {
-    const int rounds = (total + eff_grid - 1) / eff_grid;
-    const int even = rounds > 0 ? (total + rounds - 1) / rounds : eff_grid;   // CTAs needed for `rounds` each
-    if (even * 5 >= eff_grid * 4) eff_grid = even;
-  }
-  const int my_items = (static_cast<int>(blockIdx.x) < eff_grid && static_cast<int>(blockIdx.x) < total)
-                           ? (total - blockIdx.x + eff_grid - 1) / eff_grid : 0;
-  auto item_of = [&](int i) { return static_cast<int>(blockIdx.x) + i * eff_grid; };   // this CTA's i-th item
+  const Schedule sched = make_schedule<FT, SPLIT>(s_meta[0]);
+  const int my_items = sched.items();
+
+  // MMA issue, one thread of each of two warps: one has the even ring entries, one the odd ones (fixed, so that either
+  // sees every phase of its barriers: a parity wait for a phase whose predecessor is not over returns at once).  With the weights as the M operand an MMA takes
+  // 70 to 80 cycles however few columns it has (its 128 rows x 32 bytes come out of shared memory), the issuing thread
+  // is tied up while its MMAs execute and then pays the commits and the next waits (300 to 400 cycles per entry): with
+  // one issuer the tensor core idles during those, and the sizes where the kernels follow each other closely lost 1 to 5 % (T = 1024: 276 against 263 us per call).
+  auto mma_role = [&](const uint32_t par) {
+    uint32_t g = 0, ph = 0, sub = 0, pph = 0;  // smem ring entry / phase, this issuer's TMEM entry / phase
+    Place at;
+    bool alive = true;
+    // one ring entry's MMAs (Layout L)
+    auto issue = [&](auto layout, uint32_t idesc) {
+      using L = decltype(layout);
+      const uint32_t gb = smem_u32(smem + g * C::kGroupBytes);
+#pragma unroll
+      for (int tk = 0; tk < L::kKps / TKPS; ++tk) {
+        const uint32_t pr = par * SUB + sub;
+        if (!mbar_wait_bounded(&tempty[pr], pph ^ 1u, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int k2 = 0; k2 < TKPS; ++k2) {
+          const int k = tk * TKPS + k2;
+          const uint32_t d0 = tmem_base + (pr * TKPS + k2) * (2 * NT);
+          const uint64_t a0 = umma_smem_desc_sw128(gb + k * L::kWPitch);
+          const uint64_t b0 = umma_smem_desc_sw128(gb + L::kBBase + k * L::kBPitch);   // mode 2: hi rows, then lo rows
+          if constexpr (MODE == 1 && std::is_same<L, Layout<MODE, NT, kWhole>>::value) {
+            const uint64_t a1 = umma_smem_desc_sw128(gb + k * L::kWPitch + kATile);
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) {
+              // 32 bytes of K per MMA: +2 in the 16-byte-unit address field
+              umma_f8(d0, a0 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+              umma_f8(d0 + NT, a1 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+            }
+          } else {
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) umma_f8(d0, a0 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+          }
+        }
+        if (tk == L::kKps / TKPS - 1) umma_commit(&empty[g]);
+        umma_commit(&tfull[pr]);
+        if (++sub == SUB) { sub = 0; pph ^= 1u; }
+      }
+      return true;
+    };
+    for (int i = 0; i < my_items && alive; ++i) {
+      const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+      // Mode 2 issues ONE MMA of twice the loaded rows per 32 bytes of K over the adjacent hi and lo rows
+      // (the columns past the tile's n rows hold other rows' data and are never read back)
+      // instead of one per term; mode 1 needs two because up and gate are different A tiles.
+      const uint32_t idesc = umma_idesc_e4m3_m128(MODE == 1 ? static_cast<uint32_t>(im.n) : im.n <= 16 ? 32u : 2u * NT);
+      const Kind kind = kind_of<NT, SPLIT>(im);
+      const int steps = kind == kPartFew ? KB / Layout<MODE, NT, SPLIT ? kPartFew : kWhole>::kKps : KB / KPS;
+      for (int step = 0; step < steps; ++step) {
+        if ((g & 1u) == par) {
+          if (!mbar_wait_bounded(&full[g], ph, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
+          TRACE(1, step);
+          if (!SPLIT || kind == kWhole) alive = issue(Layout<MODE, NT, kWhole>{}, idesc);
+          else if constexpr (SPLIT) alive = kind == kPartFew ? issue(Layout<MODE, NT, kPartFew>{}, idesc) : issue(Layout<MODE, NT, kPart>{}, idesc);
+          if (!alive) break;
+        }
+        if (++g == G) { g = 0; ph ^= 1u; }
+      }
+    }
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one thread)
@@ -275,18 +436,74 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const uint64_t pol_b = l2_policy_evict_last();
       uint32_t it = 0, g = 0, ph = 0;      // step counter, ring entry, its phase
       uint32_t n_items = 0;                // items started (mode 2: selects the scale buffer)
-      int e_hint = 0;
+      Place at;
       bool alive = true;
       for (int i = 0; i < my_items && alive; ++i) {
-        const Item im = decode_item<FT, NT>(s_work, p.e_local, item_of(i), e_hint);
-        const int wrow = im.expert * C::kRowsPerExpert + im.ft * 128;
+        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+        const Kind kind = kind_of<NT, SPLIT>(im);
         // Tiles of at most 16 rows use the 16-row box: the token-side tiles come from L2 through the
         // same SM port as the weights, so every byte not fetched is bandwidth for the weight stream.
-        const bool small = im.n <= 16;
-        const CUtensorMap* mb0 = small ? &tm_b0s : &tm_b0;
-        const CUtensorMap* mb1 = small ? &tm_b1s : &tm_b1;
-        const uint32_t b_bytes = small ? 16 * 128 : kBTile;
-        const uint32_t group_tx = KPS * (MODE == 1 ? 2 * kATile + b_bytes : kATile + 2 * b_bytes);
+        const bool few = im.n <= 16;
+        const CUtensorMap* mb = few ? &tm_bs : &tm_b;
+        const CUtensorMap* mw = !SPLIT || im.nu == 16 ? &tm_w : im.nu == 8 ? &tm_part.m[0] : im.nu == 4 ? &tm_part.m[1] : &tm_part.m[2];
+        const uint32_t w_bytes = static_cast<uint32_t>(im.nu) * 1024;
+        const int wrow = im.ft * 128 + im.u0 * 8;
+        const int steps = kind == kPartFew ? KB / Layout<MODE, NT, SPLIT ? kPartFew : kWhole>::kKps : KB / KPS;
+        // arms ring entry g and loads the weight rows of a step into it (mode 1: up and gate rows in one box)
+        auto load_w = [&](auto layout, int step) {
+          using L = decltype(layout);
+          constexpr int kKps = L::kKps;
+          mbar_arrive_expect_tx(&full[g], kKps * ((MODE == 1 ? 2 : 1) * w_bytes + (few ? 16u : NT) * (MODE == 1 ? 128u : 256u)));
+          uint8_t* st0 = smem + g * C::kGroupBytes;
+          const int kb0 = step * kKps;
+          if (p.w_packed != nullptr) {
+            constexpr int kPacked = (MODE == 1 ? 2 : 1) * kATile;   // packed bytes of a K block
+            const uint8_t* src = p.w_packed + (static_cast<size_t>(im.expert * FT + im.ft) * KB + kb0) * kPacked + im.u0 * 1024;
+            if constexpr (!std::is_same<L, Layout<MODE, NT, kWhole>>::value) {   // a run of 8-row groups is contiguous
+#pragma unroll
+              for (int k = 0; k < kKps; ++k) {
+                bulk_load(st0 + k * L::kWPitch, src + static_cast<size_t>(k) * kPacked, w_bytes, &full[g], pol_w);
+                if (MODE == 1)
+                  bulk_load(st0 + k * L::kWPitch + w_bytes, src + static_cast<size_t>(k) * kPacked + kATile, w_bytes, &full[g], pol_w);
+              }
+            } else if (MODE == 1) {     // 32 KB per K block: up tile, gate tile
+#pragma unroll
+              for (int k = 0; k < kKps; ++k)
+                bulk_load(st0 + k * L::kWPitch, src + static_cast<size_t>(k) * kPacked, kPacked, &full[g], pol_w);
+            } else {                    // the K blocks of a step are adjacent: one copy
+              bulk_load(st0, src, kKps * kATile, &full[g], pol_w);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < kKps; ++k)
+              tma_load_3d(st0 + k * L::kWPitch, mw, &full[g], (kb0 + k) * 128, wrow, MODE == 1 ? 2 * im.expert : im.expert, pol_w);
+          }
+        };
+        // the token rows of a step (mode 2: hi and lo rows in one box)
+        auto load_b = [&](auto layout, int step, uint32_t entry) {
+          using L = decltype(layout);
+          uint8_t* st0 = smem + entry * C::kGroupBytes + L::kBBase;
+#pragma unroll
+          for (int k = 0; k < L::kKps; ++k)
+            tma_load_3d(st0 + k * L::kBPitch, mb, &full[entry], (step * L::kKps + k) * 128, im.row_start, 0, pol_b);
+        };
+        auto pick = [&](auto f) {       // f(layout of this item)
+          if constexpr (SPLIT) {
+            if (kind == kPartFew) return f(Layout<MODE, NT, kPartFew>{});
+            if (kind == kPart) return f(Layout<MODE, NT, kPart>{});
+          }
+          return f(Layout<MODE, NT, kWhole>{});
+        };
+        int ahead = 0;                  // steps of this item whose weights are already on their way
+        if (SPLIT && i == 0) {
+          // the ring's first fill needs the weights only: requested before what the token side waits for
+          for (; ahead < G && ahead < steps; ++ahead) {
+            pick([&](auto layout) { load_w(layout, ahead); });
+            ++it;
+            if (++g == G) { g = 0; ph ^= 1u; }
+          }
+          if (MODE == 1) pdl_wait();    // the gathered rows
+        }
         if (MODE == 2) {
           // This item's expert must have left GEMM1 before its rows and scales are read; the helper
           // warp checks that (see there) and counts cleared items in shared memory, so the producer
@@ -311,43 +528,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
                     KB * 4, &sfull[sb], pol_b);
           ++n_items;
         }
-        for (int step = 0; step < STEPS; ++step) {
-          if (!mbar_wait_bounded(&empty[g], ph ^ 1u, s_abort, kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
-          TRACE(0, step);
-          mbar_arrive_expect_tx(&full[g], group_tx);
-          // The boxes that continue each other along K (same rows, next 128 bytes) are issued back to
-          // back: L2 serves a row's 256 contiguous bytes far faster than two separate 128-byte visits.
-          uint8_t* st0 = smem + g * C::kGroupBytes;
-          const int x0 = step * KPS * 128;
-          if (p.w_packed != nullptr) {
-            if (MODE == 1) {            // 32 KB per K block: up tile, gate tile
-              const uint8_t* src = p.w_packed + (static_cast<size_t>(im.expert * FT + im.ft) * KB + step * KPS) * (2 * kATile);
-#pragma unroll
-              for (int k = 0; k < KPS; ++k)
-                bulk_load(st0 + w_off(k), src + static_cast<size_t>(k) * 2 * kATile, 2 * kATile, &full[g], pol_w);
-            } else {                    // the K blocks of a step are adjacent: one copy
-              const uint8_t* src = p.w_packed + (static_cast<size_t>(im.expert * FT + im.ft) * KB + step * KPS) * kATile;
-              bulk_load(st0, src, KPS * kATile, &full[g], pol_w);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < KPS; ++k) tma_load_2d(st0 + w_off(k), &tm_w, &full[g], x0 + k * 128, wrow, pol_w);
-            if (MODE == 1) {
-#pragma unroll
-              for (int k = 0; k < KPS; ++k)
-                tma_load_2d(st0 + w_off(k) + kATile, &tm_w, &full[g], x0 + k * 128, wrow + kInter, pol_w);
-            }
+        pick([&](auto layout) {
+          for (int step = 0; step < ahead; ++step) load_b(layout, step, step);   // entry of a first fill = its step
+          for (int step = ahead; step < steps; ++step) {
+            if (!mbar_wait_bounded(&empty[g], ph ^ 1u, s_abort, kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
+            TRACE(0, step);
+            load_w(layout, step);
+            TRACE(0, 300 + step);
+            load_b(layout, step, g);
+            TRACE(0, 400 + step);
+            ++it;
+            if (++g == G) { g = 0; ph ^= 1u; }
           }
-#pragma unroll
-          for (int k = 0; k < KPS; ++k) tma_load_2d(st0 + b_off(k), mb0, &full[g], x0 + k * 128, im.row_start, pol_b);
-          if (MODE == 2) {
-#pragma unroll
-            for (int k = 0; k < KPS; ++k)
-              tma_load_2d(st0 + b_off(k) + kBTile, mb1, &full[g], x0 + k * 128, im.row_start, pol_b);
-          }
-          ++it;
-          if (++g == G) { g = 0; ph ^= 1u; }
-        }
+        });
       }
       // drain: every ring entry this thread armed must have landed before the CTA may exit
       const uint32_t first = it > static_cast<uint32_t>(G) ? it - G : 0;
@@ -356,55 +549,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    // --------------------------------------------------------------- MMA issuer (one thread)
-    if (lane == 0) {
-      uint32_t g = 0, ph = 0, pr = 0, pph = 0;   // smem ring entry / phase, TMEM ring entry / phase
-      int e_hint = 0;
-      bool alive = true;
-      for (int i = 0; i < my_items && alive; ++i) {
-        const Item im = decode_item<FT, NT>(s_work, p.e_local, item_of(i), e_hint);
-        // Mode 2 issues ONE MMA of N = 2 NT per 32 bytes of K over the adjacent hi and lo tiles
-        // (the columns past the tile's n rows hold other rows' data and are never read back)
-        // instead of one per term; mode 1 needs two because up and gate are different A tiles.
-        const uint32_t idesc = umma_idesc_e4m3_m128(MODE == 1 ? static_cast<uint32_t>(im.n) : 2u * NT);
-        for (int step = 0; step < STEPS; ++step) {
-          if (!mbar_wait_bounded(&full[g], ph, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
-          TRACE(1, step);
-#pragma unroll
-          for (int tk = 0; tk < KPS / TKPS && alive; ++tk) {
-            if (!mbar_wait_bounded(&tempty[pr], pph ^ 1u, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
-            tc_fence_after();
-#pragma unroll
-            for (int k2 = 0; k2 < TKPS; ++k2) {
-              const int k = tk * TKPS + k2;
-              const uint32_t gb = smem_u32(smem + g * C::kGroupBytes);
-              const uint32_t d0 = tmem_base + (pr * TKPS + k2) * (2 * NT);
-              if (MODE == 1) {
-                const uint64_t a0 = umma_smem_desc_sw128(gb + w_off(k));
-                const uint64_t a1 = umma_smem_desc_sw128(gb + w_off(k) + kATile);
-                const uint64_t b0 = umma_smem_desc_sw128(gb + b_off(k));
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                  // 32 bytes of K per MMA: +2 in the 16-byte-unit address field
-                  umma_f8(d0, a0 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-                  umma_f8(d0 + NT, a1 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-                }
-              } else {
-                const uint64_t a0 = umma_smem_desc_sw128(gb + w_off(k));
-                const uint64_t b0 = umma_smem_desc_sw128(gb + b_off(k));   // hi rows, then lo rows
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f8(d0, a0 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-              }
-            }
-            if (tk == KPS / TKPS - 1) umma_commit(&empty[g]);
-            umma_commit(&tfull[pr]);
-            if (++pr == PAIRS) { pr = 0; pph ^= 1u; }
-          }
-          if (!alive) break;
-          if (++g == G) { g = 0; ph ^= 1u; }
-        }
-      }
-    }
+    // --------------------------------------------------------------- MMA issuer of the even ring entries
+    if (lane == 0) mma_role(0);
+    __syncwarp();
+  } else if (warp == 3 + 4 * C::kColSplit) {
+    // --------------------------------------------------------------- MMA issuer of the odd ring entries
+    if (lane == 0) mma_role(1);
     __syncwarp();
   } else if (warp == 2 + 4 * C::kColSplit) {
     // ------------------------------------------------ publisher (mode 1, one thread)
@@ -428,9 +578,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     // are executed by the publishing / acquiring lanes, not by the threads that store or that issue the
     // loads; the back-to-back bit-identity test exercises exactly this hand-off.
     if (MODE == 1 && lane == 0) {
-      int done_target = 0, e_hint = 0;
+      int done_target = 0;
+      Place at;
       for (int i = 0; i < my_items; ++i) {
-        const Item im = decode_item<FT, NT>(s_work, p.e_local, item_of(i), e_hint);
+        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
         done_target += 4 * C::kColSplit;
         const long long t0 = clock64();
         bool seen = true;
@@ -439,6 +590,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           __nanosleep(200);
         }
         if (!seen || *s_abort != 0) break;          // a failed item is never published
+        if (SPLIT && *reinterpret_cast<volatile uint8_t*>(s_pub + (i & 255)) == 0) continue;   // another CTA has the item's last part
         __threadfence();
         fence_proxy_async_all();
         red_release_gpu_add(p.ready + im.expert, 1);
@@ -449,9 +601,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     // expert.  The acquire load and the proxy fence (generic-proxy stores of GEMM1 before async-proxy
     // loads of this kernel) run here; the producer only reads the count of cleared items (s_done).
     if (MODE == 2 && lane == 0) {
-      int cleared = 0, ready_expert = -1, e_hint = 0;
+      int cleared = 0, ready_expert = -1;
+      Place at;
       for (int i = 0; i < my_items; ++i) {
-        const Item im = decode_item<FT, NT>(s_work, p.e_local, item_of(i), e_hint);
+        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
         if (im.expert != ready_expert) {
           const int need = (kInter / 128) * s_work[im.expert].tiles;
           const long long t0 = clock64();
@@ -483,18 +636,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     const int c0 = ((warp - 2) >> 2) * CN;  // first column of this thread's share
     const int et = threadIdx.x - 64;        // 0..kEpi-1 among the epilogue threads
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    uint32_t pr = 0, pph = 0;               // TMEM ring entry and its phase
+    uint32_t g = 0;                         // smem ring entry, which tells the issuer
+    uint32_t sub0 = 0, sub1 = 0, pph0 = 0, pph1 = 0;   // next TMEM entry of either issuer and its phase
     bool ok = true;
     int sbuf = 0;
     int cached_row_start = -1;              // token tile whose activation scales sit in shared memory (mode 1)
-    int e_hint = 0;
+    Place at;
     uint32_t sph = 0;                       // phase bits of sfull[0..2] (mode 2)
+    if (MODE == 1 && SPLIT) pdl_wait();     // the activation scales are the gather's
     // After a failed wait a warp keeps walking the work list and still joins every named
     // barrier below (doing no other work), so the epilogue warps can never strand each other.
     for (int i = 0; i < my_items; ++i) {
-      const Item im = decode_item<FT, NT>(s_work, p.e_local, item_of(i), e_hint);
+      const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
       const int ft = im.ft;
       const int n = ok ? im.n : 0;
+      // which lanes carry a feature (see Layout)
+      const int feats = im.nu * 8;
+      const bool part = SPLIT && im.nu < 16;
+      const int tl = q * 32 + lane;
+      const bool is_gate = MODE == 1 && part && tl >= feats;
+      const bool warp_used = !part || q * 32 < (MODE == 1 ? 2 * feats : feats);
+      const int lo_col = im.n <= 16 ? 16 : NT;                       // mode 2: where the lo products start
       if (et == 0) TRACE(2, 1000);
       float* s_act;
       float* s_ws;
@@ -568,7 +730,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           }
         }
       };
-      for (int ts = 0; ts < STEPS * (KPS / TKPS) && ok; ++ts) {
+      const int entries = (part && im.n <= 16 ? 4 : KPS) / TKPS;     // TMEM entries per smem ring entry (see Layout)
+      int left = entries;
+      for (int ts = 0; ts < KB / TKPS && ok; ++ts) {
+        const bool odd = (g & 1u) != 0;
+        const uint32_t pr = odd ? SUB + sub1 : sub0, pph = odd ? pph1 : pph0;
         if (!mbar_wait_bounded(&tfull[pr], pph, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
         tc_fence_after();
         if (et == 0) TRACE(2, ts);
@@ -576,14 +742,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         for (int k = 0; k < TKPS; ++k) {
           const int kb = ts * TKPS + k;
           const uint32_t t0 = lane_addr + (pr * TKPS + k) * (2 * NT) + c0;
-          const uint64_t ws0 = f32x2_pack(s_ws[kb], s_ws[kb]);
+          const float ws0f = s_ws[is_gate ? 64 + kb : kb];
+          const uint64_t ws0 = f32x2_pack(ws0f, ws0f);
           const uint64_t ws1 = (MODE == 1) ? f32x2_pack(s_ws[64 + kb], s_ws[64 + kb]) : 0ull;
           const float* sa = s_act + kb * NT + c0;
-          if (c0 < n) {
-            if constexpr (CN == 16) {         // both accumulators of this thread's 16 columns in flight
+          if (c0 < n && warp_used) {
+            if (MODE == 1 && part) {
+              uint32_t r0[16];
+              tmem_ld16(t0, r0);
+              tmem_ld_wait();
+              promote16(r0, r0, 0, sa, ws0, ws0, 0);
+            } else if constexpr (CN == 16) {  // both accumulators of this thread's 16 columns in flight
               uint32_t r0[16], r1[16];
               tmem_ld16(t0, r0);
-              tmem_ld16(t0 + NT, r1);
+              tmem_ld16(t0 + (MODE == 1 ? NT : lo_col), r1);
               tmem_ld_wait();
               promote16(r0, r1, 0, sa, ws0, ws1, 2);
             } else if constexpr (NT == 128 && MODE == 1) {
@@ -615,7 +787,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
                 if (c0 + c * 16 < n) {
                   uint32_t r0[16], r1[16];
                   tmem_ld16(t0 + c * 16, r0);
-                  tmem_ld16(t0 + NT + c * 16, r1);
+                  tmem_ld16(t0 + lo_col + c * 16, r1);
                   tmem_ld_wait();
                   promote16(r0, r1, c * 16, sa + c * 16, ws0, ws1, 2);
                 }
@@ -637,7 +809,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[pr]);
-        if (++pr == PAIRS) { pr = 0; pph ^= 1u; }
+        if (odd) {
+          if (++sub1 == SUB) { sub1 = 0; pph1 ^= 1u; }
+        } else {
+          if (++sub0 == SUB) { sub0 = 0; pph0 ^= 1u; }
+        }
+        if (--left == 0) {
+          left = entries;
+          if (++g == G) g = 0;
+        }
       }
       if (et == 0) TRACE(2, 1002);
       if (MODE == 2) {                        // the scale buffer goes back to the producer
@@ -655,7 +835,33 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         for (int j = 0; j < CN / 2; ++j) f32x2_unpack(acc1p[j], acc1[2 * j], acc1[2 * j + 1]);
       }
 
-      if (MODE == 1) {
+      if (MODE == 1 && part) {
+        // ---- part of an item: the accumulators go to memory, whoever stores an item's last part finishes it
+        const int f = is_gate ? tl - feats : tl;
+        if (f < feats && c0 < n_out) {
+          float* dst = p.o_rows + static_cast<size_t>(im.row_start + c0) * kHidden + ft * 128 + im.u0 * 8 + f +
+                       (is_gate ? kInter : 0);
+#pragma unroll
+          for (int j = 0; j < CN; ++j) __stcg(dst + static_cast<size_t>(j) * kHidden, acc0[j]);
+        }
+        __threadfence();
+        named_bar_sync(2, kEpi);
+        if (et == 0) {
+          const bool last = ok && atomicAdd(p.parts_done + im.tile * FT + ft, 1) == sched.parts - 1;
+          *s_last = last ? 1 : 0;
+          s_pub[i & 255] = last ? 1 : 0;
+        }
+        named_bar_sync(2, kEpi);
+        if (*s_last != 0) {
+          __threadfence();
+          for (int r = et >> 5; r < n_out; r += kEpi / 32)      // a warp per row, four features per lane
+            finish_row(p, im.row_start + r, ft, lane);
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) atomicAdd(s_done, 1);
+      } else if (MODE == 1) {
+        if (SPLIT && et == 0) s_pub[i & 255] = 1;
         // SwiGLU, then the per-row amax over the 128 features of this tile.  The fast exp and
         // divide are a few ulp off the exact ones, far below the 8-bit requantisation that follows.
         // (n is a multiple of 16, so validity is decided per block of sixteen columns and the
@@ -724,7 +930,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       } else {
         const int qrow = lane & 3;
         const int row0 = im.row_start + c0 + qrow;
-        const int col = ft * 128 + q * 32 + (lane >> 2) * 4;
+        const int col = ft * 128 + im.u0 * 8 + q * 32 + (lane >> 2) * 4;
 #pragma unroll
         for (int j = 0; j < CN; j += 4) {
           if (c0 + j < n_out) {
@@ -732,13 +938,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             quad_transpose_f32(a0, a1, a2, a3, lane);   // now: row c0 + j + qrow, four adjacent features
             // expert parallelism: the row's place in its token owner's memory (plain stores over NVLink)
             float* o = p.row_out != nullptr ? p.row_out[row0 + j] : p.o_rows + static_cast<size_t>(row0 + j) * kHidden;
-            if (o != nullptr) *reinterpret_cast<float4*>(o + col) = make_float4(a0, a1, a2, a3);
+            if (o != nullptr && (!part || q * 32 + (lane >> 2) * 4 < feats))
+              *reinterpret_cast<float4*>(o + col) = make_float4(a0, a1, a2, a3);
           }
         }
       }
     }
   }
 
+  if (MODE == 1 && SPLIT) pdl_wait();   // no CTA ends before the gather has (kernels behind this one rely on it)
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -759,8 +967,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 template <int MODE, int NT>
 cudaError_t launch_gemm(const GemmLaunch& g, const GemmArgs& a, int num_sms, cudaStream_t st) {
   return launch_dependent(grouped_gemm_kernel<MODE, NT>, dim3(num_sms), dim3(Cfg<MODE, NT>::kThreads),
-                          static_cast<size_t>(Cfg<MODE, NT>::kSmemBytes), st, g.tm_w, g.tm_b0, g.tm_b1, g.tm_b0s,
-                          g.tm_b1s, g.tm_sc, a);
+                          static_cast<size_t>(Cfg<MODE, NT>::kSmemBytes), st, g.tm_w, g.tm_b, g.tm_bs, g.tm_sc,
+                          g.tm_part, a);
 }
 
 template <int MODE, int NT>
@@ -783,8 +991,8 @@ cudaError_t gemm_set_attributes() {
 
 cudaError_t launch_gemm1(const GemmLaunch& g, const float* w13_scale, int e_local, const Workspace& ws, int num_sms,
                          cudaStream_t st) {
-  GemmArgs a{g.w_packed, ws.work, ws.meta, ws.a_scale, w13_scale, ws.c_hi, ws.c_lo, ws.c_scale, nullptr, ws.row_cap, e_local,
-             ws.ready, ws.status, ws.trace, ws.trace + 6 * 4096, g.wait_limit, g.silent_producer, nullptr};
+  GemmArgs a{g.w_packed, ws.work, ws.meta, ws.a_scale, w13_scale, ws.c_hi, ws.c_lo, ws.c_scale, ws.o_rows, ws.row_cap, e_local,
+             ws.ready, ws.parts_done, ws.status, ws.trace, ws.trace + 6 * 4096, g.wait_limit, g.silent_producer, nullptr};
   if (g.token_tile == 128) return launch_gemm<1, 128>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<1, 32>(g, a, num_sms, st) : launch_gemm<1, 64>(g, a, num_sms, st);
 }
@@ -792,7 +1000,7 @@ cudaError_t launch_gemm1(const GemmLaunch& g, const float* w13_scale, int e_loca
 cudaError_t launch_gemm2(const GemmLaunch& g, const float* w2_scale, int e_local, const Workspace& ws, int num_sms,
                          cudaStream_t st) {
   GemmArgs a{g.w_packed, ws.work, ws.meta, ws.c_scale, w2_scale, nullptr, nullptr, nullptr, ws.o_rows, ws.row_cap, e_local,
-             ws.ready, ws.status, ws.trace + 3 * 4096, ws.trace + 7 * 4096, g.wait_limit, g.silent_producer,
+             ws.ready, nullptr, ws.status, ws.trace + 3 * 4096, ws.trace + 7 * 4096, g.wait_limit, g.silent_producer,
              g.rows_to_targets ? ws.row_out : nullptr};
   if (g.token_tile == 128) return launch_gemm<2, 128>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<2, 32>(g, a, num_sms, st) : launch_gemm<2, 64>(g, a, num_sms, st);

@@ -61,6 +61,7 @@ struct Workspace {
   uint32_t* local_mask = nullptr; // [T] bit e set when local expert e was selected
   int* counts = nullptr;          // [32] rows per local expert
   int* ready = nullptr;           // [32] GEMM1 work items finished per local expert (counts + 32: zeroed together)
+  int* parts_done = nullptr;      // [row_cap / 16 + 32][16] finished parts of GEMM1's split items, per (token tile, feature tile)
   int* counts_last = nullptr;     // [32] copy of counts kept after the call (counts itself is re-zeroed for the next)
   int* meta = nullptr;            // [kMetaInts]
   int* status = nullptr;          // [4]
@@ -73,7 +74,7 @@ struct Workspace {
   uint8_t* a_perm = nullptr;      // [row_cap, 7168] e4m3 gathered activations
   float* a_scale = nullptr;       // [56, row_cap]
   uint8_t* c_hi = nullptr;        // [row_cap, 2048] e4m3 SwiGLU output, leading term
-  uint8_t* c_lo = nullptr;        // [row_cap, 2048] e4m3 residual term (scale = c_scale / 28)
+  uint8_t* c_lo = nullptr;        // [row_cap, 2048] e4m3 residual term (scale = c_scale / 28); right behind c_hi, one allocation
   float* c_scale = nullptr;       // [16, row_cap]
   float* o_rows = nullptr;        // [row_cap, 7168] f32 per-route expert outputs
   float** row_out = nullptr;      // [row_cap] expert parallelism: where GEMM2 stores each row (a peer's memory), null = nowhere
@@ -81,12 +82,20 @@ struct Workspace {
   size_t bytes = 0;
 };
 
+// Weight maps with boxes of 64, 32 and 16 rows: the rows of a part of a feature tile.
+struct PartMaps {
+  CUtensorMap m[3];
+};
+
+// Every operand is a stack of byte matrices [z][rows][K], fetched 128 bytes of K at a time: W13 as [2 E][2048][7168]
+// (up, gate, up, gate ...; a box takes both of its expert), W2 as [E][7168][2048], the gathered activations as
+// [1][row_cap][7168], the two-term intermediate as [2][row_cap][2048] (a box takes hi and lo rows).  The thread that
+// issues the loads needs about 75 cycles for each, so few and large ones matter.
 struct GemmLaunch {
-  CUtensorMap tm_w;    // weights, 2-D [E * rows_per_expert, K], box 128 x 128
-  CUtensorMap tm_b0;   // token-side operand, box token_tile x 128 (GEMM1: a_perm; GEMM2: c_hi)
-  CUtensorMap tm_b1;   // GEMM2: c_lo (unused by GEMM1)
-  CUtensorMap tm_b0s;  // same tensors with a 16-row box: tiles of <= 16 rows pull half the bytes
-  CUtensorMap tm_b1s;
+  CUtensorMap tm_w;    // weights, box 128 rows
+  CUtensorMap tm_b;    // token side, box token_tile rows
+  CUtensorMap tm_bs;   // token side, box 16 rows: tiles of <= 16 rows pull half the bytes
+  PartMaps tm_part;    // weights, smaller boxes (32-row token tile only)
   CUtensorMap tm_sc;   // GEMM2: c_scale as f32 [16, row_cap], box 16 x token_tile (one load per work item)
   const uint8_t* w_packed = nullptr;   // pre-packed weights (tm_w unused) or nullptr
   int token_tile;      // 32, 64 or 128: token rows per work item, must match the row-list kernel's

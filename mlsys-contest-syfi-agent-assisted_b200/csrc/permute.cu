@@ -145,7 +145,7 @@ constexpr int kGatherThreads = 224;  // 7168 B per row = 448 x 16 B = 2 per thre
 __global__ void __launch_bounds__(kGatherThreads)
 gather_rows_kernel(const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, int T,
                    const int* __restrict__ row_token, const int* __restrict__ meta, uint8_t* __restrict__ a_perm,
-                   float* __restrict__ a_scale, int row_cap, int* __restrict__ counts) {
+                   float* __restrict__ a_scale, int row_cap, int* __restrict__ counts, int* __restrict__ parts_done) {
   pdl_wait();
   pdl_trigger();
   // every reader of the per-expert row counters (the row-list kernel) has finished: zero them for the
@@ -153,6 +153,7 @@ gather_rows_kernel(const uint8_t* __restrict__ hidden, const float* __restrict__
   if (blockIdx.x == 0 && threadIdx.x < kMaxLocalExperts) counts[threadIdx.x] = 0;
   const int rows_total = meta[1];
   const int tid = threadIdx.x;
+  for (int i = blockIdx.x * kGatherThreads + tid; i < meta[0] * kIBlocks; i += gridDim.x * kGatherThreads) parts_done[i] = 0;
   for (int r = blockIdx.x; r < rows_total; r += gridDim.x) {
     const int t = row_token[r];
     uint4* dst = reinterpret_cast<uint4*>(a_perm + static_cast<size_t>(r) * kHidden);
@@ -192,7 +193,7 @@ cudaError_t launch_gather(const uint8_t* hidden, const float* hidden_scale, int 
   const int max_rows = 8 * T + kRowPad * kMaxLocalExperts;
   const int grid = max_rows < num_sms * 8 ? max_rows : num_sms * 8;
   return launch_dependent(gather_rows_kernel, dim3(grid), dim3(kGatherThreads), 0, st, hidden, hidden_scale, T,
-                          ws.row_token, ws.meta, ws.a_perm, ws.a_scale, ws.row_cap, ws.counts);
+                          ws.row_token, ws.meta, ws.a_perm, ws.a_scale, ws.row_cap, ws.counts, ws.parts_done);
 }
 
 }  // namespace syfi
