@@ -84,6 +84,10 @@ template <int MODE, int NT> struct Cfg {
   static_assert(kKBlocks % kKps == 0 && kSlots % kTKps == 0 && kKps % kTKps == 0,
                 "steps must tile the K blocks and the slots");
   static_assert(kThreads <= 1024, "too many epilogue warps");
+  // MMA-issuing threads (see mma_role).  The larger token tiles have only two TMEM entries (four hand-offs at 128 rows),
+  // so a second issuer finds its one entry still being promoted and adds its polling to the hand-offs: at 64 rows two
+  // issuers took 747 us where one takes 731 (4096 tokens, hot experts), 308.9 against 299.4 (2048 tokens).
+  static constexpr int kIssuers = NT == 32 ? 2 : 1;
   // The 32-row kernel cuts the items of a thin last round along the features (see Walker).
   static constexpr bool kSplit = NT == 32;
 };
@@ -280,9 +284,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   constexpr int FT = C::kFeatTiles;
   constexpr int TKPS = C::kTKps;
   constexpr int PAIRS = C::kPairs;        // TMEM ring entries, each kTKps accumulator-pair slots
-  // Half of them for each MMA issuer (see mma_role).
-  constexpr int SUB = PAIRS / 2;
-  static_assert(PAIRS % 2 == 0, "two issuers");
+  constexpr int ISSUERS = C::kIssuers;
+  constexpr int SUB = PAIRS / ISSUERS;    // each MMA issuer's share of them
+  static_assert(PAIRS % ISSUERS == 0, "whole shares");
   constexpr bool SPLIT = C::kSplit;
 
   extern __shared__ uint8_t smem_raw[];
@@ -363,7 +367,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const Schedule sched = make_schedule<FT, SPLIT>(s_meta[0]);
   const int my_items = sched.items();
 
-  // MMA issue, one thread of each of two warps: one has the even ring entries, one the odd ones (fixed, so that either
+  // MMA issue, one thread of each of kIssuers warps; of two, one has the even ring entries, one the odd ones (fixed, so that either
   // sees every phase of its barriers: a parity wait for a phase whose predecessor is not over returns at once).  With the weights as the M operand an MMA takes
   // 70 to 80 cycles however few columns it has (its 128 rows x 32 bytes come out of shared memory), the issuing thread
   // is tied up while its MMAs execute and then pays the commits and the next waits (300 to 400 cycles per entry): with
@@ -415,7 +419,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const Kind kind = kind_of<NT, SPLIT>(im);
       const int steps = kind == kPartFew ? KB / Layout<MODE, NT, SPLIT ? kPartFew : kWhole>::kKps : KB / KPS;
       for (int step = 0; step < steps; ++step) {
-        if ((g & 1u) == par) {
+        if (ISSUERS == 1 || (g & 1u) == par) {
           if (!mbar_wait_bounded(&full[g], ph, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
           TRACE(1, step);
           if (!SPLIT || kind == kWhole) alive = issue(Layout<MODE, NT, kWhole>{}, idesc);
@@ -554,7 +558,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     __syncwarp();
   } else if (warp == 3 + 4 * C::kColSplit) {
     // --------------------------------------------------------------- MMA issuer of the odd ring entries
-    if (lane == 0) mma_role(1);
+    if (ISSUERS == 2 && lane == 0) mma_role(1);
     __syncwarp();
   } else if (warp == 2 + 4 * C::kColSplit) {
     // ------------------------------------------------ publisher (mode 1, one thread)
@@ -733,7 +737,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const int entries = (part && im.n <= 16 ? 4 : KPS) / TKPS;     // TMEM entries per smem ring entry (see Layout)
       int left = entries;
       for (int ts = 0; ts < KB / TKPS && ok; ++ts) {
-        const bool odd = (g & 1u) != 0;
+        const bool odd = ISSUERS == 2 && (g & 1u) != 0;
         const uint32_t pr = odd ? SUB + sub1 : sub0, pph = odd ? pph1 : pph0;
         if (!mbar_wait_bounded(&tfull[pr], pph, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
         tc_fence_after();
