@@ -226,7 +226,11 @@ const void* mapped_alias(const void* host) {
   return nullptr;
 }
 
-constexpr int64_t kPairMinTokens = 6144;   // batches from this size on use the CTA-pair GEMM kernels (measured: even at 4096, 8 % faster at 8192, 17 % at 16384)
+// Batches from this size on use the CTA-pair GEMM kernels, with GEMM1's small remainders on the single-CTA kernel.
+// Against 64-row tiles alone, us per call, two seeds: 3072 tokens 459 / 387 and 482 / 372, 4096 tokens 523 / 435 and
+// 570 / 467, 8192 tokens 870 / 829 and 1030 / 958.
+constexpr int64_t kPairMinTokens = 3584;
+constexpr int64_t kWideListMinTokens = 6144;   // from here on the row lists of the pair configuration count 128-row tiles
 constexpr int kFlagOutF32 = 1;      // run_layer flags
 constexpr int kFlagPrepacked = 2;
 constexpr int kFlagRoutingGiven = 4;   // the workspace already holds routes, masks and row counters of all tokens (token dispatch)
@@ -291,7 +295,8 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   // only exist on the device: 32 rows while the layer is bound by streaming weights (measured faster up
   // to 1024 tokens: 8 accumulator slots in flight, two K blocks per barrier round), 64 rows beyond.
   // Large batches (experts with hundreds of rows each) run the CTA-pair kernels, which cut their own
-  // token tiles (256 rows in GEMM1, 128 in GEMM2); token_tile 256 stands for that configuration here.
+  // token tiles (256 rows in GEMM1, 128 in GEMM2), and the 64-row GEMM1 on what tail_rows() leaves to it;
+  // token_tile 256 stands for that configuration here.
   int token_tile = (T64 <= 1024) ? 32 : (T64 < kPairMinTokens || packed) ? 64 : 256;
   if (const char* ov = getenv("SYFI_MOE_TOKEN_TILE")) {   // tuning knob: force 32, 64, 128 or (pair kernels) 256
     const int v = atoi(ov);
@@ -303,7 +308,8 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
                           ctx->map_packed == packed;
   if (!maps_valid) {
   ctx->map_w13 = nullptr;
-  g1.token_tile = g2.token_tile = token_tile;
+  g1.token_tile = g2.token_tile = pair ? kTailTile : token_tile;
+  g1.tails = pair ? 1 : 0;
   g1.w_packed = packed ? static_cast<const uint8_t*>(w13) : nullptr;
   g2.w_packed = packed ? static_cast<const uint8_t*>(w2) : nullptr;
   if (pair) {
@@ -315,6 +321,10 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     if ((rc = make_map(&ctx->p2.tm_b1, ws.c_lo, ws.row_cap, kInter, 32))) return rc;
     if ((rc = make_map(&ctx->p1.tm_b0w, ws.a_perm, ws.row_cap, kHidden, 128))) return rc;
     ctx->p1.tm_b1w = ctx->p1.tm_b0w;
+    // GEMM1's remainders (see tail_rows)
+    if ((rc = make_map3(&g1.tm_w, w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128))) return rc;
+    if ((rc = make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, kTailTile))) return rc;
+    if ((rc = make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16))) return rc;
     if ((rc = make_map(&ctx->p2.tm_b0w, ws.c_hi, ws.row_cap, kInter, 128))) return rc;
     if ((rc = make_map(&ctx->p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128))) return rc;
   } else {
@@ -365,7 +375,9 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     CU_TRY(cudaEventRecord(ctx->ev_copy_done, ctx->copy_stream));
     ctx->wait_before_gather = ctx->ev_copy_done;
   }
-  CU_TRY(launch_build_rows(T, e_local, (int)offset, pair ? 128 : token_tile, ws, st));
+  // The pair configuration's kernels count their own tiles; the row lists' count is what syfi_moe_debug_read shows.
+  const int listed_tile = !pair ? token_tile : T64 < kWideListMinTokens ? 64 : 128;
+  CU_TRY(launch_build_rows(T, e_local, (int)offset, listed_tile, ws, st));
   ctx->launches += 1;
   const syfi_moe_ep_desc* ep_rows = ctx->ep_rows;
   ctx->ep_rows = nullptr;
@@ -391,8 +403,11 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   g1.silent_producer = ctx->p1.silent_producer = (fault & 1) ? 1 : 0;
   g2.silent_producer = ctx->p2.silent_producer = (fault & 8) ? 1 : 0;
   if (!(fault & 2)) {
-    if (pair) CU_TRY(launch_pair_gemm1(ctx->p1, static_cast<const float*>(w13_scale), e_local, ws, grid, st));
-    else CU_TRY(launch_gemm1(g1, static_cast<const float*>(w13_scale), e_local, ws, grid, st));
+    if (pair) {
+      CU_TRY(launch_pair_gemm1(ctx->p1, static_cast<const float*>(w13_scale), e_local, ws, grid, st));
+      ctx->launches += 1;
+    }
+    CU_TRY(launch_gemm1(g1, static_cast<const float*>(w13_scale), e_local, ws, grid, st));   // pair: the remainders
     ctx->launches += 1;
   }
   STAGE_MARK(4);

@@ -88,7 +88,7 @@ template <int MODE, int NT> struct Cfg {
   // so a second issuer finds its one entry still being promoted and adds its polling to the hand-offs: at 64 rows two
   // issuers took 747 us where one takes 731 (4096 tokens, hot experts), 308.9 against 299.4 (2048 tokens).
   static constexpr int kIssuers = NT == 32 ? 2 : 1;
-  // The 32-row kernel cuts the items of a thin last round along the features (see Walker).
+  // The 32-row kernel cuts the items of a thin last round along the features (see Schedule).
   static constexpr bool kSplit = NT == 32;
 };
 
@@ -114,6 +114,7 @@ struct GemmArgs {
   long long* trace_cta;     // [grid][5] per-CTA start/end (globaltimer, clock64) and SM id, SYFI_TRACE only
   long long wait_limit;     // SM clocks a wait may take before the CTA gives up (tests make it short)
   int silent_producer;      // test hook: the TMA producer issues nothing, so that the other roles' waits run out
+  int tails;                // mode 1 behind the pair kernel: work on the rows tail_rows() names, see below
   float* const* row_out;    // mode 2, expert parallelism: row r goes to row_out[r] (a peer's memory; null = padding row, not stored) instead of o_rows
 };
 
@@ -350,10 +351,31 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // The 32-row GEMM1 also starts on its weights before the kernel in front of it is done: that kernel, the gather,
   // lets this one start only after its own wait for the row lists, so the work table is complete here; only the
   // gathered rows and their scales are waited for (by the producer and the epilogue warps).
-  if (MODE == 1 && !SPLIT) pdl_wait();
+  // Behind the pair kernel (tails) there is nothing to wait for: every CTA of that kernel has waited for the gather
+  // before it let this one start, and the two share no output; waiting for its end would leave SMs idle.
+  if (MODE == 1 && !SPLIT && !p.tails) pdl_wait();
   pdl_trigger();
   // the work table and the two counters every role needs, fetched in one round trip
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxLocalExperts) {
+  if (MODE == 1 && NT == kTailTile && p.tails) {
+    if (warp == 2) {        // this kernel's own table: the tails of the experts, and the prefix sums of their tiles
+      // (meta[1] = 0: the row-list kernel refused the call, its work table is stale)
+      ExpertWork ew = (lane < p.e_local && p.meta[1] > 0) ? p.work[lane] : ExpertWork{0, 0, 0, 0};
+      const int tail = tail_rows(ew.rows_pad);
+      ew.row_off += ew.rows_pad - tail;
+      ew.rows_pad = tail;
+      ew.tiles = (tail + NT - 1) / NT;
+      int incl = ew.tiles;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      ew.tile_off = incl - ew.tiles;
+      s_work[lane] = ew;
+      const unsigned active = __ballot_sync(0xffffffffu, tail > 0);
+      if (lane == 31) { s_meta[0] = incl; s_meta[1] = __popc(active); }
+    }
+  } else if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxLocalExperts) {
     const int e = threadIdx.x - 64;
     s_work[e] = (e < p.e_local) ? p.work[e] : ExpertWork{0, 0, 0, 0};
   } else if (threadIdx.x == 64 + kMaxLocalExperts) {
@@ -996,7 +1018,7 @@ cudaError_t gemm_set_attributes() {
 cudaError_t launch_gemm1(const GemmLaunch& g, const float* w13_scale, int e_local, const Workspace& ws, int num_sms,
                          cudaStream_t st) {
   GemmArgs a{g.w_packed, ws.work, ws.meta, ws.a_scale, w13_scale, ws.c_hi, ws.c_lo, ws.c_scale, ws.o_rows, ws.row_cap, e_local,
-             ws.ready, ws.parts_done, ws.status, ws.trace, ws.trace + 6 * 4096, g.wait_limit, g.silent_producer, nullptr};
+             ws.ready, ws.parts_done, ws.status, ws.trace, ws.trace + 6 * 4096, g.wait_limit, g.silent_producer, g.tails, nullptr};
   if (g.token_tile == 128) return launch_gemm<1, 128>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<1, 32>(g, a, num_sms, st) : launch_gemm<1, 64>(g, a, num_sms, st);
 }
@@ -1004,7 +1026,7 @@ cudaError_t launch_gemm1(const GemmLaunch& g, const float* w13_scale, int e_loca
 cudaError_t launch_gemm2(const GemmLaunch& g, const float* w2_scale, int e_local, const Workspace& ws, int num_sms,
                          cudaStream_t st) {
   GemmArgs a{g.w_packed, ws.work, ws.meta, ws.c_scale, w2_scale, nullptr, nullptr, nullptr, ws.o_rows, ws.row_cap, e_local,
-             ws.ready, nullptr, ws.status, ws.trace + 3 * 4096, ws.trace + 7 * 4096, g.wait_limit, g.silent_producer,
+             ws.ready, nullptr, ws.status, ws.trace + 3 * 4096, ws.trace + 7 * 4096, g.wait_limit, g.silent_producer, 0,
              g.rows_to_targets ? ws.row_out : nullptr};
   if (g.token_tile == 128) return launch_gemm<2, 128>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<2, 32>(g, a, num_sms, st) : launch_gemm<2, 64>(g, a, num_sms, st);

@@ -33,6 +33,8 @@
 // mode 2: multiplies a K block's activation scales with its weight scale into a shared-memory ring),
 // warp 3 = cross-kernel bookkeeping (as in grouped_gemm.cu), warps 4..19 = promotion / epilogue
 // (a warp reads one tensor-memory lane quarter; four warps share a quarter and split the columns).
+// An expert's last rows, up to 128 that would leave a 256-row tile at most half full, are not this GEMM1's but the
+// single-CTA kernel's, launched right behind it (see tail_rows).
 // Barriers another CTA signals: full[] lives in the first CTA and counts the bytes of both CTAs' loads;
 // empty[] and tfull[] exist in both CTAs and are signalled by one tcgen05.commit each; tempty[] lives
 // in the first CTA and collects the arrivals of both CTAs' epilogue warps.
@@ -59,7 +61,7 @@ constexpr int kPairTmemCols = 512;
 template <int MODE> struct PairCfg {
   static constexpr int kKBlocks = MODE == 1 ? kHBlocks : kIBlocks;              // 56 / 16
   static constexpr int kFeatItems = MODE == 1 ? kInter / 128 : kHidden / 256;   // 16 / 28 per expert and token tile
-  static constexpr int kTokTile = MODE == 1 ? 256 : 128;
+  static constexpr int kTokTile = MODE == 1 ? kPairTile : 128;
   static constexpr int kStages = 6;
   // Two accumulator slots of 256 tensor-memory columns: the MMAs of K block k + 1 run while block k is
   // promoted.  (Four slots of 128 columns, a K block issued as two MMA groups of N = 128, doubled the
@@ -211,6 +213,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // this kernel's own tile table: token tiles of NT rows per expert and their prefix sums
     // (meta[1] = 0: the row-list kernel refused the call, its work table is stale)
     ExpertWork ew = (lane < p.e_local && p.meta[1] > 0) ? p.work[lane] : ExpertWork{0, 0, 0, 0};
+    if (MODE == 1) ew.rows_pad -= tail_rows(ew.rows_pad);   // the rest is the single-CTA kernel's
     const int tiles = (ew.rows_pad + NT - 1) / NT;
     int incl = tiles;
 #pragma unroll
@@ -221,8 +224,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     ew.tiles = tiles;
     ew.tile_off = incl - tiles;
     s_work[lane] = ew;
-    if (lane == 31) s_meta[0] = incl;
-    if (lane == 0) s_meta[1] = p.meta[3];
+    const unsigned active = __ballot_sync(0xffffffffu, tiles > 0);
+    if (lane == 31) { s_meta[0] = incl; s_meta[1] = __popc(active); }
   }
   tc_fence_before();
   __syncthreads();
@@ -459,8 +462,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       }
     } else {
       // ------------------------------------------------ publisher (mode 1) / dependency helper (mode 2)
-      // Same hand-off as in grouped_gemm.cu.  Every CTA of a pair counts its own half of an item, so an
-      // expert is complete at 2 * 16 * (its 256-row token tiles).
+      // Same hand-off as in grouped_gemm.cu.  Every CTA of a pair counts its own half of an item, the single-CTA
+      // kernel its items, so an expert is complete at 2 * 16 * (its 256-row token tiles) + 16 * (its tail tiles).
       if (MODE == 1 && lane == 0) {
         int done_target = 0, e_hint = 0;
         for (int i = 0; i < my_items; ++i) {
@@ -486,7 +489,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
           if (im.expert != ready_expert) {
             const int rows_pad = s_work[im.expert].rows_pad;
-            const int need = 2 * (kInter / 128) * ((rows_pad + PairCfg<1>::kTokTile - 1) / PairCfg<1>::kTokTile);
+            const int tail = tail_rows(rows_pad);
+            const int need = 2 * (kInter / 128) * ((rows_pad - tail + PairCfg<1>::kTokTile - 1) / PairCfg<1>::kTokTile) +
+                             (kInter / 128) * ((tail + kTailTile - 1) / kTailTile);
             const long long t0 = clock64();
             bool seen = true;
             while (ld_acquire_gpu(p.ready + im.expert) < need) {

@@ -99,10 +99,27 @@ struct GemmLaunch {
   CUtensorMap tm_sc;   // GEMM2: c_scale as f32 [16, row_cap], box 16 x token_tile (one load per work item)
   const uint8_t* w_packed = nullptr;   // pre-packed weights (tm_w unused) or nullptr
   int token_tile;      // 32, 64 or 128: token rows per work item, must match the row-list kernel's
+  int tails = 0;       // GEMM1 behind the pair kernel: only the rows tail_rows() leaves to it (token_tile = kTailTile)
   long long wait_limit = 1ll << 32;   // SM clocks a device-side wait may take (about two seconds)
   int silent_producer = 0;            // test hook, see syfi_moe_debug_fault
   int rows_to_targets = 0;            // GEMM2 stores row r at Workspace::row_out[r] instead of o_rows
 };
+
+// How a call with CTA pairs splits an expert's padded rows between GEMM1's two kernels: the pair kernel takes tiles of
+// 256 rows, and a remainder of more than kTailRows; a smaller remainder goes to the single-CTA kernel (kTailTile-row
+// tiles), because in the pair kernel the rows are the M operand, whose height is fixed, and in the other one the N
+// operand, which is as wide as there are rows.  A K block of a tile takes a pair about 2500 SM clocks however few rows
+// there are, the single-CTA kernel about 950 per 64 rows: the line lies between two and three of its tiles.  Measured, us
+// per call, pairs alone / lines at 64, 128 and 192 rows: 4096 tokens 566 / 540, 537, 532 and 496 / 450, 442, 453 (another
+// seed); 8192 tokens 916 / 874, 885, 883 and 852 / 823, 830, 848; 16384 tokens 908 / 879, 863, 863.  The remainders come
+// second: in front of the pairs they cost 1 to 3 % more, as the pairs' long last round then ends the GEMM.
+constexpr int kPairTile = 256;
+constexpr int kTailRows = 128;
+constexpr int kTailTile = 64;
+__host__ __device__ inline int tail_rows(int rows_pad) {
+  const int rest = rows_pad % kPairTile;
+  return rest <= kTailRows ? rest : 0;
+}
 
 // Tensor maps of the CTA-pair GEMM kernels (grouped_gemm_pair.cu): token-side operands use 32-row boxes.
 struct PairGemmLaunch {

@@ -255,6 +255,44 @@ def test_every_token_tile_gives_the_same_bits(T, E, off, seed, pkg, oracle, monk
         assert torch.equal(outs[0], o)
 
 
+@pytest.mark.parametrize("rows", [
+    (1,), (16,), (17, 0, 32),                        # 32-row tiles, thin last round: eight, eight and four parts an item
+    (5, 31, 16, 1), (33, 64, 2, 40, 18, 1, 70, 16),  # two parts; whole rounds in front of the split one
+    (127, 128, 129, 130), (255, 256, 257, 0, 64, 65, 1, 144), (383, 384, 385, 400, 320, 321),   # remainders of 256 rows
+])
+def test_rows_per_expert_at_the_edges_of_the_work_split(rows, pkg, oracle, monkeypatch):
+    """Exact row counts per expert.  The 32-row kernel cuts a thin last round's items along their features, the
+    CTA-pair configuration hands remainders of at most 128 rows to the single-CTA GEMM1: neither changes the
+    arithmetic of an element, so both equal the 64-row kernel, which does neither, bit for bit (plain and packed)."""
+    E, T = len(rows), max(rows) + 3
+    inp = pkg.make_inputs(num_tokens=T, seed=17, e_local=E, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    logits = torch.randn(T, 256, generator=g, device=DEV) * 0.3 - 2.0      # other groups: two scores of about 0.2
+    logits[:, :32] = -9.0
+    for e, n in enumerate(rows):
+        logits[torch.randperm(T, generator=g, device=DEV)[:n], e] = 8.0    # one score of 1: the token routes here
+    inp = pkg.MoeInputs(logits, torch.zeros_like(inp.routing_bias), *inp.args()[2:])
+    packed = pkg.prepack_weights(inp.gemm1_weights, inp.gemm2_weights)
+    outs = []
+    for tile in (64, 32, 256):
+        monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", str(tile))
+        out, _ = _run(pkg, inp)
+        counts, _ = pkg.get_context(0).debug_read("counts", torch.int32)
+        assert tuple(counts[:E].tolist()) == rows
+        outs.append(out)
+        if tile == 32:
+            out_p = torch.full_like(out, float("nan"))
+            pkg.run_moe_prepacked(*inp.args()[:4], packed, inp.gemm1_weights_scale, inp.gemm2_weights_scale, 0,
+                                  inp.routed_scaling_factor, out_p)
+            pkg.get_context(0).check()
+            outs.append(out_p)
+    ref, _, _ = oracle.moe_forward(*inp.args())
+    ok, ostats = oracle.check_output(outs[0], ref)
+    assert ok, ostats
+    for o in outs[1:]:
+        assert torch.equal(outs[0], o)
+
+
 def _swizzled_tiles(x):
     """x: [..., 128 rows, 8 chunks, 16 bytes] -> chunk c of row r moved to chunk c ^ (r & 7)."""
     r = torch.arange(128, device=x.device)[:, None]
