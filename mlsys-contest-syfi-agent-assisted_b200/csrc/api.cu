@@ -362,6 +362,22 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   // has left (or will have left, in stream order) the row counters at zero
   const bool clean = ctx->counters_clean;
   ctx->counters_clean = false;
+  const syfi_moe_ep_desc* ep_rows = ctx->ep_rows;
+  ctx->ep_rows = nullptr;
+  g2.rows_to_targets = ctx->p2.rows_to_targets = ep_rows != nullptr ? 1 : 0;
+  // Small batches whose inputs are all on the device: router, row lists and gather in one launch.  (The combine kernel
+  // must follow: it ends the tables' validity.)
+  const bool front = T <= kFrontMaxTokens && token_tile == 32 && out != nullptr && ep_rows == nullptr &&
+                     ctx->n_pending == 0 && ctx->wait_before_gather == nullptr && !(flags & kFlagRoutingGiven);
+  g1.front = g2.front = front ? 1 : 0;
+  if (front) {
+    CU_TRY(launch_front(static_cast<const float*>(logits), bias, static_cast<const uint8_t*>(hs),
+                        static_cast<const float*>(hs_scale), T, e_local, (int)offset, (float)scaling, token_tile, ws,
+                        ctx->num_sms, st));
+    ctx->launches += 1;
+    STAGE_MARK(1);
+    STAGE_MARK(2);
+  } else {
   if (!(flags & kFlagRoutingGiven)) {
     CU_TRY(launch_router(static_cast<const float*>(logits), bias, T, e_local, (int)offset, (float)scaling, ws, clean, st));
     ctx->launches += 1;
@@ -379,9 +395,6 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   const int listed_tile = !pair ? token_tile : T64 < kWideListMinTokens ? 64 : 128;
   CU_TRY(launch_build_rows(T, e_local, (int)offset, listed_tile, ws, st));
   ctx->launches += 1;
-  const syfi_moe_ep_desc* ep_rows = ctx->ep_rows;
-  ctx->ep_rows = nullptr;
-  g2.rows_to_targets = ctx->p2.rows_to_targets = ep_rows != nullptr ? 1 : 0;
   if (ep_rows != nullptr) {          // where GEMM2 will store every row: the token owners' memory
     CU_TRY(launch_ep_row_targets(*ep_rows, ctx->ep_rows_seq, ws, st));
     ctx->launches += 1;
@@ -393,6 +406,7 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   }
   CU_TRY(launch_gather(static_cast<const uint8_t*>(hs), static_cast<const float*>(hs_scale), T, ws, ctx->num_sms, st));
   ctx->launches += 1;
+  }
   STAGE_MARK(3);
   // test hook: short wait limit and roles / kernels left out for this one call (see syfi_moe_debug_fault)
   const int fault = ctx->fault_mask;

@@ -25,10 +25,12 @@ static_assert(kSegments * kCombineThreads * 4 == kHidden, "row must split evenly
 // round trips to memory, which is what this kernel's duration consists of at small batches).
 __global__ void __launch_bounds__(kCombineThreads)
 combine_segments_kernel(int T, const int* __restrict__ route_row, const float* __restrict__ topk_w,
-               const float* __restrict__ o_rows, void* __restrict__ out, int out_is_f32, int row_cap) {
+               const float* __restrict__ o_rows, void* __restrict__ out, int out_is_f32, int row_cap,
+               int* __restrict__ meta) {
   const int t = blockIdx.x, seg = blockIdx.y;
   pdl_wait();
   pdl_trigger();
+  if (t == 0 && seg == 0 && threadIdx.x == 0) meta[kMetaTables] = 0;   // see front_kernel
   if (t >= T) return;
   const int col4 = seg * kCombineThreads + threadIdx.x;        // float4 index inside the row
   int rows[kTopK];
@@ -122,7 +124,7 @@ combine_rows_kernel(int T, const int* __restrict__ route_row, const float* __res
 cudaError_t launch_combine(int T, const Workspace& ws, void* out, int out_is_f32, cudaStream_t st) {
   if (T <= 512)   // latency-bound sizes: 7 CTAs per token, all eight routes' loads in flight
     return launch_dependent(combine_segments_kernel, dim3(T, kSegments), dim3(kCombineThreads), 0, st, T,
-                            ws.route_row, ws.topk_w, ws.o_rows, out, out_is_f32, ws.row_cap);
+                            ws.route_row, ws.topk_w, ws.o_rows, out, out_is_f32, ws.row_cap, ws.meta);
   return launch_dependent(combine_rows_kernel, dim3(T), dim3(kCombineThreads), 0, st, T, ws.route_row, ws.topk_w,
                           ws.o_rows, out, out_is_f32, ws.row_cap);
 }

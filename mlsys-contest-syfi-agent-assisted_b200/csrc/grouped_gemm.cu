@@ -273,7 +273,9 @@ __device__ __forceinline__ void finish_row(const GemmArgs& p, int row, int ft, i
   if (lane == 0) p.c_scale[static_cast<size_t>(ft) * p.row_cap + row] = sc;
 }
 
-template <int MODE, int NT>
+// FRONT (32-row tile): front_kernel made the tables, see pdl_trigger below.  (Asked at run time, the question cost the
+// other calls half a microsecond.)
+template <int MODE, int NT, bool FRONT>
 __global__ void __launch_bounds__((Cfg<MODE, NT>::kThreads), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b,
                     const __grid_constant__ CUtensorMap tm_bs, const __grid_constant__ CUtensorMap tm_sc,
@@ -350,11 +352,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // counters GEMM2 reads here were complete before GEMM1 passed its own wait.
   // The 32-row GEMM1 also starts on its weights before the kernel in front of it is done: that kernel, the gather,
   // lets this one start only after its own wait for the row lists, so the work table is complete here; only the
-  // gathered rows and their scales are waited for (by the producer and the epilogue warps).
+  // gathered rows and their scales are waited for (by the producer and the epilogue warps).  Where one kernel does it all
+  // (front_kernel) a word in p.meta says that the table is there.
   // Behind the pair kernel (tails) there is nothing to wait for: every CTA of that kernel has waited for the gather
   // before it let this one start, and the two share no output; waiting for its end would leave SMs idle.
   if (MODE == 1 && !SPLIT && !p.tails) pdl_wait();
-  pdl_trigger();
+  if (!FRONT) pdl_trigger();
+  auto wait_tables = [&]() {
+    const long long t0 = clock64();
+    while (ld_acquire_gpu(p.meta + kMetaTables) == 0) {
+      if (clock64() - t0 > p.wait_limit) { *s_abort = kStatusDependencyTimeout; return false; }
+    }
+    return true;
+  };
   // the work table and the two counters every role needs, fetched in one round trip
   if (MODE == 1 && NT == kTailTile && p.tails) {
     if (warp == 2) {        // this kernel's own table: the tails of the experts, and the prefix sums of their tiles
@@ -376,15 +386,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       if (lane == 31) { s_meta[0] = incl; s_meta[1] = __popc(active); }
     }
   } else if (threadIdx.x >= 64 && threadIdx.x < 64 + kMaxLocalExperts) {
+    if (FRONT) wait_tables();
     const int e = threadIdx.x - 64;
     s_work[e] = (e < p.e_local) ? p.work[e] : ExpertWork{0, 0, 0, 0};
   } else if (threadIdx.x == 64 + kMaxLocalExperts) {
-    s_meta[0] = p.meta[0];                          // token tiles
+    const bool there = !FRONT || wait_tables();
+    s_meta[0] = there ? p.meta[0] : 0;              // token tiles
     s_meta[1] = p.meta[3];                          // active experts
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (FRONT) pdl_trigger();   // (only now: the kernel that clears the word in p.meta comes after every kernel that reads it)
   const uint32_t tmem_base = *s_tmem;
   const Schedule sched = make_schedule<FT, SPLIT>(s_meta[0]);
   const int my_items = sched.items();
@@ -990,16 +1003,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 #endif
 }
 
-template <int MODE, int NT>
+template <int MODE, int NT, bool FRONT = false>
 cudaError_t launch_gemm(const GemmLaunch& g, const GemmArgs& a, int num_sms, cudaStream_t st) {
-  return launch_dependent(grouped_gemm_kernel<MODE, NT>, dim3(num_sms), dim3(Cfg<MODE, NT>::kThreads),
+  return launch_dependent(grouped_gemm_kernel<MODE, NT, FRONT>, dim3(num_sms), dim3(Cfg<MODE, NT>::kThreads),
                           static_cast<size_t>(Cfg<MODE, NT>::kSmemBytes), st, g.tm_w, g.tm_b, g.tm_bs, g.tm_sc,
                           g.tm_part, a);
 }
 
-template <int MODE, int NT>
+template <int MODE, int NT, bool FRONT = false>
 cudaError_t set_smem_attr() {
-  return cudaFuncSetAttribute(grouped_gemm_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(grouped_gemm_kernel<MODE, NT, FRONT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               Cfg<MODE, NT>::kSmemBytes);
 }
 
@@ -1008,6 +1021,8 @@ cudaError_t set_smem_attr() {
 cudaError_t gemm_set_attributes() {
   cudaError_t e;
   if ((e = set_smem_attr<1, 32>()) != cudaSuccess) return e;
+  if ((e = set_smem_attr<1, 32, true>()) != cudaSuccess) return e;
+  if ((e = set_smem_attr<2, 32, true>()) != cudaSuccess) return e;
   if ((e = set_smem_attr<1, 64>()) != cudaSuccess) return e;
   if ((e = set_smem_attr<1, 128>()) != cudaSuccess) return e;
   if ((e = set_smem_attr<2, 32>()) != cudaSuccess) return e;
@@ -1020,6 +1035,7 @@ cudaError_t launch_gemm1(const GemmLaunch& g, const float* w13_scale, int e_loca
   GemmArgs a{g.w_packed, ws.work, ws.meta, ws.a_scale, w13_scale, ws.c_hi, ws.c_lo, ws.c_scale, ws.o_rows, ws.row_cap, e_local,
              ws.ready, ws.parts_done, ws.status, ws.trace, ws.trace + 6 * 4096, g.wait_limit, g.silent_producer, g.tails, nullptr};
   if (g.token_tile == 128) return launch_gemm<1, 128>(g, a, num_sms, st);
+  if (g.front) return launch_gemm<1, 32, true>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<1, 32>(g, a, num_sms, st) : launch_gemm<1, 64>(g, a, num_sms, st);
 }
 
@@ -1029,6 +1045,7 @@ cudaError_t launch_gemm2(const GemmLaunch& g, const float* w2_scale, int e_local
              ws.ready, nullptr, ws.status, ws.trace + 3 * 4096, ws.trace + 7 * 4096, g.wait_limit, g.silent_producer, 0,
              g.rows_to_targets ? ws.row_out : nullptr};
   if (g.token_tile == 128) return launch_gemm<2, 128>(g, a, num_sms, st);
+  if (g.front) return launch_gemm<2, 32, true>(g, a, num_sms, st);
   return g.token_tile == 32 ? launch_gemm<2, 32>(g, a, num_sms, st) : launch_gemm<2, 64>(g, a, num_sms, st);
 }
 

@@ -36,8 +36,10 @@ enum : int {
 
 // Device-side control block (one int array); the GEMM kernels read the tile count from it.
 //   meta[0] = number of token tiles, meta[1] = padded row total, meta[2] = routed (token, local expert) rows,
-//   meta[3] = active local experts
+//   meta[3] = active local experts, meta[kMetaTables] = 1 while the tables of a call that launch_front() began are valid
 constexpr int kMetaInts = 8;
+constexpr int kMetaTables = 4;
+constexpr int kFrontMaxTokens = 16;   // batches that launch_front() takes
 
 // Per local expert: its rows [row_off, row_off + rows_pad) of the permuted row space
 // (rows_pad is a multiple of 16) cut into `tiles` token tiles of the launch's tile size;
@@ -99,6 +101,7 @@ struct GemmLaunch {
   CUtensorMap tm_sc;   // GEMM2: c_scale as f32 [16, row_cap], box 16 x token_tile (one load per work item)
   const uint8_t* w_packed = nullptr;   // pre-packed weights (tm_w unused) or nullptr
   int token_tile;      // 32, 64 or 128: token rows per work item, must match the row-list kernel's
+  int front = 0;       // launch_front() made the tables (32-row token tile): wait for meta[kMetaTables]
   int tails = 0;       // GEMM1 behind the pair kernel: only the rows tail_rows() leaves to it (token_tile = kTailTile)
   long long wait_limit = 1ll << 32;   // SM clocks a device-side wait may take (about two seconds)
   int silent_producer = 0;            // test hook, see syfi_moe_debug_fault
@@ -156,6 +159,10 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // launchers (each returns the cudaGetLastError() of its launches)
 cudaError_t launch_router(const float* logits, const void* bias_bf16, int T, int e_local, int expert_offset,
                           float scaling, const Workspace& ws, bool counters_are_zero, cudaStream_t st);
+// router, row lists and gather in one launch, for T <= kFrontMaxTokens; the GEMMs must be launched with `front` set
+cudaError_t launch_front(const float* logits, const void* bias_bf16, const uint8_t* hidden, const float* hidden_scale, int T,
+                         int e_local, int expert_offset, float scaling, int token_tile, const Workspace& ws, int num_sms,
+                         cudaStream_t st);
 cudaError_t launch_build_rows(int T, int e_local, int expert_offset, int token_tile, const Workspace& ws,
                               cudaStream_t st);
 cudaError_t launch_gather(const uint8_t* hidden, const float* hidden_scale, int T, const Workspace& ws, int num_sms,

@@ -1,4 +1,4 @@
-// DeepSeek-V3 no-aux router, one warp per token.
+// DeepSeek-V3 no-aux router, one warp per token; for small batches fused with the row lists and the gather.
 //
 // Replaces the reference's route_kernel (moe/solution/cuda/moe.cu:62-188: one CTA of
 // 256 threads per token, eight block-wide argmax rounds).  Here a warp owns a token:
@@ -26,16 +26,10 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, int T, int e_local,
-             int expert_offset, float scaling, int* __restrict__ topk_idx, float* __restrict__ topk_w,
-             uint32_t* __restrict__ local_mask, int* __restrict__ route_row, int* __restrict__ counts) {
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  pdl_trigger();
-  if (t >= T) return;
+// Routes token t, one warp: lane k < 8 ends with the token's k-th expert and its weight.
+__device__ __forceinline__ void route_token(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, int t,
+                                            float scaling, int lane, int& my_idx, float& w) {
   const unsigned full = 0xffffffffu;
-
   float x[8];
   {
     const float4* lp = reinterpret_cast<const float4*>(logits + static_cast<size_t>(t) * kExpertsGlobal + lane * 8);
@@ -88,7 +82,7 @@ route_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__
   for (int i = 0; i < 8; ++i) v[i] = keep ? v[i] : -CUDART_MAX_NORMAL_F;
 
   // eight rounds of warp-wide argmax over the kept experts
-  int my_idx = 0;
+  my_idx = 0;
   float my_s = 0.0f;
 #pragma unroll 1
   for (int r = 0; r < kTopK; ++r) {
@@ -124,18 +118,153 @@ route_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__
 #pragma unroll
   for (int d = 4; d >= 1; d >>= 1) sum += __shfl_xor_sync(full, sum, d);
   sum = __shfl_sync(full, sum, 0);
-  const float w = (my_s / (sum + 1e-20f)) * scaling;
+  w = (my_s / (sum + 1e-20f)) * scaling;
+}
 
+// bit e of the token's mask: one of its routes is local expert e
+__device__ __forceinline__ uint32_t local_experts(int my_idx, int lane, int e_local, int expert_offset) {
   const int le = my_idx - expert_offset;
-  const bool local = (lane < kTopK) && le >= 0 && le < e_local;
-  const uint32_t mask = __reduce_or_sync(full, local ? (1u << le) : 0u);
+  return __reduce_or_sync(0xffffffffu, lane < kTopK && le >= 0 && le < e_local ? (1u << le) : 0u);
+}
+
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+route_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, int T, int e_local,
+             int expert_offset, float scaling, int* __restrict__ topk_idx, float* __restrict__ topk_w,
+             uint32_t* __restrict__ local_mask, int* __restrict__ route_row, int* __restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  const int t = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  pdl_trigger();
+  if (t >= T) return;
+  int my_idx;
+  float w;
+  route_token(logits, bias, t, scaling, lane, my_idx, w);
+  const uint32_t mask = local_experts(my_idx, lane, e_local, expert_offset);
   if (lane < kTopK) {
     topk_idx[t * kTopK + lane] = my_idx;
     topk_w[t * kTopK + lane] = w;
     route_row[t * kTopK + lane] = -1;
-    if (local) atomicAdd(&counts[le], 1);
+    const int le = my_idx - expert_offset;
+    if (le >= 0 && le < e_local) atomicAdd(&counts[le], 1);
   }
   if (lane == 0) local_mask[t] = mask;
+}
+
+// Router, row lists and gather of a small batch in one launch.  The three kernels are a chain of dependent round trips
+// in front of GEMM1's first weight load.  Here EVERY CTA routes all tokens, a warp per token, and derives the row lists
+// from the masks in shared memory, so no CTA waits for another; the first one also writes the tables, and the gather's
+// rows are dealt over the CTAs.  GEMM1 may start when the tables are written: that is what meta[kMetaTables] says, set
+// with a release here, cleared by the combine kernel of the same call.
+// Bound by the latency of one token's routing (eight dependent rounds) as long as an SM's schedulers hold few of them:
+// us per call, three kernels -> this one: 1 token 49.6 -> 47.6, 5 tokens 94.8 -> 93.3, 16 tokens 91.0 -> 90.2; with up to
+// 64 tokens (two per warp of 32) 32 took 117.7 -> 118.5 and 64 took 118.1 -> 123.5, hence the limit of 16.
+constexpr int kFrontThreads = 32 * kFrontMaxTokens;
+constexpr int kFrontRows = kFrontMaxTokens * kTopK + kRowPad * kMaxLocalExperts;
+constexpr int kRowVecs = kHidden / 16;                    // 448
+static_assert(kFrontMaxTokens <= 32, "an expert's tokens are one word");
+static_assert(kFrontMaxTokens <= kRowPad, "an expert's padded rows are written in one go");
+static_assert(kRowVecs + kHBlocks <= kFrontThreads, "a row and its scales at a time");
+
+__global__ void __launch_bounds__(kFrontThreads)
+front_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, const uint8_t* __restrict__ hidden,
+             const float* __restrict__ hidden_scale, int T, int e_local, int expert_offset, float scaling, int token_tile,
+             const Workspace ws) {
+  __shared__ uint32_t s_mask[32];                               // local experts of a token
+  __shared__ int s_idx[kFrontMaxTokens * kTopK];
+  __shared__ uint32_t s_bits[kMaxLocalExperts];                 // tokens of an expert
+  __shared__ int s_off[kMaxLocalExperts];
+  __shared__ int s_token[kFrontRows];
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool first = blockIdx.x == 0;
+  if (tid < 32) s_mask[tid] = 0;
+  __syncthreads();
+  if (warp < T) {
+    int my_idx;
+    float w;
+    route_token(logits, bias, warp, scaling, lane, my_idx, w);
+    const uint32_t mask = local_experts(my_idx, lane, e_local, expert_offset);
+    if (lane < kTopK) s_idx[warp * kTopK + lane] = my_idx;
+    if (lane == 0) s_mask[warp] = mask;
+    if (first) {
+      if (lane < kTopK) {
+        ws.topk_idx[warp * kTopK + lane] = my_idx;
+        ws.topk_w[warp * kTopK + lane] = w;
+      }
+      if (lane == 0) ws.local_mask[warp] = mask;
+    }
+  }
+  __syncthreads();
+  for (int e = warp; e < kMaxLocalExperts; e += kFrontThreads / 32) {
+    const uint32_t b = __ballot_sync(full, ((s_mask[lane] >> e) & 1u) != 0);
+    if (lane == 0) s_bits[e] = b;
+  }
+  __syncthreads();
+  // lane e of every warp: expert e's rows, tiles and their prefix sums (as in build_rows_kernel)
+  const int cnt = __popc(s_bits[lane]);
+  const int pad = (cnt + kRowPad - 1) / kRowPad * kRowPad;
+  const int tiles = (pad + token_tile - 1) / token_tile;
+  int rows_incl = pad, tiles_incl = tiles;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int r = __shfl_up_sync(full, rows_incl, d), tl = __shfl_up_sync(full, tiles_incl, d);
+    if (lane >= d) { rows_incl += r; tiles_incl += tl; }
+  }
+  const int rows_total = __shfl_sync(full, rows_incl, 31), tiles_total = __shfl_sync(full, tiles_incl, 31);
+  const bool fits = rows_total <= ws.row_cap;    // else: refuse to write out of bounds
+  if (first && warp == 0) {
+    const int routed = __reduce_add_sync(full, cnt);
+    const int active = __popc(__ballot_sync(full, cnt > 0));
+    ws.ready[lane] = 0;
+    ws.counts_last[lane] = cnt;
+    ws.counts[lane] = 0;                         // other calls' routers count into these
+    if (fits && lane < e_local) ws.work[lane] = ExpertWork{rows_incl - pad, pad, tiles_incl - tiles, tiles};
+    if (lane == 0) {
+      if (!fits) atomicExch(ws.status, kStatusBadIndex);
+      ws.meta[0] = fits ? tiles_total : 0;
+      ws.meta[1] = fits ? rows_total : 0;
+      ws.meta[2] = fits ? routed : 0;
+      ws.meta[3] = fits ? active : 0;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();                           // the whole warp's tables (cumulative over the barrier above)
+      st_release_gpu(ws.meta + kMetaTables, 1);
+    }
+  }
+  if (warp == 1) s_off[lane] = rows_incl - pad;
+  pdl_trigger();
+  if (!fits) {
+    if (first)
+      for (int i = tid; i < T * kTopK; i += kFrontThreads) ws.route_row[i] = -1;
+    return;
+  }
+  for (int e = warp; e < kMaxLocalExperts; e += kFrontThreads / 32) {   // rows of expert e, padding rows carry token -1
+    const int off = __shfl_sync(full, rows_incl - pad, e), c = __shfl_sync(full, cnt, e), cp = __shfl_sync(full, pad, e);
+    const uint32_t b = s_bits[e];
+    if ((b >> lane) & 1u) s_token[off + __popc(b & ((1u << lane) - 1u))] = lane;
+    if (lane >= c && lane < cp) s_token[off + lane] = -1;
+  }
+  __syncthreads();
+  if (first) {
+    for (int i = tid; i < T * kTopK; i += kFrontThreads) {
+      const int t = i / kTopK, le = s_idx[i] - expert_offset;
+      ws.route_row[i] = le >= 0 && le < e_local ? s_off[le] + __popc(s_bits[le] & ((1u << t) - 1u)) : -1;
+    }
+    for (int r = tid; r < rows_total; r += kFrontThreads) ws.row_token[r] = s_token[r];
+  }
+  for (int i = blockIdx.x * kFrontThreads + tid; i < tiles_total * kIBlocks; i += gridDim.x * kFrontThreads) ws.parts_done[i] = 0;
+  // threads 0..447: a row's bytes, 448..503: its scales
+  for (int r = blockIdx.x; r < rows_total; r += gridDim.x) {
+    const int t = s_token[r];
+    if (tid < kRowVecs) {
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (t >= 0) v = __ldg(reinterpret_cast<const uint4*>(hidden + static_cast<size_t>(t) * kHidden) + tid);
+      reinterpret_cast<uint4*>(ws.a_perm + static_cast<size_t>(r) * kHidden)[tid] = v;
+    } else if (tid < kRowVecs + kHBlocks) {
+      const int kb = tid - kRowVecs;
+      ws.a_scale[static_cast<size_t>(kb) * ws.row_cap + r] = t >= 0 ? __ldg(hidden_scale + static_cast<size_t>(kb) * T + t) : 0.0f;
+    }
+  }
 }
 
 }  // namespace
@@ -153,6 +282,17 @@ cudaError_t launch_router(const float* logits, const void* bias_bf16, int T, int
   route_kernel<<<blocks, kWarpsPerBlock * 32, 0, st>>>(logits, static_cast<const __nv_bfloat16*>(bias_bf16), T,
                                                       e_local, expert_offset, scaling, ws.topk_idx, ws.topk_w,
                                                       ws.local_mask, ws.route_row, ws.counts);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_front(const float* logits, const void* bias_bf16, const uint8_t* hidden, const float* hidden_scale, int T,
+                         int e_local, int expert_offset, float scaling, int token_tile, const Workspace& ws, int num_sms,
+                         cudaStream_t st) {
+  // at most this many rows: every route one, and an expert's padding
+  const int rows = kTopK * T + kRowPad * (e_local < kTopK * T ? e_local : kTopK * T);
+  const int grid = rows < num_sms ? rows : num_sms;
+  front_kernel<<<grid, kFrontThreads, 0, st>>>(logits, static_cast<const __nv_bfloat16*>(bias_bf16), hidden, hidden_scale, T,
+                                               e_local, expert_offset, scaling, token_tile, ws);
   return cudaGetLastError();
 }
 

@@ -293,6 +293,45 @@ def test_rows_per_expert_at_the_edges_of_the_work_split(rows, pkg, oracle, monke
         assert torch.equal(outs[0], o)
 
 
+@pytest.mark.parametrize("T,E,off", [(1, 1, 255), (2, 32, 64), (15, 3, 32), (16, 32, 0), (17, 32, 0)])
+def test_small_batches_equal_the_same_tokens_in_a_larger_one(T, E, off, pkg):
+    """Up to 16 tokens the router, the row lists and the gather are one kernel: routes, weights, the tables and every
+    token's output are those of the first tokens of a larger batch, which takes the three kernels."""
+    big = pkg.make_inputs(num_tokens=40, seed=23, e_local=E, local_expert_offset=off, device=DEV)
+    big.routing_logits[:, off: off + E] += 1.5                # some routes for every expert slice
+    ctx = pkg.get_context(0)
+    ref, _ = _run(pkg, big)
+    ref_idx, ref_w = ctx.last_routing(T)
+    a = big.args()
+    small = pkg.MoeInputs(a[0][:T].contiguous(), a[1], a[2][:T].contiguous(), a[3][:, :T].contiguous(), *a[4:])
+    for _ in range(2):                                        # the second call finds the first one's tables
+        out, stats = _run(pkg, small)
+        idx, w = ctx.last_routing(T)
+        assert torch.equal(idx, ref_idx) and torch.equal(w, ref_w)
+        assert torch.equal(out, ref[:T])
+        local = (idx >= off) & (idx < off + E)
+        counts = torch.bincount((idx[local] - off).long(), minlength=32)
+        pad = (counts + 15) // 16 * 16
+        assert stats["routes"] == int(local.sum()) and stats["padded_rows"] == int(pad.sum())
+        assert stats["active_experts"] == int((counts > 0).sum())
+        row_token, _ = ctx.debug_read("row_token", torch.int32)
+        route_row, _ = ctx.debug_read("route_row", torch.int32)
+        want = []
+        for e in range(E):
+            toks = torch.nonzero((idx == e + off).any(1)).squeeze(1).tolist()
+            want += toks + [-1] * (int(pad[e]) - len(toks))
+        assert row_token[:len(want)].tolist() == want
+        rows = route_row[: T * 8].view(T, 8)
+        assert bool((rows[~local] == -1).all())
+        assert torch.equal(row_token[rows[local].long()].long(), torch.nonzero(local)[:, 0])
+        assert torch.equal(ctx.debug_read("counts", torch.int32)[0][:32].long(), counts)
+        want = torch.tensor(want, dtype=torch.long)
+        a_perm, _ = ctx.debug_read("a_perm", torch.uint8, max_bytes=len(want) * 7168)
+        got = a_perm.view(len(want), 7168)
+        assert torch.equal(got[want >= 0], small.hidden_states.cpu().view(torch.uint8)[want[want >= 0]])
+        assert not got[want < 0].any()
+
+
 def _swizzled_tiles(x):
     """x: [..., 128 rows, 8 chunks, 16 bytes] -> chunk c of row r moved to chunk c ^ (r & 7)."""
     r = torch.arange(128, device=x.device)[:, None]
