@@ -610,10 +610,6 @@ struct Scratch {
   float* scores = nullptr;
   size_t floats = 0;
   int* status = nullptr;
-  // the last few tensor maps: they depend on an address and a row count only, which a serving loop repeats
-  struct Map { const void* base = nullptr; uint64_t rows = 0; CUtensorMap map; };
-  Map maps[8];
-  int next_map = 0;
   bool checked = false;
   int num_sms = 0;
 };
@@ -673,20 +669,9 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
         !raise(dsa_select_kernel<16, false>, kSelectSmem) || !raise(dsa_select_kernel<0, true>, kSelectSmem))
       return fail(SYFI_DSA_ERR_CUDA, "cannot raise the shared-memory limit of the indexer's kernels");
   }
-  auto map_of = [&s](const void* base, uint64_t rows) -> const CUtensorMap* {
-    for (const Scratch::Map& m : s.maps)
-      if (m.base == base && m.rows == rows) return &m.map;
-    Scratch::Map& m = s.maps[s.next_map];
-    m.base = nullptr;
-    if (!rows128_map(&m.map, base, rows)) return nullptr;
-    m.base = base;
-    m.rows = rows;
-    s.next_map = (s.next_map + 1) % 8;
-    return &m.map;
-  };
-  const CUtensorMap* tm_q = map_of(q_index_fp8, static_cast<uint64_t>(batch) * kHeads);
-  const CUtensorMap* tm_k = map_of(k_index_cache_fp8, static_cast<uint64_t>(num_pages) * kPageRows);
-  if (!tm_q || !tm_k)
+  CUtensorMap tm_q, tm_k;
+  if (!rows128_map(&tm_q, q_index_fp8, static_cast<uint64_t>(batch) * kHeads) ||
+      !rows128_map(&tm_k, k_index_cache_fp8, static_cast<uint64_t>(num_pages) * kPageRows))
     return fail(SYFI_DSA_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   // Tiles per score CTA: as few as keep a few waves of CTAs (four to five fit an SM) in flight by the table's width;
   // a short table is a matter of latency, where each tile more in a CTA's chain is about half a microsecond.
@@ -694,7 +679,7 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   const int per_cta = tiles <= 1024 ? 1 : tiles <= 4096 ? 2 : tiles <= 12288 ? 4 : kMaxTilesPerCta;
   const int runs = (max_ls + per_cta * kTokTile - 1) / (per_cta * kTokTile);
   uint2* ranges = reinterpret_cast<uint2*>(s.scores + n_scores);
-  if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, *tm_q, *tm_k,
+  if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, tm_q, tm_k,
                        static_cast<const uint8_t*>(k_index_cache_fp8), weights, seq_lens, block_table, max_pages,
                        s.scores, max_ls, per_cta, ranges, s.status) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "score kernel launch failed");
