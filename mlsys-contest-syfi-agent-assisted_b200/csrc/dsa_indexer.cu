@@ -676,7 +676,9 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   // Tiles per score CTA: as few as keep a few waves of CTAs (four to five fit an SM) in flight by the table's width;
   // a short table is a matter of latency, where each tile more in a CTA's chain is about half a microsecond.
   const int64_t tiles = static_cast<int64_t>(batch) * ((max_ls + kTokTile - 1) / kTokTile);
-  const int per_cta = tiles <= 1024 ? 1 : tiles <= 4096 ? 2 : tiles <= 12288 ? 4 : kMaxTilesPerCta;
+  // us per call with 1 / 2 / 4 / 8 tiles: 8 sequences (4096 tiles) 38.4 / 26.8 / 23.7 / 24.7, 24 (6144) 42.3 / 28.5 / 23.3 /
+  // 24.2, 16 (8192) 63.9 / 44.0 / 37.8 / 37.5, 40 (20480) 114.7 / 66.2 / 46.0 / 40.0.
+  const int per_cta = tiles <= 1024 ? 1 : tiles <= 2048 ? 2 : tiles <= 12288 ? 4 : kMaxTilesPerCta;
   const int runs = (max_ls + per_cta * kTokTile - 1) / (per_cta * kTokTile);
   uint2* ranges = reinterpret_cast<uint2*>(s.scores + n_scores);
   if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, tm_q, tm_k,
