@@ -229,7 +229,10 @@ const void* mapped_alias(const void* host) {
 // Batches from this size on use the CTA-pair GEMM kernels, with GEMM1's small remainders on the single-CTA kernel.
 // Against 64-row tiles alone, us per call, two seeds: 3072 tokens 459 / 387 and 482 / 372, 4096 tokens 523 / 435 and
 // 570 / 467, 8192 tokens 870 / 829 and 1030 / 958.
+// That is with 32 local experts.  With fewer there are fewer tiles, and pairs pay off later: 8 experts, 64-row tiles / pairs,
+// 3600 tokens 156 / 167 and 94 / 104, 4500 tokens 193 / 177 and 103 / 113, from 6144 on the pairs.
 constexpr int64_t kPairMinTokens = 3584;
+constexpr int64_t kPairMinTokensAnyExperts = 6144;
 constexpr int64_t kWideListMinTokens = 6144;   // from here on the row lists of the pair configuration count 128-row tiles
 constexpr int kFlagOutF32 = 1;      // run_layer flags
 constexpr int kFlagPrepacked = 2;
@@ -297,7 +300,8 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   // Large batches (experts with hundreds of rows each) run the CTA-pair kernels, which cut their own
   // token tiles (256 rows in GEMM1, 128 in GEMM2), and the 64-row GEMM1 on what tail_rows() leaves to it;
   // token_tile 256 stands for that configuration here.
-  int token_tile = (T64 <= 1024) ? 32 : (T64 < kPairMinTokens || packed) ? 64 : 256;
+  const bool many = T64 >= kPairMinTokensAnyExperts || T64 * e_local >= kPairMinTokens * kMaxLocalExperts;
+  int token_tile = (T64 <= 1024) ? 32 : (!many || packed) ? 64 : 256;
   if (const char* ov = getenv("SYFI_MOE_TOKEN_TILE")) {   // tuning knob: force 32, 64, 128 or (pair kernels) 256
     const int v = atoi(ov);
     if (v == 32 || v == 64 || v == 128 || (v == 256 && !packed)) token_tile = v;
