@@ -30,6 +30,8 @@ extern "C" {
  *   weights            f32 [batch, 64]
  *   seq_lens           int32 [batch]
  *   block_table        int32 [batch, max_pages]: cache page of every 64 tokens of a sequence
+ *                      (a negative entry within a sequence's length: its positions rank behind all others, in
+ *                      order of position, and come back as -1)
  *   topk_indices       int32 [batch, 2048] (output)
  * Work is enqueued on `stream` (a cudaStream_t) of the CURRENT device; the call does not synchronise.  A scratch
  * buffer of batch * max_pages * 64 floats per device is kept by the library and grows on demand.  Returns

@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "../../include/syfi_dsa.h"
+#include "dsa_bins.h"
 #include "moe_internal.h"
 #include "ptx.cuh"
 
@@ -50,12 +51,6 @@ constexpr int kScoreSmem = 1024 + kScoreStages * kTokTile * kDim + kHeads * kDim
 constexpr int kSelectThreads = 1024;
 constexpr long long kWaitLimit = 1ll << 31;   // SM clocks (about a second)
 constexpr int kStatusScoreTimeout = 201;
-
-// larger float <-> larger key (NaN aside); key 0 is below every score
-__device__ __forceinline__ uint32_t score_key(float s) {
-  const uint32_t u = __float_as_uint(s);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 
 // Score kernel: CTA (x, b) scores the x-th run of tiles_per_cta * 128 tokens of sequence b, 128 at a time, through a two-deep
 // ring of key tiles in shared memory and two accumulators in tensor memory: while the four epilogue warps turn
@@ -148,6 +143,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int tl = tid;                        // 0..127
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
     uint32_t low = 0xffffffffu, high = 0u;     // range of this thread's scores, for the selection's bins
+    bool alive = true;
     for (int i = 0; i < tiles; ++i) {
       const int st = i % kScoreStages;
       const uint32_t ph = (i / kScoreStages) & 1u;
@@ -158,7 +154,11 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float scale = valid ? __ldg(reinterpret_cast<const float*>(cache + static_cast<size_t>(page) * kPageBytes +
                                                                        kPage * kDim + (tl & (kPage - 1)) * 4))
                                 : 0.0f;
-      if (!mbar_wait_bounded(&tfull[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit)) break;
+      if (!mbar_wait_bounded(&tfull[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit)) {
+        // the rest of the run gets no score, see below
+        for (int r = t; r < n && r < t_begin + tiles * kTokTile; r += kTokTile) scores[static_cast<size_t>(b) * max_ls + r] = -INFINITY;
+        break;
+      }
       tc_fence_after();
       float acc = 0.0f;
 #pragma unroll
@@ -178,6 +178,8 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         scores[static_cast<size_t>(b) * max_ls + t] = acc;
         low = min(low, score_key(acc));
         high = max(high, score_key(acc));
+      } else if (t < n) {                      // no page here: below every score and outside the range, so that the
+        scores[static_cast<size_t>(b) * max_ls + t] = -INFINITY;   // selection never meets what an earlier call left behind
       }
     }
     low = __reduce_min_sync(0xffffffffu, low);
@@ -308,21 +310,12 @@ __device__ __forceinline__ void select_best(Get get, int per_thread, int k, unsi
   __syncthreads();
 }
 
-constexpr int kBins = 4096;        // value bins of one sequence: a score's bin is linear in the score
 constexpr int kMaxInBin = 512;     // most items a bin at or above the cut may hold, see dsa_select_kernel
 constexpr int kMaxCluster = 8;     // CTAs that share a sequence
 constexpr int kMaxListed = kKeep + kMaxInBin;
 constexpr int kTablePages = 2048;  // block-table entries kept in shared memory
 constexpr int kSelectSmem = 2 * kMaxListed * 8 + kBins * 4 + kTablePages * 4;
 static_assert(kMaxListed * 8 >= kBins * 4 && kKeep * 8 <= kBins * 4, "aliases of the selection's buffers");
-
-__device__ __forceinline__ float key_score(uint32_t key) {   // inverse of score_key
-  return __uint_as_float((key & 0x80000000u) ? (key ^ 0x80000000u) : ~key);
-}
-// rounding is monotone, so a larger score never has a smaller bin
-__device__ __forceinline__ int score_bin(float s, float lowest, float scale) {
-  return min(kBins - 1, static_cast<int>((s - lowest) * scale));
-}
 
 // Selection and sort in one pass over the scores: a counting sort by value.  A cluster of CTAs shares a sequence, CTA r
 // takes every gridDim.x-th block of 1024 positions (PER blocks at most, kept in registers; PER = 0: any number, read
@@ -502,7 +495,8 @@ dsa_select_kernel(const float* __restrict__ scores, const uint2* __restrict__ ra
 
   auto token = [&](unsigned long long item) {
     const int pos = static_cast<int>(~static_cast<uint32_t>(item)), page = pos / kPage;
-    return (page < kTablePages ? s_table[page] : table[page]) * kPage + pos % kPage;
+    const int cache_page = page < kTablePages ? s_table[page] : table[page];
+    return cache_page < 0 ? -1 : cache_page * kPage + pos % kPage;
   };
   if (cut >= 0) {
     if (joint) {

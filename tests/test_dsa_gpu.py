@@ -126,6 +126,34 @@ def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
         assert torch.equal(out[b, :k].long(), tb[best // 64] * 64 + best % 64), (b, n)
 
 
+@pytest.mark.parametrize("lens,table_pages,absent", [
+    ([3000, 700, 64], 128, [1, 5, 6]),           # one CTA per sequence; the third has no page at all
+    ([30000, 5000], 512, [0, 7, 77, 78, 79]),    # a cluster
+    ([140000], 2200, [3, 1000, 2187]),           # scores read again in every sweep
+])
+def test_indexer_ranks_absent_pages_last(lens, table_pages, absent, pkg):
+    """A negative table entry has no keys: its positions are worse than all others and come back as -1.  The call
+    before leaves other scores in the scratch buffer, which must not be met again."""
+    from oracle import dsa_oracle
+    q, cache, w, sl, table = (t.to(DEV) for t in dsa_oracle.make_inputs(lens, seed=5))
+    table = torch.nn.functional.pad(table, (0, table_pages - table.shape[1]))
+    _run(pkg, (q, cache, w * 1e6, sl, table))
+    before = _run(pkg, (q, cache, w, sl, table))
+    holes = table.clone()
+    for b, n in enumerate(lens):
+        pages = [p for p in absent if p < (n + 63) // 64] if b < 2 else list(range((n + 63) // 64))
+        holes[b, pages] = torch.tensor([-1 - 70 * p for p in pages], dtype=torch.int32, device=DEV)
+    out = _run(pkg, (q, cache, w, sl, holes))
+    for b, n in enumerate(lens):
+        pos = torch.arange(n, device=DEV)
+        left = int((holes[b].long()[pos // 64] >= 0).sum())
+        k = min(2048, left)
+        assert bool((out[b, k:] == -1).all())
+        gone = set((table[b].long()[pos // 64] * 64 + pos % 64)[holes[b].long()[pos // 64] < 0].tolist())
+        kept = [t for t in before[b].tolist() if t >= 0 and t not in gone]
+        assert out[b, :min(k, len(kept))].tolist() == kept[:k]
+
+
 def test_indexer_argument_validation(pkg):
     from oracle import dsa_oracle
     q, cache, w, sl, table = (t.to(DEV) for t in dsa_oracle.make_inputs([100], seed=1))
