@@ -33,9 +33,13 @@ extern "C" {
  *                      (a negative entry within a sequence's length: its positions rank behind all others, in
  *                      order of position, and come back as -1)
  *   topk_indices       int32 [batch, 2048] (output)
- * Work is enqueued on `stream` (a cudaStream_t) of the CURRENT device; the call does not synchronise.  A scratch
- * buffer of batch * max_pages * 64 floats per device is kept by the library and grows on demand.  Returns
- * SYFI_DSA_OK or an error code; syfi_moe_last_error() (syfi_moe.h) has the message.  The reference checks nothing
+ * Work is enqueued on `stream` (a cudaStream_t) of the CURRENT device; the call does not synchronise.  Calls on
+ * different streams may run at the same time: every stream has a scratch buffer of its own of about 65 floats
+ * per table entry, which grows on demand (that waits for the device).  Up to eight streams of a device hold one; a
+ * ninth waits for the device and takes over the least recently used.  A captured graph keeps using the buffer that its
+ * stream had then: do not replay two graphs captured on one stream at the same time, nor beside calls on that stream;
+ * and where more than eight streams call, capture after a call of the same size, and replay beside no other call.
+ * Returns SYFI_DSA_OK or an error code; syfi_moe_last_error() (syfi_moe.h) has the message.  The reference checks nothing
  * (dsa_topk_indexer.cu:476-494). */
 int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_index_cache_fp8, const float* weights,
                           const int32_t* seq_lens, const int32_t* block_table, int32_t batch, int64_t num_pages,

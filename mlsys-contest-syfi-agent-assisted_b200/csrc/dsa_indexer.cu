@@ -599,18 +599,102 @@ cudaError_t launch_select(const float* scores, const uint2* ranges, int runs, in
   return c16 == 1 ? run(launch_select_as<16, false>, 1) : run(launch_select_as<16, true>, c16);
 }
 
-// per-device scratch: the scores of every token of every sequence with their ranges, and a status word
+// The scores of every token of every sequence with their ranges, one buffer per stream: calls on one stream follow each
+// other, calls on two may run at the same time.  A stream is known by its id, which is never given out twice (a handle
+// may be, after the stream was destroyed); a stream that is being captured cannot be asked for it and is known by its
+// handle.
 struct Scratch {
+  cudaStream_t handle = nullptr;
+  unsigned long long id = 0; // 0: not known yet
+  uint64_t last_use = 0;     // 0: free
   float* scores = nullptr;
   size_t floats = 0;
+  bool captured = false;     // a graph may use it
+};
+constexpr int kMaxScratch = 8;   // streams of a device that hold one at a time; the next one takes over the least recently used
+
+struct Device {
+  Scratch scratch[kMaxScratch];
+  uint64_t calls = 0;
   int* status = nullptr;
   bool checked = false;
   int num_sms = 0;
 };
 std::mutex g_mu;
-Scratch g_scratch[64];
+Device g_devices[64];
 
 int fail(int code, const char* msg) { return set_last_error(code, msg); }
+
+// Allocation must not end a capture that is going on, on this stream or another.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// The stream's buffer of at least `need` floats; null with the error code in *rc when there is none.
+Scratch* scratch_of(Device& d, cudaStream_t st, size_t need, int* rc) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();   // the default stream beside a capture: the launch will say so
+  const bool capturing = capture != cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (!capturing && cudaStreamGetId(st, &id) != cudaSuccess) {
+    *rc = fail(SYFI_DSA_ERR_CUDA, "not a stream of the current device");
+    return nullptr;
+  }
+  // The stream's own; of two (below) the larger.
+  Scratch *s = nullptr, *spare = nullptr;
+  for (Scratch& c : d.scratch) {
+    if (c.last_use == 0) spare = &c;
+    else if ((capturing || c.id == 0 ? c.handle == st : c.id == id) && (!s || c.floats > s->floats)) s = &c;
+  }
+  if (s && s->floats < need && (capturing || s->captured) && spare) s = nullptr;   // a graph keeps the small one
+  if (capturing && !spare && (!s || s->floats < need)) {
+    // Nothing may wait now, so nothing can be freed: whichever is large enough, as if the two streams were one.
+    s = nullptr;
+    for (Scratch& c : d.scratch)
+      if (c.floats >= need && (!s || c.last_use < s->last_use)) s = &c;
+    if (!s) *rc = fail(SYFI_DSA_ERR_CUDA, "no scratch buffer is large enough, and none can be had during a capture");
+    else s->captured = true;
+    return s;
+  }
+  if (!s) {
+    s = spare;
+    if (!s) {   // the one that was not used for longest, of those that no graph needs, if there is one
+      for (Scratch& c : d.scratch)
+        if (!s || (c.captured != s->captured ? s->captured : c.last_use < s->last_use)) s = &c;
+      if (cudaDeviceSynchronize() != cudaSuccess) {
+        *rc = fail(SYFI_DSA_ERR_CUDA, "device synchronisation failed");
+        return nullptr;
+      }
+    }
+    s->handle = st;
+    s->id = 0;
+    s->captured = false;
+  }
+  if (need > s->floats) {
+    if (s->scores) {
+      if (cudaDeviceSynchronize() != cudaSuccess) {
+        *rc = fail(SYFI_DSA_ERR_CUDA, "device synchronisation failed");
+        return nullptr;
+      }
+      cudaFree(s->scores);
+    }
+    s->scores = nullptr;
+    s->floats = 0;
+    RelaxedCapture relaxed;
+    if (cudaMalloc(&s->scores, need * sizeof(float)) != cudaSuccess) {
+      s->last_use = 0;
+      *rc = fail(SYFI_DSA_ERR_CUDA, "out of device memory for the scores");
+      return nullptr;
+    }
+    s->floats = need;
+  }
+  if (id != 0) s->id = id;
+  if (capturing) s->captured = true;
+  s->last_use = ++d.calls;
+  return s;
+}
 
 }  // namespace
 
@@ -633,28 +717,23 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int max_ls = max_pages * kPage;
   std::lock_guard<std::mutex> lock(g_mu);
-  Scratch& s = g_scratch[dev];
-  if (!s.checked) {     // once per device: the attribute queries cost more than the kernels
+  Device& d = g_devices[dev];
+  if (!d.checked) {     // once per device: the attribute queries cost more than the kernels
     int major = 0;
     if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess || major != 10 ||
-        cudaDeviceGetAttribute(&s.num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaDeviceGetAttribute(&d.num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return fail(SYFI_DSA_ERR_CUDA, "this library is built for sm_100a (B200) only");
-    s.checked = true;
+    d.checked = true;
   }
   // scores, and a score range per 128 tokens at most (a multiple of 64 floats before it)
   const size_t n_scores = static_cast<size_t>(batch) * max_ls;
   const size_t need = n_scores + 2 * static_cast<size_t>(batch) * ((max_ls + kTokTile - 1) / kTokTile);
-  if (need > s.floats) {
-    if (cudaDeviceSynchronize() != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "device synchronisation failed");
-    if (s.scores) cudaFree(s.scores);
-    s.scores = nullptr;
-    s.floats = 0;
-    if (cudaMalloc(&s.scores, need * sizeof(float)) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "out of device memory for the scores");
-    s.floats = need;
-  }
-  if (!s.status) {
-    if (cudaMalloc(&s.status, 16) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "out of device memory");
-    cudaMemset(s.status, 0, 16);
+  int rc = SYFI_DSA_OK;
+  Scratch* const s = scratch_of(d, st, need, &rc);
+  if (!s) return rc;
+  if (!d.status) {
+    if (cudaMalloc(&d.status, 16) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "out of device memory");
+    cudaMemset(d.status, 0, 16);
     auto raise = [](auto* kernel, int bytes) {
       return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
@@ -674,13 +753,13 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   // 24.2, 16 (8192) 63.9 / 44.0 / 37.8 / 37.5, 40 (20480) 114.7 / 66.2 / 46.0 / 40.0.
   const int per_cta = tiles <= 1024 ? 1 : tiles <= 2048 ? 2 : tiles <= 12288 ? 4 : kMaxTilesPerCta;
   const int runs = (max_ls + per_cta * kTokTile - 1) / (per_cta * kTokTile);
-  uint2* ranges = reinterpret_cast<uint2*>(s.scores + n_scores);
+  uint2* ranges = reinterpret_cast<uint2*>(s->scores + n_scores);
   if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, tm_q, tm_k,
                        static_cast<const uint8_t*>(k_index_cache_fp8), weights, seq_lens, block_table, max_pages,
-                       s.scores, max_ls, per_cta, ranges, s.status) != cudaSuccess)
+                       s->scores, max_ls, per_cta, ranges, d.status) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "score kernel launch failed");
-  if (launch_select(s.scores, ranges, runs, per_cta * kTokTile, max_ls, seq_lens, block_table, batch, max_pages,
-                    topk_indices, s.num_sms, st) != cudaSuccess)
+  if (launch_select(s->scores, ranges, runs, per_cta * kTokTile, max_ls, seq_lens, block_table, batch, max_pages,
+                    topk_indices, d.num_sms, st) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "select kernel launch failed");
   return SYFI_DSA_OK;
 }
@@ -691,12 +770,12 @@ extern "C" int syfi_dsa_check(void* stream) {
   if (cudaStreamSynchronize(static_cast<cudaStream_t>(stream)) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "stream synchronisation failed");
   std::lock_guard<std::mutex> lock(g_mu);
-  Scratch& s = g_scratch[dev];
-  if (!s.status) return SYFI_DSA_OK;
+  Device& d = g_devices[dev];
+  if (!d.status) return SYFI_DSA_OK;
   int status = 0;
-  if (cudaMemcpy(&status, s.status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "cannot read the status word");
+  if (cudaMemcpy(&status, d.status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return fail(SYFI_DSA_ERR_CUDA, "cannot read the status word");
   if (status != 0) {
-    cudaMemset(s.status, 0, sizeof(int));
+    cudaMemset(d.status, 0, sizeof(int));
     char msg[128];
     snprintf(msg, sizeof(msg), "a kernel reported status %d (201: a bounded wait in the score kernel ran out)", status);
     return fail(SYFI_DSA_ERR_DEVICE, msg);

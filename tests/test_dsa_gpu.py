@@ -154,6 +154,48 @@ def test_indexer_ranks_absent_pages_last(lens, table_pages, absent, pkg):
         assert out[b, :min(k, len(kept))].tolist() == kept[:k]
 
 
+@pytest.mark.parametrize("streams", [2, 10])        # ten: more than hold a scratch buffer at a time
+def test_indexer_calls_on_several_streams_at_once(streams, pkg):
+    """Every stream's call has scores of its own: the outputs are those of the calls one after the other."""
+    from oracle import dsa_oracle
+    sets = [tuple(t.to(DEV) for t in dsa_oracle.make_inputs([20000 + 64 * i, 900, 9000], seed=20 + i)) for i in range(streams)]
+    want = [_run(pkg, s) for s in sets]
+    outs = [torch.full_like(w, -7) for w in want]
+    side = [torch.cuda.Stream() for _ in range(streams)]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, stream, out in zip(sets, side, outs):
+            with torch.cuda.stream(stream):
+                pkg.run_dsa_topk_indexer(*s, out)
+    torch.cuda.synchronize()
+    pkg.dsa_check()
+    for w, out in zip(want, outs):
+        assert torch.equal(w, out)
+
+
+def test_indexer_graph_beside_calls_on_other_streams(pkg):
+    """A graph captured on a stream that never ran a call keeps its own scores, also while other streams call, and a
+    larger call on another stream leaves its buffer alone."""
+    from oracle import dsa_oracle
+    a, b, c = (tuple(t.to(DEV) for t in dsa_oracle.make_inputs(lens, seed=31 + len(lens))) for lens in ([12000, 70], [9000], [40000, 3, 20000]))
+    want = [_run(pkg, x) for x in (a, b, c)]
+    outs = [torch.full_like(w, -7) for w in want]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        pkg.run_dsa_topk_indexer(*a, outs[0])
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(10):
+        graph.replay()
+        with torch.cuda.stream(other):
+            pkg.run_dsa_topk_indexer(*b, outs[1])
+            pkg.run_dsa_topk_indexer(*c, outs[2])
+    torch.cuda.synchronize()
+    pkg.dsa_check()
+    for w, out in zip(want, outs):
+        assert torch.equal(w, out)
+
+
 def test_indexer_argument_validation(pkg):
     from oracle import dsa_oracle
     q, cache, w, sl, table = (t.to(DEV) for t in dsa_oracle.make_inputs([100], seed=1))
