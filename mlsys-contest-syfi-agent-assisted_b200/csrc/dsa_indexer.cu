@@ -49,6 +49,7 @@ constexpr int kScoreThreads = 160;            // four epilogue warps (one tensor
 constexpr int kScoreStages = 2;
 constexpr int kScoreSmem = 1024 + kScoreStages * kTokTile * kDim + kHeads * kDim;   // slack + key tiles + query tile
 constexpr int kSelectThreads = 1024;
+constexpr int kMaxCluster = 8;                // select CTAs that share a sequence
 constexpr long long kWaitLimit = 1ll << 31;   // SM clocks (about a second)
 constexpr int kStatusScoreTimeout = 201;
 
@@ -200,38 +201,61 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (tid == 0 && s_abort != 0) atomicExch(status, s_abort);
 }
 
-// The best min(2048, n) of n items, best first, left in s_item[0 .. 2047] (zeros behind them); one CTA.  An item is
-// (order-preserving key of the score << 32) | ~position, so items are distinct, "larger" means "better score, then
-// lower position", and the cut is one exact item value: an 8-pass radix select over the 64 bits (one byte per
-// pass, a histogram in shared memory filled through warp-aggregated increments, since most scores of a sequence
-// share their top bytes), a compaction of the items at or above the cut, and a bitonic sort.
-// get(j) returns the calling thread's j-th item (j < per_thread), 0 where it has none.
-template <typename Get>
-__device__ __forceinline__ void select_best(Get get, int per_thread, int k, unsigned long long* s_item,
-                                            unsigned long long* s_swap, int* s_hist, int* s_misc) {
+// The best k = min(2048, n) of a sequence's n items, best first, left in the first CTA's s_item[0 .. 2047] (zeros behind
+// them); all `ctas` CTAs that share the sequence call it, each for its own items.  An item is (order-preserving key of the
+// score << 32) | ~position, so items are distinct, "larger" means "better score, then lower position", and the cut is one
+// exact item value: an 8-pass radix select over the 64 bits (one byte per pass, a histogram in shared memory, the top
+// bytes' through warp-aggregated increments, since most scores of a sequence share those), a compaction of the items at
+// or above the cut, and in the first CTA a bitonic sort.  In a pass every CTA counts its own items, and all of them sum
+// the CTAs' 256 counts and so come to the same byte; two histograms in turn need one cluster barrier per pass.
+// get(j) returns the calling thread's j-th item, 0 where it has none; j < N, or any j, with per_thread of them, where N is 0.
+template <int N, typename Get>
+__device__ __forceinline__ void select_best(Get get, int per_thread, int k, int ctas, int rank, unsigned long long* s_item,
+                                            unsigned long long* s_swap, int* s_arrived, int (*s_hist)[256], int* s_misc) {
+  cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < kKeep; i += kSelectThreads) s_item[i] = 0ull;
+  auto each = [&](auto f) {
+    if constexpr (N > 0) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f(get(j));
+    } else {
+      for (int j0 = 0; j0 < per_thread; j0 += 4) {      // four loads in flight
+        unsigned long long it[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) it[j] = get(j0 + j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f(it[j]);
+      }
+    }
+  };
   unsigned long long prefix = 0ull, mask = 0ull;
   int want = k;
   for (int shift = 56; shift >= 0; shift -= 8) {
-    if (tid < 256) s_hist[tid] = 0;
+    int* const hist = s_hist[(shift >> 3) & 1];
+    if (tid < 256) hist[tid] = 0;
     __syncthreads();
-    for (int j = 0; j < per_thread; ++j) {
-      const unsigned long long it = get(j);
+    each([&](unsigned long long it) {
       const int bin = (it != 0ull && (it & mask) == prefix) ? static_cast<int>((it >> shift) & 255ull) : 256;
       if (shift >= 48) {      // sign and exponent: a handful of values, so the warp adds up its lanes first
         const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        if (bin < 256 && lane == __ffs(peers) - 1) atomicAdd(&s_hist[bin], __popc(peers));
+        if (bin < 256 && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], __popc(peers));
       } else if (bin < 256) { // mantissa and position bytes: spread out, and fewer items match the prefix each pass
-        atomicAdd(&s_hist[bin], 1);
+        atomicAdd(&hist[bin], 1);
       }
-    }
-    __syncthreads();
+    });
+    if (ctas > 1) cluster.sync();
+    else __syncthreads();
     // the byte value at which the count from the top reaches `want`: thread t < 256 owns value 255 - t, an
     // inclusive scan in thread order counts the items with that byte or a larger one
     int h = 0, incl = 0;
     if (tid < 256) {
-      h = s_hist[255 - tid];
+      if (ctas > 1) {
+#pragma unroll
+        for (int c = 0; c < kMaxCluster; ++c)
+          if (c < ctas) h += cluster.map_shared_rank(hist, c)[255 - tid];
+      } else {
+        h = hist[255 - tid];
+      }
       incl = h;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -260,24 +284,35 @@ __device__ __forceinline__ void select_best(Get get, int per_thread, int k, unsi
   const unsigned long long cut = prefix;       // the k-th best item (its leading bytes, when the passes stopped early)
   if (tid == 0) s_misc[2] = 0;
   __syncthreads();
-  for (int j = 0; j < per_thread; ++j) {     // one counter increment per warp and round, not per winner
-    const unsigned long long it = get(j);
+  each([&](unsigned long long it) {            // one counter increment per warp and round, not per winner
     const bool win = it != 0ull && it >= cut;
     const unsigned winners = __ballot_sync(0xffffffffu, win);
     int base = 0;
     if (lane == 0 && winners != 0u) base = atomicAdd(&s_misc[2], __popc(winners));
     base = __shfl_sync(0xffffffffu, base, 0);
     if (win) s_item[base + __popc(winners & ((1u << lane) - 1u))] = it;
+  });
+  __syncthreads();
+  unsigned long long *buf = s_swap, *other = s_item;
+  if (ctas > 1) {                              // every CTA's winners in one piece to the first one
+    const int own = s_misc[2];
+    if (tid == 0) s_misc[0] = atomicAdd(cluster.map_shared_rank(s_arrived, 0), own);
+    __syncthreads();
+    unsigned long long* to = cluster.map_shared_rank(s_swap, 0) + s_misc[0];
+    for (int i = tid; i < own; i += kSelectThreads) to[i] = s_item[i];
+    cluster.sync();
+    if (rank != 0) return;
+    buf = s_item;
+    other = s_swap;
   }
+  for (int i = k + tid; i < kKeep; i += kSelectThreads) other[i] = 0ull;
   __syncthreads();
   // Bitonic sort, descending, two adjacent items per thread in registers.  A compare-exchange at distance d pairs
   // item i with item i ^ d: d = 1 is inside the thread, d = 2 .. 32 pairs this thread with lane ^ (d / 2) of its
   // warp (shuffles, no barrier), d >= 64 goes through shared memory (two buffers in turn: one barrier per stage,
   // 15 stages instead of 66 barriers).  The first of a pair keeps the larger item where the block of `size`
   // items it lies in is sorted downwards ((i & size) == 0), the smaller one otherwise.
-  unsigned long long e0 = s_item[2 * tid], e1 = s_item[2 * tid + 1];
-  unsigned long long* buf = s_swap;
-  unsigned long long* other = s_item;
+  unsigned long long e0 = other[2 * tid], e1 = other[2 * tid + 1];
   auto pick = [](unsigned long long a, unsigned long long c, bool keep_max) {
     return keep_max ? (a > c ? a : c) : (a < c ? a : c);
   };
@@ -311,7 +346,6 @@ __device__ __forceinline__ void select_best(Get get, int per_thread, int k, unsi
 }
 
 constexpr int kMaxInBin = 512;     // most items a bin at or above the cut may hold, see dsa_select_kernel
-constexpr int kMaxCluster = 8;     // CTAs that share a sequence
 constexpr int kMaxListed = kKeep + kMaxInBin;
 constexpr int kTablePages = 2048;  // block-table entries kept in shared memory
 constexpr int kSelectSmem = 2 * kMaxListed * 8 + kBins * 4 + kTablePages * 4;
@@ -334,10 +368,14 @@ static_assert(kMaxListed * 8 >= kBins * 4 && kKeep * 8 <= kBins * 4, "aliases of
 // a 66-stage bitonic sort per 16384 positions, then the same again over the chunks' candidates, took 25 us for three
 // short sequences and 22 + 32 us for 32 sequences of 65536 tokens; this one takes 6 and 12 us.
 // Where the bins do not separate the scores (a bin at or above the cut holds more than kMaxInBin items: ties, or
-// outliers that stretch the range; infinities and NaNs), the first CTA runs that radix select and sort over the whole
-// sequence instead.  Both orders are exact: by score key, then by position.
+// outliers that stretch the range; infinities and NaNs), the cluster selects by radix instead, see select_best: us per
+// call, separable scores / one outlier per sequence / the same with the first CTA alone on the whole sequence:
+// 1 sequence of 65536 tokens 19 / 39 / 124, 32 of them 58 / 87 / 177, 1 of 262144 35 / 93 / 475, of 1048576 78 / 244 / 1700.
+// Both orders are exact: by score key, then by position.
+// PER = 0 keeps to 32 registers, so that two CTAs fit an SM: 32 sequences of 140000 tokens take 113 us per call, 130 with
+// the 56 registers the compiler takes when it may.
 template <int PER, bool CLUSTER>
-__global__ void __launch_bounds__(kSelectThreads)
+__global__ void __launch_bounds__(kSelectThreads, PER == 0 ? 2 : 1)
 dsa_select_kernel(const float* __restrict__ scores, const uint2* __restrict__ ranges, int runs, int run_len, int max_ls,
                   const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ block_table, int max_pages,
                   int32_t* __restrict__ out) {
@@ -353,7 +391,7 @@ dsa_select_kernel(const float* __restrict__ scores, const uint2* __restrict__ ra
   __shared__ int s_cut[3];              // cut bin (-1: the bins do not separate the scores), candidate, items at or above it
   __shared__ int s_own, s_base;         // items this CTA has collected, their place in the first CTA's s_in
   __shared__ int s_arrived;             // first CTA: items in s_in
-  __shared__ int s_radix[256], s_misc[12];
+  __shared__ int s_radix[2][256], s_misc[12];
   cg::cluster_group cluster = cg::this_cluster();
   const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = CLUSTER ? static_cast<int>(blockIdx.x) : 0;
@@ -467,61 +505,61 @@ dsa_select_kernel(const float* __restrict__ scores, const uint2* __restrict__ ra
     cut = s_cut[0];
   }
 
-  // 4. the items at or above the cut bin, grouped by bin
   auto item_of = [](float s, int i) {
     return (static_cast<unsigned long long>(score_key(s)) << 32) | static_cast<uint32_t>(~i);
   };
-  auto bin_of = [&](unsigned long long it) { return score_bin(key_score(static_cast<uint32_t>(it >> 32)), lowest, scale); };
-  if (cut >= 0) {
-    if (rank == 0) {
-      sweep([&](float s, int i) {
-        const int bin = score_bin(s, lowest, scale);
-        if (bin >= cut) s_item[atomicAdd(&s_cursor[bin], 1)] = item_of(s, i);
-      });
-    } else {
-      sweep([&](float s, int i) {
-        if (score_bin(s, lowest, scale) >= cut) s_item[atomicAdd(&s_own, 1)] = item_of(s, i);
-      });
-      __syncthreads();
-      if (tid == 0 && s_own > 0) s_base = atomicAdd(cluster.map_shared_rank(&s_arrived, 0), s_own);
-      __syncthreads();
-      unsigned long long* in = cluster.map_shared_rank(s_in, 0) + s_base;
-      for (int i = tid; i < s_own; i += kSelectThreads) in[i] = s_item[i];
-    }
-  }
-  if (joint) cluster.sync();     // also keeps the first CTA's shared memory until the others are through with it
-  else __syncthreads();
-  if (rank != 0) return;
-
   auto token = [&](unsigned long long item) {
     const int pos = static_cast<int>(~static_cast<uint32_t>(item)), page = pos / kPage;
     const int cache_page = page < kTablePages ? s_table[page] : table[page];
     return cache_page < 0 ? -1 : cache_page * kPage + pos % kPage;
   };
-  if (cut >= 0) {
-    if (joint) {
-      for (int i = tid; i < s_arrived; i += kSelectThreads) {
-        const unsigned long long it = s_in[i];
-        s_item[atomicAdd(&s_cursor[bin_of(it)], 1)] = it;
-      }
-      __syncthreads();
-    }
-    // 5. a bin's cursor now stands at the first rank of the next lower bin
-    for (int i = tid; i < s_cut[2]; i += kSelectThreads) {
-      const unsigned long long it = s_item[i];
-      const int bin = bin_of(it), end = s_cursor[bin];
-      int at = bin == kBins - 1 ? 0 : s_cursor[bin + 1];
-      int final_rank = at;
-#pragma unroll 4
-      for (; at < end; ++at) final_rank += s_item[at] > it;
-      if (final_rank < k) o[final_rank] = token(it);
-    }
+  if (cut < 0) {
+    select_best<PER>([&](int j) {
+      const int i = first + j * step;
+      return i < n ? item_of(PER > 0 ? mine[PER > 0 ? j : 0] : __ldg(sc + i), i) : 0ull;
+    }, (n + step - 1) / step, k, ctas, rank, s_item, reinterpret_cast<unsigned long long*>(s_cursor), &s_arrived, s_radix, s_misc);
+    if (rank != 0) return;
+    for (int i = tid; i < kKeep; i += kSelectThreads) o[i] = i < k ? token(s_item[i]) : -1;
+    return;
+  }
+
+  // 4. the items at or above the cut bin, grouped by bin
+  auto bin_of = [&](unsigned long long it) { return score_bin(key_score(static_cast<uint32_t>(it >> 32)), lowest, scale); };
+  if (rank == 0) {
+    sweep([&](float s, int i) {
+      const int bin = score_bin(s, lowest, scale);
+      if (bin >= cut) s_item[atomicAdd(&s_cursor[bin], 1)] = item_of(s, i);
+    });
   } else {
-    select_best([&](int j) {
-      const int i = j * kSelectThreads + tid;
-      return i < n ? item_of(__ldg(sc + i), i) : 0ull;
-    }, (n + kSelectThreads - 1) / kSelectThreads, k, s_item, reinterpret_cast<unsigned long long*>(s_cursor), s_radix, s_misc);
-    for (int i = tid; i < k; i += kSelectThreads) o[i] = token(s_item[i]);
+    sweep([&](float s, int i) {
+      if (score_bin(s, lowest, scale) >= cut) s_item[atomicAdd(&s_own, 1)] = item_of(s, i);
+    });
+    __syncthreads();
+    if (tid == 0 && s_own > 0) s_base = atomicAdd(cluster.map_shared_rank(&s_arrived, 0), s_own);
+    __syncthreads();
+    unsigned long long* in = cluster.map_shared_rank(s_in, 0) + s_base;
+    for (int i = tid; i < s_own; i += kSelectThreads) in[i] = s_item[i];
+  }
+  if (joint) cluster.sync();     // also keeps the first CTA's shared memory until the others are through with it
+  else __syncthreads();
+  if (rank != 0) return;
+
+  if (joint) {
+    for (int i = tid; i < s_arrived; i += kSelectThreads) {
+      const unsigned long long it = s_in[i];
+      s_item[atomicAdd(&s_cursor[bin_of(it)], 1)] = it;
+    }
+    __syncthreads();
+  }
+  // 5. a bin's cursor now stands at the first rank of the next lower bin
+  for (int i = tid; i < s_cut[2]; i += kSelectThreads) {
+    const unsigned long long it = s_item[i];
+    const int bin = bin_of(it), end = s_cursor[bin];
+    int at = bin == kBins - 1 ? 0 : s_cursor[bin + 1];
+    int final_rank = at;
+#pragma unroll 4
+    for (; at < end; ++at) final_rank += s_item[at] > it;
+    if (final_rank < k) o[final_rank] = token(it);
   }
   for (int i = k + tid; i < kKeep; i += kSelectThreads) o[i] = -1;
 }

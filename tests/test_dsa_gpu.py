@@ -79,6 +79,16 @@ def test_indexer_ties_and_determinism(pkg):
     ([140000, 9000], 2200, "zeros"),
     ([9000, 4000], 256, "outlier"),                      # one score stretches the range
     ([6000], 94, "nan"),
+    # no use for the bins: every CTA of the cluster selects among its own positions, the first one among those
+    ([8193, 20000, 9216], 512, "outlier"),               # two and four CTAs, some with 1024 positions
+    ([65536, 40000, 8000], 1024, "outlier"),             # eight
+    ([131072, 17000], 2048, "outlier"),                  # sixteen positions per thread
+    ([131073, 300000], 4700, "outlier"),                 # read again in every pass
+    ([65536, 30000], 1024, "zeros"),
+    ([30000, 5000], 512, "inf"),                         # the range is not finite
+    ([30000, 5000], 512, "nan_weight"),                  # every score of the first sequence is NaN
+    ([12000 + 9 * i for i in range(80)], 200, "spread"), # one CTA per sequence, sixteen positions per thread
+    ([12000 + 9 * i for i in range(80)], 200, "outlier"),
 ])
 def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
     """Every branch of the selection, with scores that both sides compute without a rounding difference: one head of
@@ -97,6 +107,12 @@ def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
     if kind == "outlier":
         scale[0, 0] = 1e7
         keys[0, 0] = q[0, 0]
+        scale[need[0], 0] = 1e7                          # and the second sequence's first token
+        keys[need[0], 0] = q[1, 0]
+    if kind == "inf":
+        q[:, 1:] = 0                                     # (a weight of zero times infinity would be NaN)
+        scale[0, 0] = float("inf")
+        keys[0, 0] = q[0, 0]
     if kind == "nan":
         scale[0, 0] = float("nan")
     cache = torch.empty(pages, 64 * 132, dtype=torch.uint8, device=DEV)
@@ -104,7 +120,9 @@ def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
     cache[:, 8192:] = scale.view(torch.uint8)
     w = torch.zeros(B, 64, device=DEV)
     w[:, 0] = 1.0
-    perm = torch.arange(pages, device=DEV) if kind in ("outlier", "nan") else torch.randperm(pages, generator=g, device=DEV)
+    if kind == "nan_weight":
+        w[0, 1] = float("nan")
+    perm = torch.arange(pages, device=DEV) if kind in ("outlier", "inf", "nan") else torch.randperm(pages, generator=g, device=DEV)
     table = torch.zeros(B, table_pages, dtype=torch.int32, device=DEV)
     at = 0
     for b, n in enumerate(need):
@@ -121,7 +139,9 @@ def test_indexer_selection_is_exact(lens, table_pages, kind, pkg):
             continue
         tb = table[b].long()
         score = torch.relu((keys[tb[: need[b]]] @ q[b, 0]) * scale[tb[: need[b]]]).flatten()[:n]
-        score = torch.nan_to_num(score, nan=0.0)      # relu is a maximum with zero in the kernel: a NaN counts as zero
+        score = torch.nan_to_num(score, nan=0.0, posinf=float("inf"))      # relu is a maximum with zero in the kernel: a NaN counts as zero
+        if kind == "nan_weight" and b == 0:
+            score = torch.zeros_like(score)           # all the same: ties by position
         best = torch.sort(score, descending=True, stable=True).indices[:k]
         assert torch.equal(out[b, :k].long(), tb[best // 64] * 64 + best % 64), (b, n)
 
@@ -194,6 +214,37 @@ def test_indexer_graph_beside_calls_on_other_streams(pkg):
     pkg.dsa_check()
     for w, out in zip(want, outs):
         assert torch.equal(w, out)
+
+
+def _us_per_call(f, calls=20):
+    times = []
+    for _ in range(5):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        for _ in range(calls):
+            f()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end) * 1e3 / calls)
+    return min(times[1:])
+
+
+@pytest.mark.parametrize("length", [65536, 262144])
+def test_indexer_cost_without_bins_is_bounded(length, pkg):
+    """One outlier takes the bins' use away.  The selection that is left has to stay a matter of the whole cluster: 2.1
+    times (65536 tokens) and 2.7 times (262144) the call with separable scores were measured, 6.6 and 13.6 times when one
+    CTA read the whole sequence alone."""
+    from oracle import dsa_oracle
+    q, cache, w, sl, table = (t.to(DEV) for t in dsa_oracle.make_inputs([length], seed=3))
+    out = torch.empty(1, 2048, dtype=torch.int32, device=DEV)
+    plain = _us_per_call(lambda: pkg.run_dsa_topk_indexer(q, cache, w.abs(), sl, table, out))
+    stretched = cache.clone().view(-1, 64 * 132)
+    scales = stretched[int(table[0, 5]), 64 * 128:].view(torch.float32)
+    scales[7] *= 3e3
+    stretched = stretched.view(cache.shape)
+    outlier = _us_per_call(lambda: pkg.run_dsa_topk_indexer(q, stretched, w.abs(), sl, table, out))
+    assert int(out[0, 0]) == int(table[0, 5]) * 64 + 7
+    assert outlier < 4.5 * plain, (outlier, plain)
 
 
 def test_indexer_argument_validation(pkg):
