@@ -175,12 +175,11 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc = fmaf(s_w[c * 16 + j], fmaxf(__uint_as_float(r[j]) * scale, 0.0f), acc);
       }
+      // no page here: below every score and outside the range, so that the selection never meets what an earlier call left
+      if (t < n) scores[static_cast<size_t>(b) * max_ls + t] = valid ? acc : -INFINITY;
       if (valid) {
-        scores[static_cast<size_t>(b) * max_ls + t] = acc;
         low = min(low, score_key(acc));
         high = max(high, score_key(acc));
-      } else if (t < n) {                      // no page here: below every score and outside the range, so that the
-        scores[static_cast<size_t>(b) * max_ls + t] = -INFINITY;   // selection never meets what an earlier call left behind
       }
     }
     low = __reduce_min_sync(0xffffffffu, low);
@@ -568,22 +567,39 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
+typedef CUresult (*IsCapturingFn)(CUstream, CUstreamCaptureStatus*);
+typedef CUresult (*StreamIdFn)(CUstream, unsigned long long*);
+
+// Driver functions without a link to libcuda.  (The runtime has the two on streams as well; it takes 40 ns for each instead
+// of 11, and a short batch is bound by the host's part of the call.)
+struct Driver {
+  EncodeTiledFn encode_tiled = nullptr;
+  IsCapturingFn is_capturing = nullptr;
+  StreamIdFn stream_id = nullptr;
+};
+
+template <typename Fn>
+void driver_fn(const char* name, Fn* fn) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+    *fn = reinterpret_cast<Fn>(p);
+}
+
+const Driver& driver() {
+  static Driver d;
   static std::once_flag once;
   std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
+    driver_fn("cuTensorMapEncodeTiled", &d.encode_tiled);
+    driver_fn("cuStreamIsCapturing", &d.is_capturing);
+    driver_fn("cuStreamGetId", &d.stream_id);
   });
-  return fn;
+  return d;
 }
 
 // rows of 128 bytes, boxes of 64 rows, 128-byte swizzle
 bool rows128_map(CUtensorMap* m, const void* base, uint64_t rows) {
-  EncodeTiledFn fn = encode_fn();
+  const EncodeTiledFn fn = driver().encode_tiled;
   if (!fn) return false;
   const cuuint64_t dims[2] = {128, rows};
   const cuuint64_t strides[1] = {128};
@@ -672,11 +688,14 @@ struct RelaxedCapture {
 
 // The stream's buffer of at least `need` floats; null with the error code in *rc when there is none.
 Scratch* scratch_of(Device& d, cudaStream_t st, size_t need, int* rc) {
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();   // the default stream beside a capture: the launch will say so
-  const bool capturing = capture != cudaStreamCaptureStatusNone;
+  const Driver& drv = driver();
+  CUstreamCaptureStatus capture = CU_STREAM_CAPTURE_STATUS_NONE;
   unsigned long long id = 0;
-  if (!capturing && cudaStreamGetId(st, &id) != cudaSuccess) {
+  bool known = drv.is_capturing && drv.stream_id;
+  if (known && drv.is_capturing(st, &capture) != CUDA_SUCCESS) capture = CU_STREAM_CAPTURE_STATUS_NONE;   // the default stream beside a capture: the launch will say so
+  const bool capturing = capture != CU_STREAM_CAPTURE_STATUS_NONE;
+  if (known && !capturing) known = drv.stream_id(st, &id) == CUDA_SUCCESS;
+  if (!known) {
     *rc = fail(SYFI_DSA_ERR_CUDA, "not a stream of the current device");
     return nullptr;
   }
