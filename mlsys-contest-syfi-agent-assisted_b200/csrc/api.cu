@@ -333,13 +333,9 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     if ((rc = make_map(&ctx->p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128))) return rc;
   } else {
   if (!packed) {   // (packed tiles are fetched with untiled copies)
-    const int n_boxes = token_tile == 32 ? 4 : 1;
-    for (int i = 0; i < n_boxes; ++i) {
-      CUtensorMap* m1 = i == 0 ? &g1.tm_w : &g1.tm_part.m[i - 1];
-      CUtensorMap* m2 = i == 0 ? &g2.tm_w : &g2.tm_part.m[i - 1];
-      if ((rc = make_map3(m1, w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128 >> i))) return rc;
-      if ((rc = make_map3(m2, w2, e_local, kHidden, kInter, 1, 128 >> i))) return rc;
-    }
+    for (int i = 0; i < (token_tile == 32 ? 4 : 1); ++i)
+      if ((rc = make_map3(i == 0 ? &g1.tm_w : &g1.tm_part.m[i - 1], w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128 >> i))) return rc;
+    if ((rc = make_map3(&g2.tm_w, w2, e_local, kHidden, kInter, 1, 128))) return rc;
   }
   if ((rc = make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, token_tile))) return rc;
   if ((rc = make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16))) return rc;

@@ -88,8 +88,10 @@ template <int MODE, int NT> struct Cfg {
   // so a second issuer finds its one entry still being promoted and adds its polling to the hand-offs: at 64 rows two
   // issuers took 747 us where one takes 731 (4096 tokens, hot experts), 308.9 against 299.4 (2048 tokens).
   static constexpr int kIssuers = NT == 32 ? 2 : 1;
-  // The 32-row kernel cuts the items of a thin last round along the features (see Schedule).
-  static constexpr bool kSplit = NT == 32;
+  // The 32-row kernel requests its first weights before it waits for the token side.
+  static constexpr bool kEarly = NT == 32;
+  // The 32-row GEMM1 cuts the items of a thin last round along the features (see Schedule).
+  static constexpr bool kSplit = MODE == 1 && NT == 32;
 };
 
 struct GemmArgs {
@@ -154,10 +156,11 @@ template <int MODE, int NT, Kind KIND>
 struct Layout {
   using C = Cfg<MODE, NT>;
   static constexpr int kKps = KIND == kPartFew ? 4 : C::kKps;                      // K blocks per ring entry
-  static constexpr int kWPitch = KIND == kWhole ? (MODE == 1 ? C::kStageBytes : kATile) : (MODE == 1 ? kATile : kATile / 2);
+  static constexpr int kWPitch = KIND == kWhole && MODE == 1 ? C::kStageBytes : kATile;
   static constexpr int kBBase = KIND == kWhole ? (MODE == 1 ? 2 * kATile : kKps * kATile) : kKps * kWPitch;
   static constexpr int kBRows = (KIND == kPartFew ? 16 : NT) * (MODE == 1 ? 1 : 2);
   static constexpr int kBPitch = KIND == kWhole && MODE == 1 ? C::kStageBytes : kBRows * 128;
+  static_assert(KIND == kWhole || MODE == 1, "only GEMM1's items are cut");
   static_assert(KIND == kWhole || kBBase + kKps * kBRows * 128 <= C::kGroupBytes, "a part's K blocks fit the ring entry");
   static_assert(KIND == kWhole || (kKps - 1) * kWPitch + kATile <= C::kGroupBytes, "and the tile an MMA reads lies inside it");
   static_assert(C::kKBlocks % kKps == 0 && kKps % C::kTKps == 0, "whole steps");
@@ -181,25 +184,31 @@ struct Place {
 // The last round.  Fewer CTAs with equally many items each, when that costs at most a fifth of the SMs, finish sooner
 // than a last round that keeps only some SMs busy: a single SM draws at most 57 GB/s from HBM, 1.3x its fair share.
 // Failing that, when the last round's items occupy at most half of the SMs (with three active experts, a token or two,
-// GEMM1 has 48 items for 148 SMs), the 32-row kernel cuts each of them along its features into two, four or eight parts,
+// GEMM1 has 48 items for 148 SMs), the 32-row GEMM1 cuts each of them along its features into two, four or eight parts,
 // as many as there are SMs for: each of the round's CTAs gets one part.  (Runs of equal length over all CTAs,
 // whatever item boundaries they cross, were slower: a part costs a pass over K of its own, whose MMAs take the same time
 // for 16 features as for 64.)  Cutting along K instead (stream-K) would change the order of the sums; cutting features
-// changes no arithmetic.  In mode 1 the requantisation needs all 128 features: parts store their accumulators and
+// changes no arithmetic.  The requantisation needs all 128 features: parts store their accumulators and
 // whoever stores an item's last part finishes it; nobody waits.
+// us per call, whole / cut, for token tiles of 16 rows: 1 tile (16 items) 40.6 / 37.2, 3 (48) 47.5 / 44.9, 10 (148 + 12)
+// 94.1 / 90.1, 13 (148 + 60) 108.0 / 104.4, 20 (296 + 24) 156.6 / 151.3, 22 (296 + 56) 164.6 / 160.9.  A round of a few
+// items behind two or more whole ones is left as it is: GEMM2 works on the other SMs meanwhile (19 tiles, 296 + 8 items,
+// 141.5 / 150.1; 28 tiles, 444 + 4, 196.9 / 201.7).  GEMM2's items take 5 us, not 30: cutting its last round gained nothing
+// (1 tile 37.2 either way) and cost 1 us elsewhere.
 struct Schedule {
   int grid, cta, rounds;        // whole items of this CTA: cta + i * grid, i < rounds
-  int tail_first, parts;        // split last round: its first item, parts per item
+  int tail_first, parts;        // split last round: its first item, parts per item (1, 2, 4 or 8)
   int n_items;
   __device__ __forceinline__ int items() const { return n_items; }
-  template <int FT, int NT>
+  template <int FT, int NT, bool SPLIT>
   __device__ __forceinline__ Item item(const ExpertWork* s_work, int e_local, int i, Place& at) const {
     Item it{0, 0, 0, 0, 0, 0, 16};
     int w = cta + i * grid;
-    if (i >= rounds) {
-      w = tail_first + cta / parts;
-      const int part = cta % parts;
-      it.nu = 16 / parts;
+    if (SPLIT && i >= rounds) {
+      const int lg = 31 - __clz(parts);      // (with divisions by `parts` here and below, calls WITHOUT a split round took 1.5 % more)
+      w = tail_first + (cta >> lg);
+      const int part = cta & (parts - 1);
+      it.nu = 16 >> lg;
       it.u0 = part * it.nu;
     }
     for (int e = at.expert; e < e_local; ++e) {
@@ -230,10 +239,10 @@ __device__ __forceinline__ Schedule make_schedule(int token_tiles) {
   const int even = rounds > 0 ? (total + rounds - 1) / rounds : s.grid;   // CTAs needed for `rounds` items each
   if (even * 5 >= s.grid * 4) {
     s.grid = even;
-  } else if (SPLIT && rest * 2 <= s.grid) {
+  } else if (SPLIT && rest * 2 <= s.grid && !(full >= 2 && rest * 8 <= s.grid)) {
     s.rounds = full;
     s.tail_first = full * s.grid;
-    s.parts = s.grid / rest >= 8 ? 8 : s.grid / rest >= 4 ? 4 : 2;
+    s.parts = rest * 8 <= s.grid ? 8 : rest * 4 <= s.grid ? 4 : 2;
     s.n_items = full + (cta < rest * s.parts ? 1 : 0);
     return s;
   }
@@ -290,7 +299,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   constexpr int ISSUERS = C::kIssuers;
   constexpr int SUB = PAIRS / ISSUERS;    // each MMA issuer's share of them
   static_assert(PAIRS % ISSUERS == 0, "whole shares");
-  constexpr bool SPLIT = C::kSplit;
+  constexpr bool EARLY = C::kEarly;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -356,7 +365,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // (front_kernel) a word in p.meta says that the table is there.
   // Behind the pair kernel (tails) there is nothing to wait for: every CTA of that kernel has waited for the gather
   // before it let this one start, and the two share no output; waiting for its end would leave SMs idle.
-  if (MODE == 1 && !SPLIT && !p.tails) pdl_wait();
+  if (MODE == 1 && !EARLY && !p.tails) pdl_wait();
   if (!FRONT) pdl_trigger();
   auto wait_tables = [&]() {
     const long long t0 = clock64();
@@ -399,8 +408,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   tc_fence_after();
   if (FRONT) pdl_trigger();   // (only now: the kernel that clears the word in p.meta comes after every kernel that reads it)
   const uint32_t tmem_base = *s_tmem;
-  const Schedule sched = make_schedule<FT, SPLIT>(s_meta[0]);
+  const Schedule sched = make_schedule<FT, C::kSplit>(s_meta[0]);
   const int my_items = sched.items();
+
+  // The roles, in two versions: most calls have no split round, and the code for parts in the roles' loops would cost them
+  // 1 to 5 % (128 items 74.2 us per call with it, 72.5 without; 18 tiles of 6 experts 103 / 95).
+  auto roles = [&](auto split) {
+  constexpr bool SPLIT = decltype(split)::value;
+  using Whole = Layout<MODE, NT, kWhole>;
+  using Few = Layout<MODE, NT, SPLIT ? kPartFew : kWhole>;
+  using Part = Layout<MODE, NT, SPLIT ? kPart : kWhole>;
 
   // MMA issue, one thread of each of kIssuers warps; of two, one has the even ring entries, one the odd ones (fixed, so that either
   // sees every phase of its barriers: a parity wait for a phase whose predecessor is not over returns at once).  With the weights as the M operand an MMA takes
@@ -426,7 +443,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           const uint32_t d0 = tmem_base + (pr * TKPS + k2) * (2 * NT);
           const uint64_t a0 = umma_smem_desc_sw128(gb + k * L::kWPitch);
           const uint64_t b0 = umma_smem_desc_sw128(gb + L::kBBase + k * L::kBPitch);   // mode 2: hi rows, then lo rows
-          if constexpr (MODE == 1 && std::is_same<L, Layout<MODE, NT, kWhole>>::value) {
+          if constexpr (MODE == 1 && std::is_same<L, Whole>::value) {
             const uint64_t a1 = umma_smem_desc_sw128(gb + k * L::kWPitch + kATile);
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4) {
@@ -446,19 +463,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       return true;
     };
     for (int i = 0; i < my_items && alive; ++i) {
-      const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+      const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
       // Mode 2 issues ONE MMA of twice the loaded rows per 32 bytes of K over the adjacent hi and lo rows
       // (the columns past the tile's n rows hold other rows' data and are never read back)
       // instead of one per term; mode 1 needs two because up and gate are different A tiles.
       const uint32_t idesc = umma_idesc_e4m3_m128(MODE == 1 ? static_cast<uint32_t>(im.n) : im.n <= 16 ? 32u : 2u * NT);
       const Kind kind = kind_of<NT, SPLIT>(im);
-      const int steps = kind == kPartFew ? KB / Layout<MODE, NT, SPLIT ? kPartFew : kWhole>::kKps : KB / KPS;
+      const int steps = kind == kPartFew ? KB / Few::kKps : KB / KPS;
       for (int step = 0; step < steps; ++step) {
         if (ISSUERS == 1 || (g & 1u) == par) {
           if (!mbar_wait_bounded(&full[g], ph, s_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
           TRACE(1, step);
-          if (!SPLIT || kind == kWhole) alive = issue(Layout<MODE, NT, kWhole>{}, idesc);
-          else if constexpr (SPLIT) alive = kind == kPartFew ? issue(Layout<MODE, NT, kPartFew>{}, idesc) : issue(Layout<MODE, NT, kPart>{}, idesc);
+          if (!SPLIT || kind == kWhole) alive = issue(Whole{}, idesc);
+          else if constexpr (SPLIT) alive = kind == kPartFew ? issue(Few{}, idesc) : issue(Part{}, idesc);
           if (!alive) break;
         }
         if (++g == G) { g = 0; ph ^= 1u; }
@@ -478,16 +495,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       Place at;
       bool alive = true;
       for (int i = 0; i < my_items && alive; ++i) {
-        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+        const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
         const Kind kind = kind_of<NT, SPLIT>(im);
         // Tiles of at most 16 rows use the 16-row box: the token-side tiles come from L2 through the
         // same SM port as the weights, so every byte not fetched is bandwidth for the weight stream.
         const bool few = im.n <= 16;
         const CUtensorMap* mb = few ? &tm_bs : &tm_b;
         const CUtensorMap* mw = !SPLIT || im.nu == 16 ? &tm_w : im.nu == 8 ? &tm_part.m[0] : im.nu == 4 ? &tm_part.m[1] : &tm_part.m[2];
-        const uint32_t w_bytes = static_cast<uint32_t>(im.nu) * 1024;
-        const int wrow = im.ft * 128 + im.u0 * 8;
-        const int steps = kind == kPartFew ? KB / Layout<MODE, NT, SPLIT ? kPartFew : kWhole>::kKps : KB / KPS;
+        const uint32_t w_bytes = SPLIT ? static_cast<uint32_t>(im.nu) * 1024 : kATile;
+        const int wrow = im.ft * 128 + (SPLIT ? im.u0 * 8 : 0);
+        const int steps = kind == kPartFew ? KB / Few::kKps : KB / KPS;
         // arms ring entry g and loads the weight rows of a step into it (mode 1: up and gate rows in one box)
         auto load_w = [&](auto layout, int step) {
           using L = decltype(layout);
@@ -497,13 +514,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           const int kb0 = step * kKps;
           if (p.w_packed != nullptr) {
             constexpr int kPacked = (MODE == 1 ? 2 : 1) * kATile;   // packed bytes of a K block
-            const uint8_t* src = p.w_packed + (static_cast<size_t>(im.expert * FT + im.ft) * KB + kb0) * kPacked + im.u0 * 1024;
-            if constexpr (!std::is_same<L, Layout<MODE, NT, kWhole>>::value) {   // a run of 8-row groups is contiguous
+            const uint8_t* src = p.w_packed + (static_cast<size_t>(im.expert * FT + im.ft) * KB + kb0) * kPacked +
+                                 (SPLIT ? im.u0 * 1024 : 0);
+            if constexpr (!std::is_same<L, Whole>::value) {   // a run of 8-row groups is contiguous
 #pragma unroll
               for (int k = 0; k < kKps; ++k) {
                 bulk_load(st0 + k * L::kWPitch, src + static_cast<size_t>(k) * kPacked, w_bytes, &full[g], pol_w);
-                if (MODE == 1)
-                  bulk_load(st0 + k * L::kWPitch + w_bytes, src + static_cast<size_t>(k) * kPacked + kATile, w_bytes, &full[g], pol_w);
+                bulk_load(st0 + k * L::kWPitch + w_bytes, src + static_cast<size_t>(k) * kPacked + kATile, w_bytes, &full[g], pol_w);
               }
             } else if (MODE == 1) {     // 32 KB per K block: up tile, gate tile
 #pragma unroll
@@ -528,13 +545,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         };
         auto pick = [&](auto f) {       // f(layout of this item)
           if constexpr (SPLIT) {
-            if (kind == kPartFew) return f(Layout<MODE, NT, kPartFew>{});
-            if (kind == kPart) return f(Layout<MODE, NT, kPart>{});
+            if (kind == kPartFew) return f(Few{});
+            if (kind == kPart) return f(Part{});
           }
-          return f(Layout<MODE, NT, kWhole>{});
+          return f(Whole{});
         };
         int ahead = 0;                  // steps of this item whose weights are already on their way
-        if (SPLIT && i == 0) {
+        if (EARLY && i == 0) {
           // the ring's first fill needs the weights only: requested before what the token side waits for
           for (; ahead < G && ahead < steps; ++ahead) {
             pick([&](auto layout) { load_w(layout, ahead); });
@@ -620,7 +637,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       int done_target = 0;
       Place at;
       for (int i = 0; i < my_items; ++i) {
-        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+        const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
         done_target += 4 * C::kColSplit;
         const long long t0 = clock64();
         bool seen = true;
@@ -643,7 +660,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       int cleared = 0, ready_expert = -1;
       Place at;
       for (int i = 0; i < my_items; ++i) {
-        const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+        const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
         if (im.expert != ready_expert) {
           const int need = (kInter / 128) * s_work[im.expert].tiles;
           const long long t0 = clock64();
@@ -682,19 +699,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     int cached_row_start = -1;              // token tile whose activation scales sit in shared memory (mode 1)
     Place at;
     uint32_t sph = 0;                       // phase bits of sfull[0..2] (mode 2)
-    if (MODE == 1 && SPLIT) pdl_wait();     // the activation scales are the gather's
+    if (MODE == 1 && EARLY) pdl_wait();     // the activation scales are the gather's
     // After a failed wait a warp keeps walking the work list and still joins every named
     // barrier below (doing no other work), so the epilogue warps can never strand each other.
     for (int i = 0; i < my_items; ++i) {
-      const Item im = sched.item<FT, NT>(s_work, p.e_local, i, at);
+      const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
       const int ft = im.ft;
       const int n = ok ? im.n : 0;
       // which lanes carry a feature (see Layout)
       const int feats = im.nu * 8;
       const bool part = SPLIT && im.nu < 16;
       const int tl = q * 32 + lane;
-      const bool is_gate = MODE == 1 && part && tl >= feats;
-      const bool warp_used = !part || q * 32 < (MODE == 1 ? 2 * feats : feats);
+      const bool is_gate = part && tl >= feats;
+      const bool warp_used = !part || q * 32 < 2 * feats;
       const int lo_col = im.n <= 16 ? 16 : NT;                       // mode 2: where the lo products start
       if (et == 0) TRACE(2, 1000);
       float* s_act;
@@ -786,7 +803,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           const uint64_t ws1 = (MODE == 1) ? f32x2_pack(s_ws[64 + kb], s_ws[64 + kb]) : 0ull;
           const float* sa = s_act + kb * NT + c0;
           if (c0 < n && warp_used) {
-            if (MODE == 1 && part) {
+            if (part) {
               uint32_t r0[16];
               tmem_ld16(t0, r0);
               tmem_ld_wait();
@@ -874,7 +891,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         for (int j = 0; j < CN / 2; ++j) f32x2_unpack(acc1p[j], acc1[2 * j], acc1[2 * j + 1]);
       }
 
-      if (MODE == 1 && part) {
+      if (part) {
         // ---- part of an item: the accumulators go to memory, whoever stores an item's last part finishes it
         const int f = is_gate ? tl - feats : tl;
         if (f < feats && c0 < n_out) {
@@ -969,7 +986,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       } else {
         const int qrow = lane & 3;
         const int row0 = im.row_start + c0 + qrow;
-        const int col = ft * 128 + im.u0 * 8 + q * 32 + (lane >> 2) * 4;
+        const int col = ft * 128 + q * 32 + (lane >> 2) * 4;
 #pragma unroll
         for (int j = 0; j < CN; j += 4) {
           if (c0 + j < n_out) {
@@ -977,15 +994,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             quad_transpose_f32(a0, a1, a2, a3, lane);   // now: row c0 + j + qrow, four adjacent features
             // expert parallelism: the row's place in its token owner's memory (plain stores over NVLink)
             float* o = p.row_out != nullptr ? p.row_out[row0 + j] : p.o_rows + static_cast<size_t>(row0 + j) * kHidden;
-            if (o != nullptr && (!part || q * 32 + (lane >> 2) * 4 < feats))
-              *reinterpret_cast<float4*>(o + col) = make_float4(a0, a1, a2, a3);
+            if (o != nullptr) *reinterpret_cast<float4*>(o + col) = make_float4(a0, a1, a2, a3);
           }
         }
       }
     }
   }
 
-  if (MODE == 1 && SPLIT) pdl_wait();   // no CTA ends before the gather has (kernels behind this one rely on it)
+  };
+  if (C::kSplit && sched.parts > 1) roles(std::integral_constant<bool, C::kSplit>{});
+  else roles(std::false_type{});
+
+  if (MODE == 1 && EARLY) pdl_wait();   // no CTA ends before the gather has (kernels behind this one rely on it)
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -97,7 +97,7 @@ struct GemmLaunch {
   CUtensorMap tm_w;    // weights, box 128 rows
   CUtensorMap tm_b;    // token side, box token_tile rows
   CUtensorMap tm_bs;   // token side, box 16 rows: tiles of <= 16 rows pull half the bytes
-  PartMaps tm_part;    // weights, smaller boxes (32-row token tile only)
+  PartMaps tm_part;    // weights, smaller boxes (32-row GEMM1 only)
   CUtensorMap tm_sc;   // GEMM2: c_scale as f32 [16, row_cap], box 16 x token_tile (one load per work item)
   const uint8_t* w_packed = nullptr;   // pre-packed weights (tm_w unused) or nullptr
   int token_tile;      // 32, 64 or 128: token rows per work item, must match the row-list kernel's

@@ -258,6 +258,7 @@ def test_every_token_tile_gives_the_same_bits(T, E, off, seed, pkg, oracle, monk
 @pytest.mark.parametrize("rows", [
     (1,), (16,), (17, 0, 32),                        # 32-row tiles, thin last round: eight, eight and four parts an item
     (5, 31, 16, 1), (33, 64, 2, 40, 18, 1, 70, 16),  # two parts; whole rounds in front of the split one
+    (16,) * 8 + (60,), (16,) * 12 + (200,),          # eight parts behind a whole round; eight items behind two, not cut
     (127, 128, 129, 130), (255, 256, 257, 0, 64, 65, 1, 144), (383, 384, 385, 400, 320, 321),   # remainders of 256 rows
 ])
 def test_rows_per_expert_at_the_edges_of_the_work_split(rows, pkg, oracle, monkeypatch):
