@@ -25,15 +25,17 @@ struct syfi_moe_ctx {
   // staging buffers of syfi_moe_forward_host
   void* stage = nullptr;
   size_t stage_bytes = 0;
-  // tensor maps of the last call: they only depend on the operand addresses, the expert count and
-  // the token tile, which rarely change between calls (re-encoding costs a few microseconds of host time)
+  // Tensor maps of the last call (encoding one takes a third of a microsecond of host time).  Those of the workspace's
+  // buffers depend on the workspace and the token tile; those of the weights on their addresses as well, and a model with
+  // several layers encodes these in every call.
   GemmLaunch g1, g2;
   PairGemmLaunch p1, p2;             // tensor maps of the CTA-pair kernels (large batches)
-  const void* map_w13 = nullptr;
+  bool ws_maps = false;              // the workspace's are those of map_token_tile
+  const void* map_w13 = nullptr;     // the weights' are those of these four; null: of none
   const void* map_w2 = nullptr;
-  const void* map_ws = nullptr;      // workspace generation the maps were built for (a_perm pointer)
   int map_e_local = 0, map_token_tile = 0;
   bool map_packed = false;
+  int maps_encoded = 0;              // by the last call (syfi_moe_debug_read)
   // true while the row counters of the workspace are known to be zero at the point of the next launch
   bool counters_clean = false;
   // second stream of syfi_moe_forward_host: the hidden states travel while the router runs
@@ -279,7 +281,7 @@ int ensure_capacity(syfi_moe_ctx* ctx, int64_t T) {
   if (T <= ctx->ws.max_tokens && (ctx->reserved_rows > 0 || ctx->ws.row_cap >= default_rows(T))) return SYFI_MOE_OK;
   // growing frees buffers that earlier calls may still be using
   CU_TRY(cudaDeviceSynchronize());
-  ctx->map_w13 = nullptr;   // cached tensor maps point into the old workspace
+  ctx->ws_maps = false;     // they point into the old workspace
   ctx->counters_clean = false;
   return alloc_workspace(ctx->ws, T > ctx->ws.max_tokens ? T : ctx->ws.max_tokens, ctx->reserved_rows);
 }
@@ -307,50 +309,57 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     if (v == 32 || v == 64 || v == 128 || (v == 256 && !packed)) token_tile = v;
   }
   const bool pair = token_tile == 256;
-  const bool maps_valid = ctx->map_w13 == w13 && ctx->map_w2 == w2 && ctx->map_ws == ws.a_perm &&
-                          ctx->map_e_local == e_local && ctx->map_token_tile == token_tile &&
-                          ctx->map_packed == packed;
-  if (!maps_valid) {
-  ctx->map_w13 = nullptr;
   g1.token_tile = g2.token_tile = pair ? kTailTile : token_tile;
   g1.tails = pair ? 1 : 0;
   g1.w_packed = packed ? static_cast<const uint8_t*>(w13) : nullptr;
   g2.w_packed = packed ? static_cast<const uint8_t*>(w2) : nullptr;
-  if (pair) {
-    if ((rc = make_map(&ctx->p1.tm_w, w13, (uint64_t)e_local * 2 * kInter, kHidden, 128))) return rc;
-    if ((rc = make_map(&ctx->p2.tm_w, w2, (uint64_t)e_local * kHidden, kInter, 128))) return rc;
-    if ((rc = make_map(&ctx->p1.tm_b0, ws.a_perm, ws.row_cap, kHidden, 32))) return rc;
-    ctx->p1.tm_b1 = ctx->p1.tm_b0;
-    if ((rc = make_map(&ctx->p2.tm_b0, ws.c_hi, ws.row_cap, kInter, 32))) return rc;
-    if ((rc = make_map(&ctx->p2.tm_b1, ws.c_lo, ws.row_cap, kInter, 32))) return rc;
-    if ((rc = make_map(&ctx->p1.tm_b0w, ws.a_perm, ws.row_cap, kHidden, 128))) return rc;
-    ctx->p1.tm_b1w = ctx->p1.tm_b0w;
-    // GEMM1's remainders (see tail_rows)
-    if ((rc = make_map3(&g1.tm_w, w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128))) return rc;
-    if ((rc = make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, kTailTile))) return rc;
-    if ((rc = make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16))) return rc;
-    if ((rc = make_map(&ctx->p2.tm_b0w, ws.c_hi, ws.row_cap, kInter, 128))) return rc;
-    if ((rc = make_map(&ctx->p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128))) return rc;
-  } else {
-  if (!packed) {   // (packed tiles are fetched with untiled copies)
-    for (int i = 0; i < (token_tile == 32 ? 4 : 1); ++i)
-      if ((rc = make_map3(i == 0 ? &g1.tm_w : &g1.tm_part.m[i - 1], w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128 >> i))) return rc;
-    if ((rc = make_map3(&g2.tm_w, w2, e_local, kHidden, kInter, 1, 128))) return rc;
+  ctx->maps_encoded = 0;
+#define MAP_TRY(expr) do { ++ctx->maps_encoded; if ((rc = (expr))) return rc; } while (0)
+  if (ctx->map_token_tile != token_tile) {
+    ctx->ws_maps = false;
+    ctx->map_w13 = nullptr;
+    ctx->map_token_tile = token_tile;
   }
-  if ((rc = make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, token_tile))) return rc;
-  if ((rc = make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16))) return rc;
-  if ((rc = make_map3(&g2.tm_b, ws.c_hi, 2, ws.row_cap, kInter, 2, token_tile))) return rc;
-  if ((rc = make_map3(&g2.tm_bs, ws.c_hi, 2, ws.row_cap, kInter, 2, 16))) return rc;
-  if ((rc = make_scale_map(&g2.tm_sc, ws.c_scale, kIBlocks, ws.row_cap, token_tile))) return rc;
-  g1.tm_sc = g2.tm_sc;
+  PairGemmLaunch& p1 = ctx->p1;
+  PairGemmLaunch& p2 = ctx->p2;
+  if (!ctx->ws_maps) {
+    if (pair) {
+      MAP_TRY(make_map(&p1.tm_b0, ws.a_perm, ws.row_cap, kHidden, 32));
+      p1.tm_b1 = p1.tm_b0;
+      MAP_TRY(make_map(&p2.tm_b0, ws.c_hi, ws.row_cap, kInter, 32));
+      MAP_TRY(make_map(&p2.tm_b1, ws.c_lo, ws.row_cap, kInter, 32));
+      MAP_TRY(make_map(&p1.tm_b0w, ws.a_perm, ws.row_cap, kHidden, 128));
+      p1.tm_b1w = p1.tm_b0w;
+      MAP_TRY(make_map(&p2.tm_b0w, ws.c_hi, ws.row_cap, kInter, 128));
+      MAP_TRY(make_map(&p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128));
+    } else {
+      MAP_TRY(make_map3(&g2.tm_b, ws.c_hi, 2, ws.row_cap, kInter, 2, token_tile));
+      MAP_TRY(make_map3(&g2.tm_bs, ws.c_hi, 2, ws.row_cap, kInter, 2, 16));
+      MAP_TRY(make_scale_map(&g2.tm_sc, ws.c_scale, kIBlocks, ws.row_cap, token_tile));
+      g1.tm_sc = g2.tm_sc;
+    }
+    MAP_TRY(make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, g1.token_tile));   // pair: GEMM1's remainders (see tail_rows)
+    MAP_TRY(make_map3(&g1.tm_bs, ws.a_perm, 1, ws.row_cap, kHidden, 1, 16));
+    ctx->ws_maps = true;
   }
-  ctx->map_w13 = w13;
-  ctx->map_w2 = w2;
-  ctx->map_ws = ws.a_perm;
-  ctx->map_e_local = e_local;
-  ctx->map_token_tile = token_tile;
-  ctx->map_packed = packed;
+  if (ctx->map_w13 != w13 || ctx->map_w2 != w2 || ctx->map_e_local != e_local || ctx->map_packed != packed) {
+    ctx->map_w13 = nullptr;
+    if (pair) {
+      MAP_TRY(make_map(&p1.tm_w, w13, (uint64_t)e_local * 2 * kInter, kHidden, 128));
+      MAP_TRY(make_map(&p2.tm_w, w2, (uint64_t)e_local * kHidden, kInter, 128));
+    }
+    if (!packed) {   // (packed tiles are fetched with untiled copies)
+      const int boxes = token_tile == 32 ? 4 : 1;      // 128 rows; 64, 32 and 16 for the parts of a split round
+      for (int i = 0; i < boxes; ++i)
+        MAP_TRY(make_map3(i == 0 ? &g1.tm_w : &g1.tm_part.m[i - 1], w13, 2 * (uint64_t)e_local, kInter, kHidden, 2, 128 >> i));
+      if (!pair) MAP_TRY(make_map3(&g2.tm_w, w2, e_local, kHidden, kInter, 1, 128));
+    }
+    ctx->map_w13 = w13;
+    ctx->map_w2 = w2;
+    ctx->map_e_local = e_local;
+    ctx->map_packed = packed;
   }
+#undef MAP_TRY
 
   const int grid = ctx->num_sms < kMaxGrid ? ctx->num_sms : kMaxGrid;
   ctx->launches = 0;
@@ -509,7 +518,7 @@ int syfi_moe_reserve(syfi_moe_ctx* ctx, int64_t max_tokens, int64_t max_rows) {
   DeviceGuard guard(ctx->ws.device);
   if (!guard.ok) return fail(SYFI_MOE_ERR_CUDA, "cannot select device %d", ctx->ws.device);
   CU_TRY(cudaDeviceSynchronize());       // earlier calls may still be using the buffers that are replaced
-  ctx->map_w13 = nullptr;
+  ctx->ws_maps = false;
   ctx->counters_clean = false;
   ctx->reserved_rows = max_rows;
   return alloc_workspace(ctx->ws, max_tokens, max_rows);
@@ -997,7 +1006,7 @@ int syfi_moe_debug_read(syfi_moe_ctx* ctx, const char* name, void* dst_host, int
       {"a_perm", ws.a_perm, R * kHidden},        {"a_scale", ws.a_scale, R * kHBlocks * 4},
       {"c_hi", ws.c_hi, R * kInter},             {"c_lo", ws.c_lo, R * kInter},
       {"c_scale", ws.c_scale, R * kIBlocks * 4}, {"o_rows", ws.o_rows, R * kHidden * 4},
-      {"trace", ws.trace, 8 * 4096 * 8},
+      {"trace", ws.trace, 8 * 4096 * 8},         {"maps_encoded", &ctx->maps_encoded, 4},
       {"topk_idx", ws.topk_idx, T * kTopK * 4},  {"topk_w", ws.topk_w, T * kTopK * 4},
   };
   for (const Entry& e : table) {
@@ -1006,7 +1015,7 @@ int syfi_moe_debug_read(syfi_moe_ctx* ctx, const char* name, void* dst_host, int
       if (row_cap) *row_cap = ws.row_cap;
       if (dst_host && max_bytes > 0) {
         CU_TRY(cudaDeviceSynchronize());
-        CU_TRY(cudaMemcpy(dst_host, e.ptr, (size_t)(e.bytes < max_bytes ? e.bytes : max_bytes), cudaMemcpyDeviceToHost));
+        CU_TRY(cudaMemcpy(dst_host, e.ptr, (size_t)(e.bytes < max_bytes ? e.bytes : max_bytes), cudaMemcpyDefault));
       }
       return SYFI_MOE_OK;
     }

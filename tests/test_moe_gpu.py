@@ -333,6 +333,29 @@ def test_small_batches_equal_the_same_tokens_in_a_larger_one(T, E, off, pkg):
         assert not got[want < 0].any()
 
 
+def test_layers_in_turn_share_the_workspace_maps(pkg, oracle, monkeypatch):
+    """A model calls its layers one after the other through one context: a call with other weights encodes the weights'
+    tensor maps only (the workspace's stay), one with the same weights none, and each computes with its own."""
+    layers = [pkg.make_inputs(num_tokens=24, seed=60 + i, e_local=2 + i, local_expert_offset=8 * i, device=DEV) for i in range(2)]
+    refs = [oracle.moe_forward(*inp.args())[0] for inp in layers]
+    encoded = lambda: int(pkg.get_context(0).debug_read("maps_encoded", torch.int32)[0][0])
+    for tile, weights in ((32, 5), (64, 2), (256, 3)):
+        monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", str(tile))
+        for rnd in range(3):
+            for inp, ref in zip(layers, refs):
+                out, _ = _run(pkg, inp)
+                assert rnd == 0 or encoded() == weights
+                ok, stats = oracle.check_output(out, ref)
+                assert ok, stats
+        _run(pkg, inp)
+        assert encoded() == 0
+    pkg.get_context(0).reserve(64, 0)
+    out, _ = _run(pkg, inp)                              # the workspace's buffers are new
+    assert encoded() == 8
+    ok, stats = oracle.check_output(out, ref)
+    assert ok, stats
+
+
 def _swizzled_tiles(x):
     """x: [..., 128 rows, 8 chunks, 16 bytes] -> chunk c of row r moved to chunk c ^ (r & 7)."""
     r = torch.arange(128, device=x.device)[:, None]
