@@ -380,6 +380,8 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
                      ctx->n_pending == 0 && ctx->wait_before_gather == nullptr && !(flags & kFlagRoutingGiven);
   g1.front = g2.front = front ? 1 : 0;
   if (front) {
+    // a call that failed behind its front kernel has left the tables valid
+    if (!clean) CU_TRY(cudaMemsetAsync(ws.meta + kMetaTables, 0, sizeof(int), st));
     CU_TRY(launch_front(static_cast<const float*>(logits), bias, static_cast<const uint8_t*>(hs),
                         static_cast<const float*>(hs_scale), T, e_local, (int)offset, (float)scaling, token_tile, ws,
                         ctx->num_sms, st));

@@ -996,7 +996,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (C::kSplit && sched.parts > 1) roles(std::integral_constant<bool, C::kSplit>{});
   else roles(std::false_type{});
 
-  if (MODE == 1 && EARLY) pdl_wait();   // no CTA ends before the gather has (kernels behind this one rely on it)
+  // The 32-row kernels start before the kernel in front of GEMM1 is done, and that one writes more than GEMM1 waits for (the
+  // front kernel writes the routes' rows last).  No GEMM1 CTA ends before it has.  GEMM2 has waited for GEMM1's items, hence
+  // for that kernel, unless there are none: then it waits for GEMM1 itself, so that the combine kernel, which waits for
+  // GEMM2 only, finds everything written.
+  if (EARLY && (MODE == 1 || s_meta[0] == 0)) pdl_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

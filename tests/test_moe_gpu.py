@@ -422,6 +422,38 @@ def test_tokens_without_local_route_get_zero(pkg):
     assert stats["routes"] == int(hit.sum())
 
 
+@pytest.mark.parametrize("T", [1, 16, 17, 40])
+def test_small_batches_without_any_local_route(T, pkg):
+    """No row, no token tile: GEMM2 has nothing whose completion it could wait for, and still the combine kernel must not
+    run before the routes' rows are written.  Every call follows one that left rows for the same tokens, eagerly and
+    replayed from a graph (up to 16 tokens the router, the row lists and the gather are one kernel)."""
+    hit = pkg.make_inputs(num_tokens=T, seed=41, e_local=4, device=DEV)
+    hit.routing_logits[:, :4] += 9.0
+    miss = pkg.MoeInputs(hit.routing_logits.clone(), *hit.args()[1:])
+    miss.routing_logits[:, :32] -= 30.0                       # the whole group of the local experts
+    want, stats = _run(pkg, hit)
+    assert stats["routes"] >= T and bool((want.float().abs().amax(1) > 0).all())
+    zero, stats = _run(pkg, miss)
+    assert stats["routes"] == 0 and stats["token_tiles"] == 0 and not zero.any()
+    outs = [torch.empty_like(want) for _ in range(2)]
+    for _ in range(100):
+        outs[1].fill_(1.0)
+        pkg.run_moe(*hit.args(), outs[0])
+        pkg.run_moe(*miss.args(), outs[1])
+        assert torch.equal(outs[0], want) and not outs[1].any()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pkg.run_moe(*hit.args(), outs[0])
+        pkg.run_moe(*miss.args(), outs[1])
+        pkg.run_moe(*hit.args(), outs[0])
+    for _ in range(20):
+        outs[0].zero_()
+        outs[1].fill_(1.0)
+        graph.replay()
+        assert torch.equal(outs[0], want) and not outs[1].any()
+    pkg.get_context(0).check()
+
+
 def test_deterministic_and_workspace_reuse(pkg):
     inp = pkg.make_inputs(num_tokens=200, seed=11, e_local=8, device=DEV)
     a, _ = _run(pkg, inp)
