@@ -298,7 +298,7 @@ def gemm1_roofline(T, rows, active, stage_ms, peaks, world):
         achieved = flops / t / 1e12
         peak = 2.0 * peaks["bf16_tflops_sustained"]
         key = "pair_gemm_kernel<1>@T8192_E32" if (T == 8192 and world == 1 and active >= 24) else None
-        return {"kernel": "pair_gemm_kernel<1> (GEMM1 + SwiGLU + two-term requantisation, CTA pairs, tcgen05 cta_group::2)",
+        return {"kernel": "pair_gemm_kernel<1> and, on the experts' remainders, grouped_gemm_kernel<1,64> (GEMM1 + SwiGLU + two-term requantisation, CTA pairs, tcgen05 cta_group::2)",
                 "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "peak_note": "no FP8 figure in MEASURED_PEAKS.json: 2 x bf16_tflops_sustained as the measured proxy "
                              "(kernel timed inside a long step)",

@@ -229,13 +229,18 @@ const void* mapped_alias(const void* host) {
 }
 
 // Batches from this size on use the CTA-pair GEMM kernels, with GEMM1's small remainders on the single-CTA kernel.
-// Against 64-row tiles alone, us per call, two seeds: 3072 tokens 459 / 387 and 482 / 372, 4096 tokens 523 / 435 and
-// 570 / 467, 8192 tokens 870 / 829 and 1030 / 958.
-// That is with 32 local experts.  With fewer there are fewer tiles, and pairs pay off later: 8 experts, 64-row tiles / pairs,
+// 64-row tiles / pairs, us per call, four expert loads (the second and fourth with hot experts elsewhere), 32 local experts:
+// 2560 tokens 420 / 424, 282 / 297, 377 / 354, 214 / 229; 3072 tokens 472 / 457, 326 / 329, 420 / 388, 240 / 247; 3328 tokens
+// 529 / 473, 339 / 347, 443 / 414, 240 / 262; 3600 tokens 528 / 495, 345 / 363, 453 / 420, 267 / 265; 4000 tokens 554 / 533,
+// 382 / 381, 494 / 464, 278 / 268; 5000 tokens 655 / 597, 523 / 456, 631 / 595, 512 / 437: below the line one load gains
+// what another loses.
+// With fewer experts there are fewer tiles, and pairs pay off later: 8 experts, 64-row tiles / pairs,
 // 3600 tokens 156 / 167 and 94 / 104, 4500 tokens 193 / 177 and 103 / 113, from 6144 on the pairs.
 constexpr int64_t kPairMinTokens = 3584;
 constexpr int64_t kPairMinTokensAnyExperts = 6144;
-constexpr int64_t kWideListMinTokens = 6144;   // from here on the row lists of the pair configuration count 128-row tiles
+// The pair configuration's kernels count their own tiles; what the row lists count is a statistic (syfi_moe_check), of
+// 64-row tiles below this many tokens and of 128-row tiles from there on.
+constexpr int64_t kWideListMinTokens = 6144;
 constexpr int kFlagOutF32 = 1;      // run_layer flags
 constexpr int kFlagPrepacked = 2;
 constexpr int kFlagRoutingGiven = 4;   // the workspace already holds routes, masks and row counters of all tokens (token dispatch)
@@ -402,7 +407,6 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
     CU_TRY(cudaEventRecord(ctx->ev_copy_done, ctx->copy_stream));
     ctx->wait_before_gather = ctx->ev_copy_done;
   }
-  // The pair configuration's kernels count their own tiles; the row lists' count is what syfi_moe_debug_read shows.
   const int listed_tile = !pair ? token_tile : T64 < kWideListMinTokens ? 64 : 128;
   CU_TRY(launch_build_rows(T, e_local, (int)offset, listed_tile, ws, st));
   ctx->launches += 1;

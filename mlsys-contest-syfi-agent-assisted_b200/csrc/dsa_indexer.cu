@@ -7,7 +7,7 @@
 // (dsa_indexer/solution/python/dsa_topk_indexer.py:64-112, pure torch):
 //     score[t] = sum_h weights[b, h] * relu(q[b, h, :] . (k8[t, :] * kscale[t])),   best 2048 tokens, best first.
 //
-//   score kernel : one CTA per (sequence, 1024 tokens), 128 tokens = two cache pages per MMA, key tiles and
+//   score kernel : one CTA per (sequence, run of 128 to 1024 tokens), 128 tokens = two cache pages per MMA, key tiles and
 //                  accumulators double-buffered.  The pages' 64 x 128 e4m3 bytes are
 //                  contiguous in the cache (a page is 64 rows of 128 bytes followed by 64 f32 scales = 66 rows of
 //                  128 bytes), so one tensor map over the cache as rows of 128 bytes fetches a page with one TMA
@@ -16,7 +16,8 @@
 //                  exact, so the token's scale is applied once, after the sum over K.  Each thread then owns a
 //                  token: relu, times the head weight, summed over the 64 heads in head order.
 //   select kernel: a counting sort by value over a cluster of CTAs per sequence (best first, ties by position), with an
-//                  exact radix select and bitonic sort for score distributions that it does not separate.
+//                  exact radix select over the cluster and a bitonic sort for score distributions that it does not
+//                  separate.
 // Every wait is bounded; a failure is recorded in the status word the host entry point reads back.
 #include <cooperative_groups.h>
 #include <cuda.h>
