@@ -366,7 +366,8 @@ static_assert(kMaxListed * 8 >= kBins * 4 && kKeep * 8 <= kBins * 4, "aliases of
 //      2048 best are written best first without a sorting network.
 // The kernel is a chain of short steps between barriers, so what counts is their number: an eight-pass radix select and
 // a 66-stage bitonic sort per 16384 positions, then the same again over the chunks' candidates, took 25 us for three
-// short sequences and 22 + 32 us for 32 sequences of 65536 tokens; this one takes 6 and 12 us.
+// short sequences and 22 + 32 us for 32 sequences of 65536 tokens; this one takes about 6 us and
+// 16 us (the latter under ncu, with cold caches).
 // Where the bins do not separate the scores (a bin at or above the cut holds more than kMaxInBin items: ties, or
 // outliers that stretch the range; infinities and NaNs), the cluster selects by radix instead, see select_best: us per
 // call, separable scores / one outlier per sequence / the same with the first CTA alone on the whole sequence:
