@@ -245,14 +245,14 @@ constexpr int kFlagOutF32 = 1;      // run_layer flags
 constexpr int kFlagPrepacked = 2;
 constexpr int kFlagRoutingGiven = 4;   // the workspace already holds routes, masks and row counters of all tokens (token dispatch)
 
-// f32 matrix [rows, cols] (cols contiguous), box [rows, box_cols], no swizzle: the per-K-block scales of a
+// f32 matrix [rows, cols] (cols contiguous), box [box_rows, box_cols], no swizzle: the per-K-block scales of a
 // token tile, fetched with one load.
-int make_scale_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_cols) {
+int make_scale_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return fail(SYFI_MOE_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * 4};
-  const cuuint32_t box[2] = {box_cols, (cuuint32_t)rows};
+  const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -334,13 +334,13 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
       MAP_TRY(make_map(&p2.tm_b0, ws.c_hi, ws.row_cap, kInter, 32));
       MAP_TRY(make_map(&p2.tm_b1, ws.c_lo, ws.row_cap, kInter, 32));
       MAP_TRY(make_map(&p1.tm_b0w, ws.a_perm, ws.row_cap, kHidden, 128));
-      p1.tm_b1w = p1.tm_b0w;
-      MAP_TRY(make_map(&p2.tm_b0w, ws.c_hi, ws.row_cap, kInter, 128));
-      MAP_TRY(make_map(&p2.tm_b1w, ws.c_lo, ws.row_cap, kInter, 128));
+      MAP_TRY(make_map(&p2.tm_b0w, ws.c_hi, 2 * (uint64_t)ws.row_cap, kInter, 128));
+      MAP_TRY(make_scale_map(&p1.tm_sc, ws.a_scale, kHBlocks, ws.row_cap, kHBlocks / 2, 128));
+      p2.tm_sc = p1.tm_sc;
     } else {
       MAP_TRY(make_map3(&g2.tm_b, ws.c_hi, 2, ws.row_cap, kInter, 2, token_tile));
       MAP_TRY(make_map3(&g2.tm_bs, ws.c_hi, 2, ws.row_cap, kInter, 2, 16));
-      MAP_TRY(make_scale_map(&g2.tm_sc, ws.c_scale, kIBlocks, ws.row_cap, token_tile));
+      MAP_TRY(make_scale_map(&g2.tm_sc, ws.c_scale, kIBlocks, ws.row_cap, kIBlocks, token_tile));
       g1.tm_sc = g2.tm_sc;
     }
     MAP_TRY(make_map3(&g1.tm_b, ws.a_perm, 1, ws.row_cap, kHidden, 1, g1.token_tile));   // pair: GEMM1's remainders (see tail_rows)

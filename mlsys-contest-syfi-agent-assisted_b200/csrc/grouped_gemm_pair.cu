@@ -24,13 +24,20 @@
 //     token rows, CTA 1 the lo term (N operand), so accumulator columns [0, n) are hi products and
 //     [n, 2n) lo products.
 //
-// Per K block (128 bytes of K) the raw e4m3 products accumulate in tensor memory (4 MMAs of K = 32) and
-// are then promoted into f32 registers with activation scale x weight scale; tensor memory holds two
-// accumulator slots of 256 columns, so the MMAs of block k + 1 run while block k is promoted.
+// Per K block (128 bytes of K) the raw e4m3 products accumulate in tensor memory (4 MMAs of K = 32 per slot) and
+// are then promoted into f32 registers with activation scale x weight scale.  Tensor memory holds two K blocks: mode 2
+// in two slots of 256 columns, mode 1 in four of 128, one per half of the features (up and gate), so that a half is
+// promoted while the other's MMAs still run.
 //
-// Roles per CTA: warp 0 = TMA producer (one thread), warp 1 = tensor memory owner and, in the pair's
-// first CTA, the MMA issuer, warp 2 = scale warp (mode 1: fetches the weight scales of the next item;
-// mode 2: multiplies a K block's activation scales with its weight scale into a shared-memory ring),
+// What bounds mode 1 (clocks per K block at 8192 tokens, parts switched off): MMAs alone 531, with the loads 642, with
+// the hand-off of the slots 757, complete 879, of which the epilogue (SwiGLU, requantisation, stores) about 80.  The
+// promotion warps use two thirds of the issue slots (160 instructions per warp and K block when it took 990, 64 of them
+// the FMAs), so fewer instructions there is what counts: 32-bit barrier addresses, scales that arrive by TMA instead of
+// through the epilogue's registers, eight columns per tcgen05.ld (sixteen make the compiler keep values in local memory).
+//
+// Roles per CTA: warp 0 = TMA producer (one thread; mode 1: the activation and weight scales too), warp 1 = tensor memory
+// owner and, in the pair's first CTA, MMA issuer (mode 1: of the even K blocks), warp 2 = issuer of the odd K blocks
+// (mode 1) / scale warp (mode 2: multiplies a K block's activation scales with its weight scale into a shared-memory ring),
 // warp 3 = cross-kernel bookkeeping (as in grouped_gemm.cu), warps 4..19 = promotion / epilogue
 // (a warp reads one tensor-memory lane quarter; four warps share a quarter and split the columns).
 // An expert's last rows, up to 128 that would leave a 256-row tile at most half full, are not this GEMM1's but the
@@ -51,7 +58,8 @@ namespace {
 constexpr int kTile = 128 * 128;             // operand tile: 128 rows x 128 bytes of K
 constexpr int kBox = 32 * 128;               // token-side TMA box: 32 rows x 128 bytes
 constexpr int kStageBytes = 2 * kTile;       // one K block: M-side tile, then N-side tile
-constexpr int kScaleRing = 16;               // K blocks of scales in flight
+constexpr int kScaleRing = 16;               // mode 2: K blocks of scales in flight
+constexpr int kScaleChunk = kHBlocks / 2;    // mode 1: K blocks per buffer of activation scales (two buffers hold an item's)
 constexpr int kEpiWarps = 16;
 constexpr int kEpiThreads = 32 * kEpiWarps;
 constexpr int kPairThreads = 128 + kEpiThreads;
@@ -63,16 +71,15 @@ template <int MODE> struct PairCfg {
   static constexpr int kFeatItems = MODE == 1 ? kInter / 128 : kHidden / 256;   // 16 / 28 per expert and token tile
   static constexpr int kTokTile = MODE == 1 ? kPairTile : 128;
   static constexpr int kStages = 6;
-  // Two accumulator slots of 256 tensor-memory columns: the MMAs of K block k + 1 run while block k is
-  // promoted.  (Four slots of 128 columns, a K block issued as two MMA groups of N = 128, doubled the
-  // hand-offs between the MMA thread and the promotion warps and were slower.)
-  static constexpr int kSlots = 2;
+  static constexpr int kSlots = MODE == 1 ? 4 : 2;
   static constexpr int kSlotCols = kPairTmemCols / kSlots;
-  static constexpr int kScaleEntry = 128;   // floats per ring entry: one per token lane (mode 1) / token column (mode 2)
-  // mode 1: the activation scales of a whole item, [56][128]; mode 2: a ring of K blocks of scale products
+  static constexpr int kScaleEntry = 128;   // floats per K block: one per token lane (mode 1) / token column (mode 2)
+  // mode 1: the activation scales of a whole item, [56][128], in two buffers; mode 2: a ring of K blocks of scale products
   static constexpr int kScaleFloats = MODE == 1 ? kHBlocks * 128 : kScaleRing * kScaleEntry;
+  static constexpr int kScaleBufs = MODE == 1 ? 2 : kScaleRing;
+  static constexpr int kBarriers = kStages + kStages / 2 + 2 * kMaxSlots + 2 * kScaleBufs + 4;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleFloats * 4 +
-                                    (MODE == 1 ? 4 * 128 * 4 + 2 * 128 * 4 : 0) + 8 * 64 +
+                                    (MODE == 1 ? 2 * 4 * 128 * 4 + 2 * 128 * 4 : 0) + 8 * kBarriers +
                                     kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 64;
   static_assert(kSmemBytes <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
   static_assert(kStages % 2 == 0 && kKBlocks % 2 == 0, "stages are filled in K-adjacent pairs");
@@ -149,7 +156,7 @@ template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
                  const __grid_constant__ CUtensorMap tm_b1, const __grid_constant__ CUtensorMap tm_b0w,
-                 const __grid_constant__ CUtensorMap tm_b1w, const PairArgs p) {
+                 const __grid_constant__ CUtensorMap tm_sc, const PairArgs p) {
   using C = PairCfg<MODE>;
   constexpr int G = C::kStages;
   constexpr int KB = C::kKBlocks;
@@ -158,20 +165,20 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   constexpr int SE = C::kScaleEntry;
   constexpr int kSlots = C::kSlots;
   constexpr int kSlotCols = C::kSlotCols;
-  constexpr int kIssuers = MODE == 1 ? 2 : 1;   // MMA-issuing threads (see mma_role)
+  constexpr int kIssuers = MODE == 1 ? 2 : 1;   // MMA-issuing threads
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   float* s_scale = reinterpret_cast<float*>(smem + G * kStageBytes);           // mode 1: [56][128]; mode 2: [kScaleRing][SE]
-  float* s_red = s_scale + C::kScaleFloats;                                    // [4][128] partial amax (mode 1)
-  float* s_ws = s_red + (MODE == 1 ? 4 * 128 : 0);                             // [2][128] weight scales of an item (mode 1)
+  float* s_red = s_scale + C::kScaleFloats;                                    // [2][4][128] partial amax of an item (mode 1)
+  float* s_ws = s_red + (MODE == 1 ? 2 * 4 * 128 : 0);                         // [2][128] weight scales of an item (mode 1)
   uint64_t* full = reinterpret_cast<uint64_t*>(s_ws + (MODE == 1 ? 2 * 128 : 0));   // [G]   first CTA's are used
   uint64_t* empty = full + G;                                                  // [G/2] per CTA
   uint64_t* tfull = empty + G / 2;                                             // [4]   per CTA
   uint64_t* tempty = tfull + kMaxSlots;                                        // [4]   first CTA's are used
-  uint64_t* sfull = tempty + kMaxSlots;                                         // [16]  per CTA
-  uint64_t* sempty = sfull + kScaleRing;                                       // [16]  per CTA
-  uint64_t* wfull = sempty + kScaleRing;                                       // [2]   mode 1: an item's weight scales are there
+  uint64_t* sfull = tempty + kMaxSlots;                                        // [2 or 16] per CTA
+  uint64_t* sempty = sfull + C::kScaleBufs;                                    // [2 or 16] per CTA
+  uint64_t* wfull = sempty + C::kScaleBufs;                                       // [2]   mode 1: an item's weight scales are there
   uint64_t* wempty = wfull + 2;                                                // [2]
   ExpertWork* s_work = reinterpret_cast<ExpertWork*>(wempty + 2);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_work + kMaxLocalExperts);
@@ -182,13 +189,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const uint32_t peer = rank ^ 1u;
-  const uint32_t peer_abort = mapa_u32(smem_u32(const_cast<int*>(s_abort)), peer);
+  const uint32_t abort_flag = smem_u32(const_cast<int*>(s_abort));
+  const uint32_t peer_abort = mapa_u32(abort_flag, peer);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < G; ++i) mbar_init(&full[i], 1);
     for (int i = 0; i < G / 2; ++i) mbar_init(&empty[i], kIssuers);   // one commit per MMA issuer
-    for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 2 * kEpiWarps); }
-    for (int i = 0; i < kScaleRing; ++i) { mbar_init(&sfull[i], 1); mbar_init(&sempty[i], kEpiWarps); }
+    for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], (MODE == 1 ? 1 : 2) * kEpiWarps); }
+    for (int i = 0; i < C::kScaleBufs; ++i) { mbar_init(&sfull[i], 1); mbar_init(&sempty[i], kEpiWarps); }
     for (int i = 0; i < 2; ++i) { mbar_init(&wfull[i], 1); mbar_init(&wempty[i], kEpiWarps); }
     *s_abort = 0;
     *s_done = 0;
@@ -196,7 +204,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     tma_prefetch_desc(&tm_w);
     tma_prefetch_desc(&tm_b0);
     tma_prefetch_desc(&tm_b0w);
-    if (MODE == 2) { tma_prefetch_desc(&tm_b1); tma_prefetch_desc(&tm_b1w); }
+    if (MODE == 1) tma_prefetch_desc(&tm_sc);
+    if (MODE == 2) tma_prefetch_desc(&tm_b1);
   }
   // both CTAs' barriers exist before anyone signals across the pair
   cluster_sync_all();
@@ -238,53 +247,85 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int my_items = cluster_id < total ? (total - cluster_id + n_clusters - 1) / n_clusters : 0;
   auto item_of = [&](int i) { return cluster_id + i * n_clusters; };
 
-  // MMA issue, one thread of the pair's first CTA per K-block parity.  Two issuers (even K blocks -> slot 0,
-  // odd -> slot 1) because an issuer is tied up for the whole execution time of its MMAs (the queue behind
-  // tcgen05.mma is shallow) and then pays its commits and the wait for its slot: with one issuer the tensor
-  // pipe idles during those; with two, one's waits overlap the other's MMAs.  MMAs of different slots are
-  // independent, and tcgen05.commit tracks the MMAs of the committing thread only, so each issuer commits its
-  // own slot and its own half of the stage pair (empty[] counts two arrivals).
-  auto mma_role = [&](const uint32_t par) {
-    uint32_t g = par, ph = 0, sph = 0;      // this issuer's next stage and its phase, phase of its slot
-    uint32_t slot = par;                    // mode 2 (one issuer): alternates between the two slots
-    int e_hint = 0;
-    bool alive = true;
+  // MMA issue, mode 1: one thread of the pair's first CTA per K-block parity, which issues a K block as two groups of
+  // N = 128, one per half of the features, each with its own accumulator slot.  (An issuer is tied up for the whole
+  // execution time of its MMAs, as the queue behind tcgen05.mma is shallow, and then pays its commits and the wait for
+  // its slot; of two issuers, one's waits overlap the other's MMAs.  MMAs of different slots are independent, and
+  // tcgen05.commit tracks the MMAs of the committing thread only, so each commits its own slots and its own half of the
+  // stage pair: empty[] counts two arrivals.)  Two groups of N = 128 take the tensor core as long as one of N = 256 (528 and
+  // 531 clocks per K block, MMAs alone), and a half's eight promotion warps start while the other half's MMAs run.  An
+  // issuer has no more instructions between a slot's release and the next MMAs than it must: it shares its scheduler with
+  // four promotion warps.  Clocks per K block of the whole kernel at 8192 tokens, slots of 256 / of 128 columns with an
+  // issuer per half / per parity: 950 / 985 / 940.
+  auto mma_halves = [&](const uint32_t par) {
+    const uint32_t sb = smem_u32(smem) + par * kStageBytes;
+    const uint64_t a0 = umma_smem_desc_sw128(sb), b0 = umma_smem_desc_sw128(sb + kTile);
+    constexpr uint64_t kNext = 2 * kStageBytes >> 4, kHalfRows = (kTile / 2) >> 4;   // descriptor steps
+    constexpr uint32_t idesc = umma_idesc_e4m3_m256(128u);
+    uint32_t ph = 0, sph = 1;
+    const int total = my_items * (KB / 2);
     ST_DECL;
     const long long st_start = clock64();
     (void)st_start;
-    for (int i = 0; i < my_items && alive; ++i) {
+    for (int n = 0; n < total;) {
+#pragma unroll
+      for (int j = 0; j < G / 2; ++j) {
+        if (n == total) break;
+        if (!mbar_wait_bounded_tell(smem_u32(&full[2 * j + par]), ph, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t slot = 2 * par + h;
+          if (!mbar_wait_bounded_tell(smem_u32(&tempty[slot]), sph, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
+          tc_fence_after();
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4)
+            umma_f8_pair(tmem_base + slot * kSlotCols, a0 + j * kNext + 2 * k4, b0 + j * kNext + h * kHalfRows + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+          umma_commit_pair(&tfull[slot], 3);
+        }
+        umma_commit_pair(&empty[j], 3);
+        sph ^= 1u;
+        ++n;
+      }
+      ph ^= 1u;
+    }
+    ST_WRITE(4, par == 0);
+  };
+
+  // mode 2: one issuer, two slots in turn
+  auto mma_whole = [&]() {
+    uint32_t g = 0, ph = 0, slot = 0, sph = 0;
+    int e_hint = 0;
+    ST_DECL;
+    const long long st_start = clock64();
+    (void)st_start;
+    for (int i = 0; i < my_items; ++i) {
       const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
-      const uint32_t idesc = umma_idesc_e4m3_m256(MODE == 1 ? 256u : 2u * im.n);
-      for (int kb = static_cast<int>(par); kb < KB; kb += kIssuers) {
+      const uint32_t idesc = umma_idesc_e4m3_m256(2u * im.n);
+      for (int kb = 0; kb < KB; ++kb) {
         ST_BEGIN();
-        if (!mbar_wait_bounded_tell(&full[g], ph, s_abort, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
+        if (!mbar_wait_bounded_tell(smem_u32(&full[g]), ph, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
         ST_END(0);
         const uint32_t sb = smem_u32(smem + g * kStageBytes);
         const uint64_t a0 = umma_smem_desc_sw128(sb);
         const uint64_t b0 = umma_smem_desc_sw128(sb + kTile);
         ST_BEGIN();
-        if (!mbar_wait_bounded_tell(&tempty[slot], sph ^ 1u, s_abort, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) { alive = false; break; }
+        if (!mbar_wait_bounded_tell(smem_u32(&tempty[slot]), sph ^ 1u, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
         ST_END(1);
         tc_fence_after();
         const uint32_t d0 = tmem_base + slot * kSlotCols;
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) umma_f8_pair(d0, a0 + 2 * k4, b0 + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-        if (kIssuers == 2 || (g & 1u)) umma_commit_pair(&empty[g >> 1], 3);
+        if (g & 1u) umma_commit_pair(&empty[g >> 1], 3);
         umma_commit_pair(&tfull[slot], 3);
-        if (kIssuers == 2) {
-          sph ^= 1u;
-        } else {
-          slot ^= 1u;
-          if (slot == 0) sph ^= 1u;
-        }
-        g += kIssuers;
-        if (g >= static_cast<uint32_t>(G)) { g -= G; ph ^= 1u; }
+        slot ^= 1u;
+        if (slot == 0) sph ^= 1u;
+        if (++g == static_cast<uint32_t>(G)) { g = 0; ph ^= 1u; }
       }
     }
 #ifdef SYFI_PAIR_STATS
     st_acc[2] = clock64() - st_start;
 #endif
-    ST_WRITE(4, par == 0);
+    ST_WRITE(4, true);
   };
 
   if (warp < 4) {
@@ -293,18 +334,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (lane == 0 && !p.silent_producer) {
         const uint64_t pol_w = s_meta[0] > s_meta[1] ? l2_policy_evict_last() : l2_policy_evict_first();
         const uint64_t pol_b = l2_policy_evict_last();
-        uint32_t full0[G];                     // the first CTA's full barriers as cluster addresses
-#pragma unroll
-        for (int i = 0; i < G; ++i) full0[i] = mapa_u32(smem_u32(&full[i]), 0);
+        const uint32_t full0 = mapa_u32(smem_u32(&full[0]), 0);   // the first CTA's full[0]; the others follow at 8 bytes each
         uint32_t it = 0, g = 0, ph = 0;        // stage pairs armed, next stage, phase of its empty barrier
-        uint32_t s = 0, sp = 0;                // scale ring entry and phase (mode 1)
         uint32_t wp = 0;                       // phase bits of wempty[0..1] (mode 1)
         uint32_t n_items = 0;
         int e_hint = 0;
         bool alive = true;
         ST_DECL;
         const long long st_start = clock64();
-        (void)st_start; (void)s; (void)sp; (void)wp;
+        (void)st_start; (void)wp;
         for (int i = 0; i < my_items && alive; ++i) {
           const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
           int my_rows, my_row, wrow, tok_off, w_off;
@@ -324,7 +362,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             my_rows = im.n;                                      // all rows of one term
             my_row = im.row_start;
             wrow = im.expert * kHidden + (2 * im.ft + static_cast<int>(rank)) * 128;
-            mb = my_rows > 64 ? (rank == 0 ? &tm_b0w : &tm_b1w) : (rank == 0 ? &tm_b0 : &tm_b1);
+            mb = my_rows > 64 ? &tm_b0w : rank == 0 ? &tm_b0 : &tm_b1;
+            if (my_rows > 64 && rank == 1) my_row += p.row_cap;   // (tm_b0w has the lo term's rows behind the hi term's)
             tok_off = kTile;
             w_off = 0;
             stage_tx = 2u * static_cast<uint32_t>(kTile + box_bytes(im.n));
@@ -334,7 +373,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             // weight scales of the item, [0..55] up block and [64..119] gate block, into the buffer the
             // epilogue released two items ago
             const int par = i & 1;
-            if (!mbar_wait_bounded_tell(&wempty[par], ((wp >> par) & 1u) ^ 1u, s_abort, peer_abort,
+            if (!mbar_wait_bounded_tell(smem_u32(&wempty[par]), ((wp >> par) & 1u) ^ 1u, abort_flag, peer_abort,
                                         kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
             wp ^= 1u << par;
             mbar_arrive_expect_tx(&wfull[par], 2u * kHBlocks * 4u);
@@ -364,9 +403,25 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             __threadfence_block();
             ++n_items;
           }
-          for (int kb = 0; kb < KB; kb += 2) {
+          // activation scales: an item's first buffer is free once the promotion is half through the item before, its second
+          // once it is through with it; asked for where the promotion, which is at most 8 K blocks behind, has passed that
+          auto load_scales = [&](const PItem& of, int buf, int phase) {
+            if (!mbar_wait_bounded_tell(smem_u32(&sempty[buf]), static_cast<uint32_t>(phase) ^ 1u, abort_flag, peer_abort,
+                                        kStatusWaitTimeoutProducer, p.wait_limit)) return false;
+            mbar_arrive_expect_tx(&sfull[buf], kScaleChunk * 128 * 4);
+            tma_load_2d(s_scale + buf * kScaleChunk * 128, &tm_sc, &sfull[buf], of.row_start + 128 * static_cast<int>(rank),
+                        buf * kScaleChunk, pol_b);
+            return true;
+          };
+          if (MODE == 1 && i == 0) alive = load_scales(im, 0, 0);
+          for (int kb = 0; kb < KB && alive; kb += 2) {
+            if (MODE == 1 && kb == 12 && !load_scales(im, 1, i & 1)) { alive = false; break; }
+            if (MODE == 1 && kb == 40 && i + 1 < my_items) {
+              int eh = e_hint;
+              if (!load_scales(decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i + 1), eh), 0, (i + 1) & 1)) { alive = false; break; }
+            }
             ST_BEGIN();
-            if (!mbar_wait_bounded_tell(&empty[g >> 1], ph ^ 1u, s_abort, peer_abort, kStatusWaitTimeoutProducer,
+            if (!mbar_wait_bounded_tell(smem_u32(&empty[g >> 1]), ph ^ 1u, abort_flag, peer_abort, kStatusWaitTimeoutProducer,
                                         p.wait_limit)) { alive = false; break; }
             ST_END(0);
             if (rank == 0) {
@@ -378,11 +433,11 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             uint8_t* st0 = smem + g * kStageBytes;
             uint8_t* st1 = st0 + kStageBytes;
             const int x0 = kb * 128;
-            tma_load_2d_pair(st0 + w_off, &tm_w, full0[g], x0, wrow, pol_w);
-            tma_load_2d_pair(st1 + w_off, &tm_w, full0[g + 1], x0 + 128, wrow, pol_w);
+            tma_load_2d_pair(st0 + w_off, &tm_w, full0 + 8u * g, x0, wrow, pol_w);
+            tma_load_2d_pair(st1 + w_off, &tm_w, full0 + 8u * g + 8u, x0 + 128, wrow, pol_w);
             for (int b = 0; b < boxes; ++b) {
-              tma_load_2d_pair(st0 + tok_off + b * box_pitch, mb, full0[g], x0, my_row + box_rows * b, pol_b);
-              tma_load_2d_pair(st1 + tok_off + b * box_pitch, mb, full0[g + 1], x0 + 128, my_row + box_rows * b, pol_b);
+              tma_load_2d_pair(st0 + tok_off + b * box_pitch, mb, full0 + 8u * g, x0, my_row + box_rows * b, pol_b);
+              tma_load_2d_pair(st1 + tok_off + b * box_pitch, mb, full0 + 8u * g + 8u, x0 + 128, my_row + box_rows * b, pol_b);
             }
             ++it;
             g += 2;
@@ -399,19 +454,22 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           const uint32_t armed = 2 * it;
           const uint32_t first = armed > static_cast<uint32_t>(G) ? armed - G : 0;
           for (uint32_t i = first; i < armed; ++i)
-            mbar_wait_bounded_tell(&full[i % G], (i / G) & 1, s_abort, peer_abort, kStatusWaitTimeoutProducer, 1ll << 28);
+            mbar_wait_bounded_tell(smem_u32(&full[i % G]), (i / G) & 1, abort_flag, peer_abort, kStatusWaitTimeoutProducer, 1ll << 28);
         }
       }
       __syncwarp();
     } else if (warp == 1) {
       // --------------------------------------------------------------- MMA issuer for the even K blocks
-      if (lane == 0 && rank == 0) mma_role(0);
+      if (lane == 0 && rank == 0) {
+        if constexpr (MODE == 1) mma_halves(0);
+        else mma_whole();
+      }
       __syncwarp();
     } else if (warp == 2) {
       // --------------------------------------------------------------- scale warp
       if (MODE == 1) {
         // ------------------------------------------------------------- MMA issuer for the odd K blocks
-        if (lane == 0 && rank == 0) mma_role(1);
+        if (lane == 0 && rank == 0) mma_halves(1);
         __syncwarp();
       } else {
         // entry s of the ring holds, for one K block, act_scale[row, kb] * w_scale[kb] of every token column
@@ -448,7 +506,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
               const float ws = __shfl_sync(0xffffffffu, ws_a, kb0 + k);
-              bool ok = mbar_wait_bounded_tell(&sempty[s], sp ^ 1u, s_abort, peer_abort, kStatusWaitTimeoutProducer, p.wait_limit);
+              bool ok = mbar_wait_bounded_tell(smem_u32(&sempty[s]), sp ^ 1u, abort_flag, peer_abort, kStatusWaitTimeoutProducer, p.wait_limit);
               ok = __all_sync(0xffffffffu, ok);
               if (!ok) { alive = false; break; }
               *reinterpret_cast<float4*>(s_scale + s * SE + col) =
@@ -522,7 +580,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const int tl = q * 32 + lane;                 // tensor-memory lane: mode 1 token of this CTA, mode 2 feature
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t mapa_tempty = mapa_u32(smem_u32(&tempty[0]), 0);   // the first CTA's tempty[0]; the others follow at 8 bytes each
-    uint32_t sl = 0, sph = 0;                     // accumulator slot and its phase
+    const int half = grp >> 1;                    // mode 1: which half of the features
+    uint32_t sl = 0, sph = 0;                     // accumulator slot (mode 1: of this half) and its phase
     uint32_t s = 0, sp = 0;                       // scale ring entry and its phase
     uint32_t wp = 0;                              // phase bits of wfull[0..1] (mode 1)
     bool ok = true;
@@ -532,67 +591,61 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const long long st_start = clock64();
     (void)st_start; (void)inv_ratio; (void)wp;
 
-    if (MODE == 1 && my_items > 0) {
-      // activation scales of the first item (later items: fetched during the previous item's epilogue)
-      int eh = 0;
-      const PItem f = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(0), eh);
-      const int nrows = rank == 0 ? min(f.n, 128) : max(f.n - 128, 0);
-      const float* src = p.act_scale + static_cast<size_t>(grp) * (kHBlocks / 4) * p.row_cap + f.row_start + 128 * rank + tl;
-#pragma unroll
-      for (int k = 0; k < kHBlocks / 4; ++k)
-        s_scale[(grp * (kHBlocks / 4) + k) * 128 + tl] = tl < nrows ? __ldg(src + static_cast<size_t>(k) * p.row_cap) : 0.0f;
-      named_bar_sync(1 + q, 128);
-    }
     for (int i = 0; i < my_items; ++i) {
       const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
 
       if (MODE == 1) {
-        // ===== token-major: lane = token, columns [32 grp, +32) = up, [128 + 32 grp, +32) = gate
+        // ===== token-major: lane = token; the half's accumulator has its 64 up columns, then its 64 gate columns
         const int par = i & 1;
         const float* ws = s_ws + par * 128;
-        if (ok && !mbar_wait_bounded_tell(&wfull[par], (wp >> par) & 1u, s_abort, peer_abort,
+        if (ok && !mbar_wait_bounded_tell(smem_u32(&wfull[par]), (wp >> par) & 1u, abort_flag, peer_abort,
                                           kStatusWaitTimeoutEpilogue, p.wait_limit)) ok = false;
         wp ^= 1u << par;
         float up[32], gt[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) { up[j] = 0.0f; gt[j] = 0.0f; }
-        for (int kb = 0; kb < KB && ok; ++kb) {
-          // block scale of this thread's token: its activation scale (staged in shared memory for the whole
-          // item, see the end of the previous item) times the weight scales of the up and the gate block
-          const float a = s_scale[kb * 128 + tl];
-          const float su = a * ws[kb], sg = a * ws[64 + kb];
-          ST_BEGIN();
-          if (!mbar_wait_bounded_tell(&tfull[sl], sph, s_abort, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
-          ST_END(0);
-          tc_fence_after();
+        for (int buf = 0; buf < 2; ++buf) {
+          if (!ok || !mbar_wait_bounded_tell(smem_u32(&sfull[buf]), par, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+          const float* sc = s_scale + buf * kScaleChunk * 128 + tl;
+          const float* wk = ws + buf * kScaleChunk;
+          for (int k = 0; k < kScaleChunk; ++k) {
+            // block scale of this thread's token: its activation scale times the weight scales of the up and the gate block
+            const float a = sc[k * 128];
+            const float su = a * wk[k], sg = a * wk[64 + k];
+            ST_BEGIN();
+            if (!mbar_wait_bounded_tell(smem_u32(&tfull[2 * sl + half]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+            ST_END(0);
+            tc_fence_after();
 #ifdef SYFI_PAIR_STATS
-          const long long st_p0 = clock64();
+            const long long st_p0 = clock64();
 #endif
-          const uint32_t t0 = lane_addr + sl * kSlotCols + grp * 32;
-          // scalar FMAs (measured faster here than packed f32x2 ones, whose operand pairs cost extra moves);
-          // the slot goes back to the MMA thread as soon as its last values are in registers
+            const uint32_t t0 = lane_addr + (2 * sl + half) * kSlotCols + (grp & 1) * 32;
+            // eight columns at a time: with sixteen the compiler keeps 30 values in local memory
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const bool is_gate = c >= 2;
-            const int cc = c & 1;
-            uint32_t r[16];
-            tmem_ld16(t0 + (is_gate ? 128 : 0) + cc * 16, r);
-            tmem_ld_wait();
-            if (c == 3) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster_relaxed(mapa_tempty + 8u * sl);
-            }
+            for (int c = 0; c < 8; ++c) {
+              uint32_t r[8];
+              tmem_ld8(t0 + (c >> 2) * 64 + (c & 3) * 8, r);
+              tmem_ld_wait_for(r);
+              if (c == 7) {      // the slot goes back as soon as its last values are in registers
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster_relaxed(mapa_tempty + 8u * (2 * sl + half));
+              }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (!is_gate) up[cc * 16 + j] = fmaf(__uint_as_float(r[j]), su, up[cc * 16 + j]);
-              else gt[cc * 16 + j] = fmaf(__uint_as_float(r[j]), sg, gt[cc * 16 + j]);
+              for (int j = 0; j < 8; ++j) {
+                float& acc = c < 4 ? up[c * 8 + j] : gt[(c - 4) * 8 + j];
+                acc = fmaf(__uint_as_float(r[j]), c < 4 ? su : sg, acc);
+              }
             }
+            sl ^= 1u;
+            if (sl == 0) sph ^= 1u;
+#ifdef SYFI_PAIR_STATS
+            st_acc[2] += clock64() - st_p0;
+#endif
           }
-          if (++sl == kSlots) { sl = 0; sph ^= 1u; }
-#ifdef SYFI_PAIR_STATS
-          st_acc[2] += clock64() - st_p0;
-#endif
+          if (!ok) break;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sempty[buf]);   // the buffer goes back to the producer
         }
         if (ok) {   // the weight scales go back to the producer
           __syncwarp();
@@ -603,19 +656,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // column quarter), two-term requantisation; the fast exp and divide are a few ulp off the exact ones,
         // far below the 8-bit requantisation that follows
         const int my_rows = ok ? (rank == 0 ? min(im.n, 128) : max(im.n - 128, 0)) : 0;
-        // the next item's activation scales are requested now (this thread: 14 K blocks of its token) and
-        // stored once every warp of this lane quarter has left the K loop (the barrier below)
-        float nxt[kHBlocks / 4];
-        {
-          const bool more = i + 1 < my_items;
-          int eh = e_hint;
-          const PItem nx = more ? decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i + 1), eh) : PItem{0, 0, 0, 0};
-          const int nrows = rank == 0 ? min(nx.n, 128) : max(nx.n - 128, 0);
-          const float* src = p.act_scale + static_cast<size_t>(grp) * (kHBlocks / 4) * p.row_cap + nx.row_start + 128 * rank + tl;
-#pragma unroll
-          for (int k = 0; k < kHBlocks / 4; ++k)
-            nxt[k] = (more && tl < nrows) ? __ldg(src + static_cast<size_t>(k) * p.row_cap) : 0.0f;
-        }
         float c[32];
         float amax = 0.0f;
 #pragma unroll
@@ -624,12 +664,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           c[j] = g * __fdividef(1.0f, 1.0f + __expf(-g)) * up[j];
           amax = fmaxf(amax, fabsf(c[j]));
         }
-        float* red = s_red;
+        float* red = s_red + par * 4 * 128;     // (two in turn: one barrier per item)
         red[grp * 128 + tl] = amax;
         named_bar_sync(1 + q, 128);             // the four warps that share this lane quarter
         amax = fmaxf(fmaxf(red[tl], red[128 + tl]), fmaxf(red[256 + tl], red[384 + tl]));
-#pragma unroll
-        for (int k = 0; k < kHBlocks / 4; ++k) s_scale[(grp * (kHBlocks / 4) + k) * 128 + tl] = nxt[k];
         if (tl < my_rows) {
           const float scv = fmaxf(amax * (1.0f / 448.0f), 1e-12f);
           const float inv = 1.0f / scv;
@@ -658,7 +696,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           *reinterpret_cast<uint4*>(p.c_lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
           *reinterpret_cast<uint4*>(p.c_lo + off + 16) = make_uint4(lw[4], lw[5], lw[6], lw[7]);
         }
-        named_bar_sync(1 + q, 128);             // the next item's scales are in place, the amax exchange is free
         // hand the item to the publisher warp (see grouped_gemm.cu)
         __threadfence_block();
         __syncwarp();
@@ -674,10 +711,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         for (int j = 0; j < CN / 2; ++j) acc[j] = 0ull;
         for (int kb = 0; kb < KB && ok; ++kb) {
           ST_BEGIN();
-          if (!mbar_wait_bounded_tell(&tfull[sl], sph, s_abort, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+          if (!mbar_wait_bounded_tell(smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
           ST_END(0);
           tc_fence_after();
-          if (!mbar_wait_bounded_tell(&sfull[s], sp, s_abort, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+          if (!mbar_wait_bounded_tell(smem_u32(&sfull[s]), sp, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
 #ifdef SYFI_PAIR_STATS
           const long long st_p0 = clock64();
 #endif
@@ -757,8 +794,7 @@ template <int MODE>
 cudaError_t launch_pair(const PairGemmLaunch& g, const PairArgs& a, int num_sms, cudaStream_t st) {
   const int grid = num_sms & ~1;   // whole pairs
   return launch_dependent(pair_gemm_kernel<MODE>, dim3(grid), dim3(kPairThreads),
-                          static_cast<size_t>(PairCfg<MODE>::kSmemBytes), st, g.tm_w, g.tm_b0, g.tm_b1, g.tm_b0w, g.tm_b1w,
-                          a);
+                          static_cast<size_t>(PairCfg<MODE>::kSmemBytes), st, g.tm_w, g.tm_b0, g.tm_b1, g.tm_b0w, g.tm_sc, a);
 }
 
 }  // namespace

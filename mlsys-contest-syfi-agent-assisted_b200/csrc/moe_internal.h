@@ -129,8 +129,8 @@ struct PairGemmLaunch {
   CUtensorMap tm_w;    // weights, 2-D [E * rows_per_expert, K], box 128 x 128
   CUtensorMap tm_b0;   // GEMM1: a_perm; GEMM2: c_hi; box 32 x 128
   CUtensorMap tm_b1;   // GEMM2: c_lo (unused by GEMM1)
-  CUtensorMap tm_b0w;  // the same tensors with 128-row boxes (tiles of more than 64 rows: one load instead of four)
-  CUtensorMap tm_b1w;
+  CUtensorMap tm_b0w;  // the same with 128-row boxes (tiles of more than 64 rows: one load instead of four); GEMM2: both terms, c_lo's rows behind c_hi's
+  CUtensorMap tm_sc;   // GEMM1: a_scale as f32 [56, row_cap], box 28 x 128 (half the K blocks of a CTA's token rows)
   long long wait_limit = 1ll << 32;   // SM clocks a device-side wait may take (about two seconds)
   int silent_producer = 0;            // test hook, see syfi_moe_debug_fault
   int rows_to_targets = 0;            // GEMM2 stores row r at Workspace::row_out[r] instead of o_rows

@@ -180,6 +180,13 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The same, naming the registers of the load it waits for, so that no arithmetic on them can move in front of it.
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :: "memory");
+}
+
 // Packed pairs of f32 (sm_100 issues one FMA or multiply on both halves per instruction; each half is
 // the IEEE operation, so results equal the scalar ones bit for bit).
 __device__ __forceinline__ uint64_t f32x2_pack(float lo, float hi) {
@@ -291,17 +298,30 @@ __device__ __forceinline__ bool mbar_wait_bounded_pair(uint64_t* bar, uint32_t p
 }
 // The same for barriers that only this CTA's threads, its own loads or tcgen05.commit signal (CTA-scope
 // acquire), still telling the partner when it gives up.  (Polling with mbarrier.test_wait instead of
-// try_wait was measured and changed nothing.)
-__device__ __forceinline__ bool mbar_wait_bounded_tell(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                       uint32_t peer_abort_cluster_addr, int code,
-                                                       long long limit_cycles = (1ll << 31)) {
-  if (mbar_try_wait(bar, parity)) return true;
+// try_wait was measured and changed nothing.)  Shared-memory addresses, not pointers: the promotion warps have no
+// registers to spare for 64-bit ones.
+__device__ __forceinline__ bool mbar_wait_bounded_tell(uint32_t bar, uint32_t parity, uint32_t abort_flag, uint32_t peer_abort_cluster_addr,
+                                                       int code, long long limit_cycles) {
+  auto try_wait = [&]() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  if (try_wait()) return true;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag != 0) return false;
+    if (try_wait()) return true;
+    int aborted;
+    asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(aborted) : "r"(abort_flag) : "memory");
+    if (aborted != 0) return false;
     if (clock64() - t0 > limit_cycles) {
-      *abort_flag = code;
+      asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(abort_flag), "r"(code) : "memory");
       st_cluster_u32(peer_abort_cluster_addr, static_cast<uint32_t>(code));
       return false;
     }
@@ -338,7 +358,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mas
                ::"r"(smem_u32(bar)), "h"(cta_mask)
                : "memory");
 }
-__device__ __forceinline__ uint32_t umma_idesc_e4m3_m256(uint32_t n) {
+__host__ __device__ constexpr uint32_t umma_idesc_e4m3_m256(uint32_t n) {
   return (1u << 4) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
 // Tiled load into THIS CTA's shared memory whose completion is counted on an mbarrier that may live in
