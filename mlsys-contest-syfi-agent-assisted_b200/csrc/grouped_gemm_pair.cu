@@ -37,7 +37,7 @@
 //
 // Roles per CTA: warp 0 = TMA producer (one thread; mode 1: the activation and weight scales too), warp 1 = tensor memory
 // owner and, in the pair's first CTA, MMA issuer (mode 1: of the even K blocks), warp 2 = issuer of the odd K blocks
-// (mode 1) / scale warp (mode 2: multiplies a K block's activation scales with its weight scale into a shared-memory ring),
+// (mode 1) / scale warp (mode 2: multiplies an item's activation scales with its weight scales into shared memory),
 // warp 3 = cross-kernel bookkeeping (as in grouped_gemm.cu), warps 4..19 = promotion / epilogue
 // (a warp reads one tensor-memory lane quarter; four warps share a quarter and split the columns).
 // An expert's last rows, up to 128 that would leave a 256-row tile at most half full, are not this GEMM1's but the
@@ -58,7 +58,6 @@ namespace {
 constexpr int kTile = 128 * 128;             // operand tile: 128 rows x 128 bytes of K
 constexpr int kBox = 32 * 128;               // token-side TMA box: 32 rows x 128 bytes
 constexpr int kStageBytes = 2 * kTile;       // one K block: M-side tile, then N-side tile
-constexpr int kScaleRing = 16;               // mode 2: K blocks of scales in flight
 constexpr int kScaleChunk = kHBlocks / 2;    // mode 1: K blocks per buffer of activation scales (two buffers hold an item's)
 constexpr int kEpiWarps = 16;
 constexpr int kEpiThreads = 32 * kEpiWarps;
@@ -74,9 +73,9 @@ template <int MODE> struct PairCfg {
   static constexpr int kSlots = MODE == 1 ? 4 : 2;
   static constexpr int kSlotCols = kPairTmemCols / kSlots;
   static constexpr int kScaleEntry = 128;   // floats per K block: one per token lane (mode 1) / token column (mode 2)
-  // mode 1: the activation scales of a whole item, [56][128], in two buffers; mode 2: a ring of K blocks of scale products
-  static constexpr int kScaleFloats = MODE == 1 ? kHBlocks * 128 : kScaleRing * kScaleEntry;
-  static constexpr int kScaleBufs = MODE == 1 ? 2 : kScaleRing;
+  // mode 1: the activation scales of a whole item, [56][128], in two buffers; mode 2: an item's scale products, [16][128], twice
+  static constexpr int kScaleFloats = (MODE == 1 ? kHBlocks : 2 * kIBlocks) * kScaleEntry;
+  static constexpr int kScaleBufs = 2;
   static constexpr int kBarriers = kStages + kStages / 2 + 2 * kMaxSlots + 2 * kScaleBufs + 4;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleFloats * 4 +
                                     (MODE == 1 ? 2 * 4 * 128 * 4 + 2 * 128 * 4 : 0) + 8 * kBarriers +
@@ -169,15 +168,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  float* s_scale = reinterpret_cast<float*>(smem + G * kStageBytes);           // mode 1: [56][128]; mode 2: [kScaleRing][SE]
+  float* s_scale = reinterpret_cast<float*>(smem + G * kStageBytes);           // mode 1: [56][128]; mode 2: [2][16][128]
   float* s_red = s_scale + C::kScaleFloats;                                    // [2][4][128] partial amax of an item (mode 1)
   float* s_ws = s_red + (MODE == 1 ? 2 * 4 * 128 : 0);                         // [2][128] weight scales of an item (mode 1)
   uint64_t* full = reinterpret_cast<uint64_t*>(s_ws + (MODE == 1 ? 2 * 128 : 0));   // [G]   first CTA's are used
   uint64_t* empty = full + G;                                                  // [G/2] per CTA
   uint64_t* tfull = empty + G / 2;                                             // [4]   per CTA
   uint64_t* tempty = tfull + kMaxSlots;                                        // [4]   first CTA's are used
-  uint64_t* sfull = tempty + kMaxSlots;                                        // [2 or 16] per CTA
-  uint64_t* sempty = sfull + C::kScaleBufs;                                    // [2 or 16] per CTA
+  uint64_t* sfull = tempty + kMaxSlots;                                        // [2]   per CTA
+  uint64_t* sempty = sfull + C::kScaleBufs;                                    // [2]   per CTA
   uint64_t* wfull = sempty + C::kScaleBufs;                                       // [2]   mode 1: an item's weight scales are there
   uint64_t* wempty = wfull + 2;                                                // [2]
   ExpertWork* s_work = reinterpret_cast<ExpertWork*>(wempty + 2);
@@ -472,10 +471,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         if (lane == 0 && rank == 0) mma_halves(1);
         __syncwarp();
       } else {
-        // entry s of the ring holds, for one K block, act_scale[row, kb] * w_scale[kb] of every token column
-        // of the item; lane l serves columns 4 l .. 4 l + 3
+        // a buffer holds act_scale[row, kb] * w_scale[kb] of an item's K blocks and token columns; lane l serves columns
+        // 4 l .. 4 l + 3
         constexpr int kBatch = 4;
-        uint32_t s = 0, sp = 0;
         uint32_t n_items = 0;
         int e_hint = 0;
         bool alive = true;
@@ -496,7 +494,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           const int col = 4 * lane;
           const bool v0 = col < im.n;
           const float* src = p.act_scale + im.row_start + col;
-          for (int kb0 = 0; kb0 < KB && alive; kb0 += kBatch) {
+          float* dst = s_scale + (i & 1) * KB * SE + col;
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded_tell(smem_u32(&sempty[i & 1]), ((i >> 1) & 1) ^ 1u, abort_flag, peer_abort,
+                                                              kStatusWaitTimeoutProducer, p.wait_limit))) break;
+          for (int kb0 = 0; kb0 < KB; kb0 += kBatch) {
             float4 a[kBatch];
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
@@ -506,16 +507,11 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
               const float ws = __shfl_sync(0xffffffffu, ws_a, kb0 + k);
-              bool ok = mbar_wait_bounded_tell(smem_u32(&sempty[s]), sp ^ 1u, abort_flag, peer_abort, kStatusWaitTimeoutProducer, p.wait_limit);
-              ok = __all_sync(0xffffffffu, ok);
-              if (!ok) { alive = false; break; }
-              *reinterpret_cast<float4*>(s_scale + s * SE + col) =
-                  make_float4(a[k].x * ws, a[k].y * ws, a[k].z * ws, a[k].w * ws);
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&sfull[s]);
-              if (++s == kScaleRing) { s = 0; sp ^= 1u; }
+              *reinterpret_cast<float4*>(dst + (kb0 + k) * SE) = make_float4(a[k].x * ws, a[k].y * ws, a[k].z * ws, a[k].w * ws);
             }
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sfull[i & 1]);
         }
       }
     } else {
@@ -582,7 +578,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const uint32_t mapa_tempty = mapa_u32(smem_u32(&tempty[0]), 0);   // the first CTA's tempty[0]; the others follow at 8 bytes each
     const int half = grp >> 1;                    // mode 1: which half of the features
     uint32_t sl = 0, sph = 0;                     // accumulator slot (mode 1: of this half) and its phase
-    uint32_t s = 0, sp = 0;                       // scale ring entry and its phase
     uint32_t wp = 0;                              // phase bits of wfull[0..1] (mode 1)
     bool ok = true;
     int e_hint = 0;
@@ -709,49 +704,51 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         uint64_t acc[CN / 2];
 #pragma unroll
         for (int j = 0; j < CN / 2; ++j) acc[j] = 0ull;
-        for (int kb = 0; kb < KB && ok; ++kb) {
-          ST_BEGIN();
-          if (!mbar_wait_bounded_tell(smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
-          ST_END(0);
-          tc_fence_after();
-          if (!mbar_wait_bounded_tell(smem_u32(&sfull[s]), sp, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+        // One wait for the scales per item, and two K blocks per trip with their slots as constants: with a ring of scales per
+        // K block and a running slot the promotion, which bounds this mode, had two waits and more address arithmetic per K
+        // block (us per call 4096 tokens 512 / 501 and 586 / 573, 8192 tokens 864 / 843, 16384 with hot experts 2886 / 2842).
+        if (ok && !mbar_wait_bounded_tell(smem_u32(&sfull[i & 1]), (i >> 1) & 1, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) ok = false;
+        const float* sc = s_scale + (i & 1) * KB * SE + c0;
+        for (int kb2 = 0; kb2 < KB && ok; kb2 += 2, sph ^= 1u, sc += 2 * SE) {
+#pragma unroll
+          for (int sl = 0; sl < 2; ++sl) {
+            ST_BEGIN();
+            if (!mbar_wait_bounded_tell(smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+            ST_END(0);
+            tc_fence_after();
 #ifdef SYFI_PAIR_STATS
-          const long long st_p0 = clock64();
+            const long long st_p0 = clock64();
 #endif
-          const float* sc = s_scale + s * SE + c0;
-          const uint32_t t0 = lane_addr + sl * kSlotCols + c0;
-          // (handing the slot back before the arithmetic of the last chunk, as mode 1 does, costs registers
-          // here and was slower: 400 us against 359 us)
+            const uint32_t t0 = lane_addr + sl * kSlotCols + c0;
+            // (handing the slot back before the arithmetic of the last chunk, as mode 1 does, costs registers
+            // here and was slower: 400 us against 359 us)
 #pragma unroll
-          for (int ch = 0; ch < CN / 16; ++ch) {
-            if (c0 + ch * 16 < n) {
-              const ulonglong2* sp4 = reinterpret_cast<const ulonglong2*>(sc + ch * 16);
-              uint32_t r[16], l[16];
-              tmem_ld16(t0 + ch * 16, r);                 // hi products
-              tmem_ld16(t0 + im.n + ch * 16, l);          // lo products of the same token columns
-              const ulonglong2 s0 = sp4[0], s1 = sp4[1], s2 = sp4[2], s3 = sp4[3];
-              tmem_ld_wait();
-              const uint64_t sv[8] = {s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, s3.y};
+            for (int ch = 0; ch < CN / 16; ++ch) {
+              if (c0 + ch * 16 < n) {
+                const ulonglong2* sp4 = reinterpret_cast<const ulonglong2*>(sc + sl * SE + ch * 16);
+                uint32_t r[16], l[16];
+                tmem_ld16(t0 + ch * 16, r);                 // hi products
+                tmem_ld16(t0 + im.n + ch * 16, l);          // lo products of the same token columns
+                const ulonglong2 s0 = sp4[0], s1 = sp4[1], s2 = sp4[2], s3 = sp4[3];
+                tmem_ld_wait();
+                const uint64_t sv[8] = {s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, s3.y};
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const uint64_t v = f32x2_fma(f32x2_pack_bits(l[2 * j], l[2 * j + 1]), inv_ratio,
-                                             f32x2_pack_bits(r[2 * j], r[2 * j + 1]));
-                acc[ch * 8 + j] = f32x2_fma(v, sv[j], acc[ch * 8 + j]);
+                for (int j = 0; j < 8; ++j) {
+                  const uint64_t v = f32x2_fma(f32x2_pack_bits(l[2 * j], l[2 * j + 1]), inv_ratio,
+                                               f32x2_pack_bits(r[2 * j], r[2 * j + 1]));
+                  acc[ch * 8 + j] = f32x2_fma(v, sv[j], acc[ch * 8 + j]);
+                }
               }
             }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_cluster_relaxed(mapa_tempty + 8u * sl);
-            mbar_arrive(&sempty[s]);
-          }
-          if (++sl == kSlots) { sl = 0; sph ^= 1u; }
-          if (++s == kScaleRing) { s = 0; sp ^= 1u; }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(mapa_tempty + 8u * sl);
 #ifdef SYFI_PAIR_STATS
-          st_acc[2] += clock64() - st_p0;
+            st_acc[2] += clock64() - st_p0;
 #endif
+          }
         }
+        if (ok && lane == 0) mbar_arrive(&sempty[i & 1]);   // every lane has read its scales: the __syncwarp above
         const int n_out = ok ? n : 0;               // a failed item stores nothing
         ST_BEGIN();
         float out[CN];

@@ -294,6 +294,30 @@ def test_rows_per_expert_at_the_edges_of_the_work_split(rows, pkg, oracle, monke
         assert torch.equal(outs[0], o)
 
 
+@pytest.mark.parametrize("rows", [(1300, 16, 400), (2100,), (256, 0, 137)])
+def test_pairs_with_several_items_in_turn_equal_the_64_row_kernels(rows, pkg, monkeypatch):
+    """A pair of CTAs that walks through many work items reuses its buffers of scales (two halves of GEMM1's K blocks, two
+    items of GEMM2) and its accumulator slots across items of different height; one item per pair, where nothing is reused,
+    with a second CTA that has few rows.  The sums are those of the single-CTA kernels, bit for bit, also unrounded."""
+    E, T = len(rows), max(rows) + 5
+    inp = pkg.make_inputs(num_tokens=T, seed=23, e_local=E, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    logits = torch.randn(T, 256, generator=g, device=DEV) * 0.3 - 2.0
+    logits[:, :32] = -9.0
+    for e, n in enumerate(rows):
+        logits[torch.randperm(T, generator=g, device=DEV)[:n], e] = 8.0
+    inp = pkg.MoeInputs(logits, torch.zeros_like(inp.routing_bias), *inp.args()[2:])
+    outs = []
+    for tile in (64, 256, 256):
+        monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", str(tile))
+        out = torch.full((T, 7168), float("nan"), dtype=torch.float32, device=DEV)
+        pkg.run_moe(*inp.args(), out)
+        pkg.get_context(0).check()
+        assert tuple(pkg.get_context(0).debug_read("counts", torch.int32)[0][:E].tolist()) == rows
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 @pytest.mark.parametrize("T,E,off", [(1, 1, 255), (2, 32, 64), (15, 3, 32), (16, 32, 0), (17, 32, 0)])
 def test_small_batches_equal_the_same_tokens_in_a_larger_one(T, E, off, pkg):
     """Up to 16 tokens the router, the row lists and the gather are one kernel: routes, weights, the tables and every
