@@ -234,9 +234,13 @@ const void* mapped_alias(const void* host) {
 // 529 / 473, 339 / 347, 443 / 414, 240 / 262; 3600 tokens 528 / 495, 345 / 363, 453 / 420, 267 / 265; 4000 tokens 554 / 533,
 // 382 / 381, 494 / 464, 278 / 268; 5000 tokens 655 / 597, 523 / 456, 631 / 595, 512 / 437: below the line one load gains
 // what another loses.
-// With fewer experts there are fewer tiles, and pairs pay off later: 8 experts, 64-row tiles / pairs,
-// 3600 tokens 156 / 167 and 94 / 104, 4500 tokens 193 / 177 and 103 / 113, from 6144 on the pairs.
+// With fewer experts there are fewer tiles, and pairs pay off later.  64-row tiles / pairs, us per call, four loads: 16 experts,
+// 4000 tokens 255 / 241, 363 / 317, 240 / 258, 174 / 182; 5000 tokens 365 / 318, 631 / 530, 292 / 276, 425 / 348; 8 experts, 4500
+// tokens 192 / 174, 203 / 185, 157 / 164, 87 / 96; 5000 tokens 241 / 202, 476 / 412, 178 / 175, 261 / 242; 5600 tokens 261 / 235,
+// 537 / 439, 191 / 195, 301 / 258; 4 experts, 5000 tokens 179 / 157, 448 / 351, 107 / 112, 248 / 195; 1 expert 147 / 127, 79 / 85,
+// 70 / 77, 36 / 42 (one kernel more, and few rows to gain on).
 constexpr int64_t kPairMinTokens = 3584;
+constexpr int64_t kPairMinTokens8Experts = 5000;
 constexpr int64_t kPairMinTokensAnyExperts = 6144;
 // The pair configuration's kernels count their own tiles; what the row lists count is a statistic (syfi_moe_check), of
 // 64-row tiles below this many tokens and of 128-row tiles from there on.
@@ -307,7 +311,7 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   // Large batches (experts with hundreds of rows each) run the CTA-pair kernels, which cut their own
   // token tiles (256 rows in GEMM1, 128 in GEMM2), and the 64-row GEMM1 on what tail_rows() leaves to it;
   // token_tile 256 stands for that configuration here.
-  const bool many = T64 >= kPairMinTokensAnyExperts || T64 * e_local >= kPairMinTokens * kMaxLocalExperts;
+  const bool many = T64 >= (e_local >= 8 ? kPairMinTokens8Experts : kPairMinTokensAnyExperts) || T64 * e_local >= kPairMinTokens * kMaxLocalExperts;
   int token_tile = (T64 <= 1024) ? 32 : (!many || packed) ? 64 : 256;
   if (const char* ov = getenv("SYFI_MOE_TOKEN_TILE")) {   // tuning knob: force 32, 64, 128 or (pair kernels) 256
     const int v = atoi(ov);
