@@ -156,11 +156,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float scale = valid ? __ldg(reinterpret_cast<const float*>(cache + static_cast<size_t>(page) * kPageBytes +
                                                                        kPage * kDim + (tl & (kPage - 1)) * 4))
                                 : 0.0f;
-      if (!mbar_wait_bounded(&tfull[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit)) {
-        // the rest of the run gets no score, see below
-        for (int r = t; r < n && r < t_begin + tiles * kTokTile; r += kTokTile) scores[static_cast<size_t>(b) * max_ls + r] = -INFINITY;
-        break;
-      }
+      mbar_wait_or_clear(alive, &tfull[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit);   // (failed: the rest of the run has no scores)
       tc_fence_after();
       float acc = 0.0f;
 #pragma unroll
@@ -177,8 +173,9 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         for (int j = 0; j < 16; ++j) acc = fmaf(s_w[c * 16 + j], fmaxf(__uint_as_float(r[j]) * scale, 0.0f), acc);
       }
       // no page here: below every score and outside the range, so that the selection never meets what an earlier call left
-      if (t < n) scores[static_cast<size_t>(b) * max_ls + t] = valid ? acc : -INFINITY;
-      if (valid) {
+      const bool scored = valid && alive;
+      if (t < n) scores[static_cast<size_t>(b) * max_ls + t] = scored ? acc : -INFINITY;
+      if (scored) {
         low = min(low, score_key(acc));
         high = max(high, score_key(acc));
       }

@@ -705,6 +705,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     if (MODE == 1 && EARLY) pdl_wait();     // the activation scales are the gather's
     // After a failed wait a warp keeps walking the work list and still joins every named
     // barrier below (doing no other work), so the epilogue warps can never strand each other.
+    // (Inside the K loop a failed lane goes on with the others: see mbar_wait_or_clear.)
     for (int i = 0; i < my_items; ++i) {
       const Item im = sched.item<FT, NT, SPLIT>(s_work, p.e_local, i, at);
       const int ft = im.ft;
@@ -750,7 +751,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         // rows' scales and are never read.
         s_act = s_scales + sbuf * kScaleStride;
         s_ws = s_act + KB * NT;
-        if (ok && !mbar_wait_bounded(&sfull[sbuf], (sph >> sbuf) & 1u, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) ok = false;
+        mbar_wait_or_clear(ok, &sfull[sbuf], (sph >> sbuf) & 1u, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
+        ok = __all_sync(0xffffffffu, ok);
         sph ^= 1u << sbuf;
       }
       if (et == 0) TRACE(2, 1001);
@@ -791,10 +793,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       };
       const int entries = (part && im.n <= 16 ? 4 : KPS) / TKPS;     // TMEM entries per smem ring entry (see Layout)
       int left = entries;
-      for (int ts = 0; ts < KB / TKPS && ok; ++ts) {
+      if (ok) for (int ts = 0; ts < KB / TKPS; ++ts) {
         const bool odd = ISSUERS == 2 && (g & 1u) != 0;
         const uint32_t pr = odd ? SUB + sub1 : sub0, pph = odd ? pph1 : pph0;
-        if (!mbar_wait_bounded(&tfull[pr], pph, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+        mbar_wait_or_clear(ok, &tfull[pr], pph, s_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
         tc_fence_after();
         if (et == 0) TRACE(2, ts);
 #pragma unroll
@@ -867,6 +869,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           if (++g == G) g = 0;
         }
       }
+      ok = __all_sync(0xffffffffu, ok);
       if (et == 0) TRACE(2, 1002);
       if (MODE == 2) {                        // the scale buffer goes back to the producer
         __syncwarp();

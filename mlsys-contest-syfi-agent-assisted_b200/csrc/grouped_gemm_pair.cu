@@ -593,14 +593,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // ===== token-major: lane = token; the half's accumulator has its 64 up columns, then its 64 gate columns
         const int par = i & 1;
         const float* ws = s_ws + par * 128;
-        if (ok && !mbar_wait_bounded_tell(smem_u32(&wfull[par]), (wp >> par) & 1u, abort_flag, peer_abort,
-                                          kStatusWaitTimeoutEpilogue, p.wait_limit)) ok = false;
+        mbar_wait_or_clear_tell(ok, smem_u32(&wfull[par]), (wp >> par) & 1u, abort_flag, peer_abort,
+                                kStatusWaitTimeoutEpilogue, p.wait_limit);
+        ok = __all_sync(0xffffffffu, ok);
         wp ^= 1u << par;
         float up[32], gt[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) { up[j] = 0.0f; gt[j] = 0.0f; }
-        for (int buf = 0; buf < 2; ++buf) {
-          if (!ok || !mbar_wait_bounded_tell(smem_u32(&sfull[buf]), par, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+        if (ok) for (int buf = 0; buf < 2; ++buf) {
+          mbar_wait_or_clear_tell(ok, smem_u32(&sfull[buf]), par, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
           const float* sc = s_scale + buf * kScaleChunk * 128 + tl;
           const float* wk = ws + buf * kScaleChunk;
           for (int k = 0; k < kScaleChunk; ++k) {
@@ -608,7 +609,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             const float a = sc[k * 128];
             const float su = a * wk[k], sg = a * wk[64 + k];
             ST_BEGIN();
-            if (!mbar_wait_bounded_tell(smem_u32(&tfull[2 * sl + half]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+            mbar_wait_or_clear_tell(ok, smem_u32(&tfull[2 * sl + half]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
             ST_END(0);
             tc_fence_after();
 #ifdef SYFI_PAIR_STATS
@@ -638,14 +639,11 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             st_acc[2] += clock64() - st_p0;
 #endif
           }
-          if (!ok) break;
           __syncwarp();
           if (lane == 0) mbar_arrive(&sempty[buf]);   // the buffer goes back to the producer
         }
-        if (ok) {   // the weight scales go back to the producer
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&wempty[par]);
-        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0 && ok) mbar_arrive(&wempty[par]);     // the weight scales go back to the producer
         ST_BEGIN();
         // ---- SwiGLU of this token's 32 features, amax over the token's 128 features (four threads, one per
         // column quarter), two-term requantisation; the fast exp and divide are a few ulp off the exact ones,
@@ -700,20 +698,21 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // ===== feature-major: lane = output feature, columns [32 grp, +32) = hi, [n + 32 grp, +32) = lo
         constexpr int CN = 32;
         const int c0 = grp * CN;
-        const int n = ok ? im.n : 0;
         uint64_t acc[CN / 2];
 #pragma unroll
         for (int j = 0; j < CN / 2; ++j) acc[j] = 0ull;
         // One wait for the scales per item, and two K blocks per trip with their slots as constants: with a ring of scales per
         // K block and a running slot the promotion, which bounds this mode, had two waits and more address arithmetic per K
         // block (us per call 4096 tokens 512 / 501 and 586 / 573, 8192 tokens 864 / 843, 16384 with hot experts 2886 / 2842).
-        if (ok && !mbar_wait_bounded_tell(smem_u32(&sfull[i & 1]), (i >> 1) & 1, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) ok = false;
+        mbar_wait_or_clear_tell(ok, smem_u32(&sfull[i & 1]), (i >> 1) & 1, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
+        ok = __all_sync(0xffffffffu, ok);
+        const int n = ok ? im.n : 0;
         const float* sc = s_scale + (i & 1) * KB * SE + c0;
-        for (int kb2 = 0; kb2 < KB && ok; kb2 += 2, sph ^= 1u, sc += 2 * SE) {
+        if (ok) for (int kb2 = 0; kb2 < KB; kb2 += 2, sph ^= 1u, sc += 2 * SE) {
 #pragma unroll
           for (int sl = 0; sl < 2; ++sl) {
             ST_BEGIN();
-            if (!mbar_wait_bounded_tell(smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit)) { ok = false; break; }
+            mbar_wait_or_clear_tell(ok, smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
             ST_END(0);
             tc_fence_after();
 #ifdef SYFI_PAIR_STATS
@@ -748,6 +747,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #endif
           }
         }
+        ok = __all_sync(0xffffffffu, ok);
         if (ok && lane == 0) mbar_arrive(&sempty[i & 1]);   // every lane has read its scales: the __syncwarp above
         const int n_out = ok ? n : 0;               // a failed item stores nothing
         ST_BEGIN();

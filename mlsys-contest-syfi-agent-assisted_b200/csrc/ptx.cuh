@@ -67,6 +67,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for the warps that read tensor memory.  Each lane asks for itself and the lanes may disagree about a wait that
+// runs out, but the loads of tensor memory and the shuffles behind them need all 32: so a failed lane clears `ok`, stays in
+// its loop without waiting any more, and the warp votes on `ok` behind the loop.  (Nothing but the wait's fast path is
+// executed where it succeeds; leaving by `ok` before each wait and each arrival cost the CTA pairs 1 %.)
+__device__ __forceinline__ void mbar_wait_or_clear(bool& ok, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                   int code, long long limit_cycles) {
+  if (!mbar_try_wait(bar, parity) && ok) ok = mbar_wait_bounded(bar, parity, abort_flag, code, limit_cycles);
+}
+
 // Cross-CTA hand-off through a counter in global memory: the writers' data stores happen before the
 // release increment, the reader's acquire load happens before its dependent loads.  The proxy fence
 // orders generic-proxy accesses against async-proxy ones (TMA), which otherwise have no mutual order.
@@ -296,27 +305,27 @@ __device__ __forceinline__ bool mbar_wait_bounded_pair(uint64_t* bar, uint32_t p
     }
   }
 }
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // The same for barriers that only this CTA's threads, its own loads or tcgen05.commit signal (CTA-scope
 // acquire), still telling the partner when it gives up.  (Polling with mbarrier.test_wait instead of
 // try_wait was measured and changed nothing.)  Shared-memory addresses, not pointers: the promotion warps have no
 // registers to spare for 64-bit ones.
 __device__ __forceinline__ bool mbar_wait_bounded_tell(uint32_t bar, uint32_t parity, uint32_t abort_flag, uint32_t peer_abort_cluster_addr,
                                                        int code, long long limit_cycles) {
-  auto try_wait = [&]() {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-  };
-  if (try_wait()) return true;
+  if (mbar_try_wait_at(bar, parity)) return true;
   const long long t0 = clock64();
   while (true) {
-    if (try_wait()) return true;
+    if (mbar_try_wait_at(bar, parity)) return true;
     int aborted;
     asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(aborted) : "r"(abort_flag) : "memory");
     if (aborted != 0) return false;
@@ -326,6 +335,12 @@ __device__ __forceinline__ bool mbar_wait_bounded_tell(uint32_t bar, uint32_t pa
       return false;
     }
   }
+}
+// as mbar_wait_or_clear
+__device__ __forceinline__ void mbar_wait_or_clear_tell(bool& ok, uint32_t bar, uint32_t parity, uint32_t abort_flag,
+                                                        uint32_t peer_abort_cluster_addr, int code, long long limit_cycles) {
+  if (!mbar_try_wait_at(bar, parity) && ok)
+    ok = mbar_wait_bounded_tell(bar, parity, abort_flag, peer_abort_cluster_addr, code, limit_cycles);
 }
 // Tensor memory of both CTAs of the pair: the same warp of each CTA executes these.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {

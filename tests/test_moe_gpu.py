@@ -849,6 +849,25 @@ def test_bounded_waits_run_out_and_the_context_recovers(T, E, tile, mask, expect
     assert torch.equal(before, after)
 
 
+@pytest.mark.parametrize("T,E,tile", [(200, 8, None), (40, 3, None), (300, 4, 64), (300, 4, 128), (700, 4, 256)])
+def test_waits_that_run_out_at_once_leave_whole_warps(T, E, tile, pkg, monkeypatch):
+    """The lanes of a promotion warp ask a barrier each for itself; the loads of tensor memory and the shuffles behind it
+    need all 32.  With a limit of a few clocks every lane's first look may be the one that gives up, in every item that the
+    warp walks through; nothing is on its way, as the producer is silent."""
+    if tile is not None:
+        monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", str(tile))
+    inp = pkg.make_inputs(num_tokens=T, seed=44, e_local=E, device=DEV)
+    before, _ = _run(pkg, inp)
+    ctx = pkg.get_context(0)
+    for limit in (1, 40, 700):
+        ctx.debug_fault(1 | 4, limit)
+        pkg.run_moe(*inp.args(), torch.empty_like(before))
+        with pytest.raises(pkg.MoeError, match="status 10[23]"):
+            ctx.check()
+        after, _ = _run(pkg, inp)
+        assert torch.equal(before, after), limit
+
+
 def test_row_capacity_overflow_is_reported_not_written(pkg):
     """The workspace holds 3 rows per token beyond 2048 tokens (a token sends about one of its 8 routes to 32 of
     256 experts).  Every local expert made hot sends far more: the row-list kernel refuses to write past the
