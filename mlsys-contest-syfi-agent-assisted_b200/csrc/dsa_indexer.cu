@@ -163,7 +163,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int c = 0; c < kHeads / 16; ++c) {
         uint32_t r[16];
         tmem_ld16(lane_addr + st * kHeads + c * 16, r);
-        tmem_ld_wait();
+        tmem_ld_wait_for(r);
         if (c == kHeads / 16 - 1) {            // the accumulator is in registers: hand it back
           tc_fence_before();
           __syncwarp();

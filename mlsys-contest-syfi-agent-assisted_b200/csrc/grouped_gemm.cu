@@ -811,13 +811,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (part) {
               uint32_t r0[16];
               tmem_ld16(t0, r0);
-              tmem_ld_wait();
+              tmem_ld_wait_for(r0);
               promote16(r0, r0, 0, sa, ws0, ws0, 0);
             } else if constexpr (CN == 16) {  // both accumulators of this thread's 16 columns in flight
               uint32_t r0[16], r1[16];
               tmem_ld16(t0, r0);
               tmem_ld16(t0 + (MODE == 1 ? NT : lo_col), r1);
-              tmem_ld_wait();
+              tmem_ld_wait_for(r0, r1);
               promote16(r0, r1, 0, sa, ws0, ws1, 2);
             } else if constexpr (NT == 128 && MODE == 1) {
               // 18 warps share the register file and 64 registers of a thread hold accumulators: eight
@@ -829,13 +829,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
                   const ulonglong2 s03 = sp[0], s47 = sp[1];
                   uint32_t r[8];
                   tmem_ld8(t0 + c * 8, r);
-                  tmem_ld_wait();
+                  tmem_ld_wait_for(r);
                   acc0p[c * 4 + 0] = f32x2_fma(f32x2_pack_bits(r[0], r[1]), f32x2_mul(s03.x, ws0), acc0p[c * 4 + 0]);
                   acc0p[c * 4 + 1] = f32x2_fma(f32x2_pack_bits(r[2], r[3]), f32x2_mul(s03.y, ws0), acc0p[c * 4 + 1]);
                   acc0p[c * 4 + 2] = f32x2_fma(f32x2_pack_bits(r[4], r[5]), f32x2_mul(s47.x, ws0), acc0p[c * 4 + 2]);
                   acc0p[c * 4 + 3] = f32x2_fma(f32x2_pack_bits(r[6], r[7]), f32x2_mul(s47.y, ws0), acc0p[c * 4 + 3]);
                   tmem_ld8(t0 + NT + c * 8, r);
-                  tmem_ld_wait();
+                  tmem_ld_wait_for(r);
                   acc1p[c * 4 + 0] = f32x2_fma(f32x2_pack_bits(r[0], r[1]), f32x2_mul(s03.x, ws1), acc1p[c * 4 + 0]);
                   acc1p[c * 4 + 1] = f32x2_fma(f32x2_pack_bits(r[2], r[3]), f32x2_mul(s03.y, ws1), acc1p[c * 4 + 1]);
                   acc1p[c * 4 + 2] = f32x2_fma(f32x2_pack_bits(r[4], r[5]), f32x2_mul(s47.x, ws1), acc1p[c * 4 + 2]);
@@ -849,7 +849,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
                   uint32_t r0[16], r1[16];
                   tmem_ld16(t0 + c * 16, r0);
                   tmem_ld16(t0 + lo_col + c * 16, r1);
-                  tmem_ld_wait();
+                  tmem_ld_wait_for(r0, r1);
                   promote16(r0, r1, c * 16, sa + c * 16, ws0, ws1, 2);
                 }
               }

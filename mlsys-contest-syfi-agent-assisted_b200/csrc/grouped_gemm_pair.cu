@@ -729,7 +729,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 tmem_ld16(t0 + ch * 16, r);                 // hi products
                 tmem_ld16(t0 + im.n + ch * 16, l);          // lo products of the same token columns
                 const ulonglong2 s0 = sp4[0], s1 = sp4[1], s2 = sp4[2], s3 = sp4[3];
-                tmem_ld_wait();
+                tmem_ld_wait_for(r, l);
                 const uint64_t sv[8] = {s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, s3.y};
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
