@@ -80,8 +80,8 @@ template <int MODE, int NT> struct Cfg {
   static constexpr int kThreads = 64 + 128 * kColSplit + 64;
   static constexpr int kSmemBytes = 1024 /* alignment slack */ + kGroups * kGroupBytes +
                                     4 * (kScaleBufs * (kKBlocks * NT + 128) + 4 * NT + 2 * NT) +
-                                    8 * (2 * kGroups + 2 * kPairs + 6) +
-                                    kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 24 + (MODE == 1 ? 256 : 8);
+                                    8 * (2 * kGroups + 2 * kPairs + 8) +
+                                    kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 32 + (MODE == 1 ? 256 : 8);
   static_assert(kSmemBytes <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
   static_assert(kKBlocks % kKps == 0 && kSlots % kTKps == 0 && kKps % kTKps == 0,
                 "steps must tile the K blocks and the slots");
@@ -316,11 +316,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   uint64_t* tempty = tfull + PAIRS;
   uint64_t* sfull = tempty + PAIRS;       // [3] mode 2: a scale buffer has landed
   uint64_t* sempty = sfull + 3;           // [3] mode 2: the epilogue is done with a scale buffer
-  ExpertWork* s_work = reinterpret_cast<ExpertWork*>(sempty + 3);
+  uint64_t* idle = sempty + 3;            // [2] a CTA that gave up: an issuer's MMAs are over
+  ExpertWork* s_work = reinterpret_cast<ExpertWork*>(idle + 2);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_work + kMaxLocalExperts);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   int* s_meta = reinterpret_cast<int*>(s_tmem + 3);   // [2] token tiles, active experts (copied from p.meta)
-  uint8_t* s_pub = reinterpret_cast<uint8_t*>(s_tmem + 6);   // mode 1, [256] ring: does this CTA publish its i-th item?
+  int* s_armed = reinterpret_cast<int*>(s_tmem + 6);  // [2] ring entries and (mode 2) scale buffers the producer has asked for
+  uint8_t* s_pub = reinterpret_cast<uint8_t*>(s_tmem + 8);   // mode 1, [256] ring: does this CTA publish its i-th item?
   int* s_last = reinterpret_cast<int*>(s_tmem + 5);   // mode 1: this CTA finished the last part of a split item
   int* s_done = reinterpret_cast<int*>(s_tmem + 2);   // mode 1: epilogue warps that finished storing an item (running total); mode 2: items cleared for loading
 
@@ -342,6 +344,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     for (int i = 0; i < G; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < PAIRS; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 4 * C::kColSplit); }
     for (int i = 0; i < 3; ++i) { mbar_init(&sfull[i], 1); mbar_init(&sempty[i], 4 * C::kColSplit); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&idle[i], 1); s_armed[i] = 0; }
     *s_abort = 0;
     *s_done = 0;
     fence_barrier_init();
@@ -573,23 +576,25 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
               if (*s_abort != 0) { alive = false; break; }
               if (clock64() - t0 > p.wait_limit) { *s_abort = kStatusDependencyTimeout; alive = false; break; }
             }
-            if (!alive) break;
           }
           __threadfence_block();
           // scales of the item: [16 K blocks x NT rows] activation scales through a tensor map and the
           // 16 weight scales as a 64-byte bulk copy, into the buffer the epilogue released three items ago
           const uint32_t sb = n_items % 3u, sp = (n_items / 3u) & 1u;
-          if (!mbar_wait_bounded(&sempty[sb], sp ^ 1u, s_abort, kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
-          float* d_act = s_scales + sb * kScaleStride;
-          mbar_arrive_expect_tx(&sfull[sb], (KB * NT + KB) * 4);
-          tma_load_2d(d_act, &tm_sc, &sfull[sb], im.row_start, 0, pol_b);
-          bulk_load(d_act + KB * NT, p.w_scale + (static_cast<size_t>(im.expert) * kHBlocks + im.ft) * kIBlocks,
-                    KB * 4, &sfull[sb], pol_b);
-          ++n_items;
+          if (alive && !mbar_wait_bounded(&sempty[sb], sp ^ 1u, s_abort, kStatusWaitTimeoutProducer, p.wait_limit)) alive = false;
+          if (alive) {
+            float* d_act = s_scales + sb * kScaleStride;
+            mbar_arrive_expect_tx(&sfull[sb], (KB * NT + KB) * 4);
+            tma_load_2d(d_act, &tm_sc, &sfull[sb], im.row_start, 0, pol_b);
+            bulk_load(d_act + KB * NT, p.w_scale + (static_cast<size_t>(im.expert) * kHBlocks + im.ft) * kIBlocks,
+                      KB * 4, &sfull[sb], pol_b);
+            ++n_items;
+          }
         }
         pick([&](auto layout) {
-          for (int step = 0; step < ahead; ++step) load_b(layout, step, step);   // entry of a first fill = its step
-          for (int step = ahead; step < steps; ++step) {
+          // (entry of a first fill = its step; also when the expert's rows never came, because the entries are armed for both sides)
+          for (int step = 0; step < ahead; ++step) load_b(layout, step, step);
+          for (int step = ahead; step < steps && alive; ++step) {
             if (!mbar_wait_bounded(&empty[g], ph ^ 1u, s_abort, kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
             TRACE(0, step);
             load_w(layout, step);
@@ -601,10 +606,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           }
         });
       }
-      // drain: every ring entry this thread armed must have landed before the CTA may exit
-      const uint32_t first = it > static_cast<uint32_t>(G) ? it - G : 0;
-      for (uint32_t i = first; i < it; ++i)
-        mbar_wait_bounded(&full[i % G], (i / G) & 1, s_abort, kStatusWaitTimeoutProducer, 1ll << 28);
+      // (nothing to wait for here: the epilogue has used all that was asked for, or the CTA gives up, see the end of the kernel)
+      s_armed[0] = static_cast<int>(it);
+      s_armed[1] = static_cast<int>(n_items);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1007,6 +1011,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (EARLY && (MODE == 1 || s_meta[0] == 0)) pdl_wait();
   tc_fence_before();
   __syncthreads();
+  if (*s_abort != 0) {
+    // A role gave up: copies and MMAs may still be on their way, which otherwise the epilogue has waited for.
+    if (threadIdx.x == 0) {
+      for (int i = max(s_armed[0] - G, 0); i < s_armed[0]; ++i) mbar_wait_landed(&full[i % G], (i / G) & 1);
+      for (int i = max(s_armed[1] - 3, 0); i < s_armed[1]; ++i) mbar_wait_landed(&sfull[i % 3], (i / 3) & 1);
+    }
+    if (lane == 0 && (warp == 1 || (ISSUERS == 2 && warp == 3 + 4 * C::kColSplit))) {   // the threads that issued MMAs
+      umma_commit(&idle[warp == 1 ? 0 : 1]);
+      mbar_wait_landed(&idle[warp == 1 ? 0 : 1], 0);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

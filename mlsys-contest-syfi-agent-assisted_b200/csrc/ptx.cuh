@@ -76,6 +76,13 @@ __device__ __forceinline__ void mbar_wait_or_clear(bool& ok, uint64_t* bar, uint
   if (!mbar_try_wait(bar, parity) && ok) ok = mbar_wait_bounded(bar, parity, abort_flag, code, limit_cycles);
 }
 
+// Waits for copies or MMAs that are already on their way.  They need nobody's help, so no abort flag ends this wait, which is
+// for a CTA that gave up: its memory must not be handed to the next CTA with a write still coming.  Bounded all the same.
+__device__ __forceinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity) && clock64() - t0 < (1ll << 28)) {}
+}
+
 // Cross-CTA hand-off through a counter in global memory: the writers' data stores happen before the
 // release increment, the reader's acquire load happens before its dependent loads.  The proxy fence
 // orders generic-proxy accesses against async-proxy ones (TMA), which otherwise have no mutual order.

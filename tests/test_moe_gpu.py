@@ -868,6 +868,30 @@ def test_waits_that_run_out_at_once_leave_whole_warps(T, E, tile, pkg, monkeypat
         assert torch.equal(before, after), limit
 
 
+@pytest.mark.parametrize("T,E,tile", [(12, 5, None), (40, 3, None), (200, 8, None), (300, 4, 64), (300, 4, 128)])
+def test_calls_that_give_up_halfway_leave_nothing_on_its_way(T, E, tile, pkg, monkeypatch):
+    """Limits between the latency of one load and the length of the call: CTAs give up with copies and MMAs under way and
+    must see those land before they hand their shared and tensor memory on.  The call reports a status (a long limit may
+    pass), and the kernels behind it find everything as it should be."""
+    if tile is not None:
+        monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", str(tile))
+    inp = pkg.make_inputs(num_tokens=T, seed=45, e_local=E, device=DEV)
+    before, _ = _run(pkg, inp)
+    ctx = pkg.get_context(0)
+    failed = 0
+    for limit in (300, 1000, 2000, 4000, 8000, 16000, 40000):
+        ctx.debug_fault(0, limit)
+        pkg.run_moe(*inp.args(), torch.empty_like(before))
+        try:
+            ctx.check()
+        except pkg.MoeError as err:
+            assert any(f"status {c}" in str(err) for c in (101, 102, 103, 106)), str(err)
+            failed += 1
+        after, _ = _run(pkg, inp)
+        assert torch.equal(before, after), limit
+    assert failed >= 2, failed
+
+
 def test_row_capacity_overflow_is_reported_not_written(pkg):
     """The workspace holds 3 rows per token beyond 2048 tokens (a token sends about one of its 8 routes to 32 of
     256 experts).  Every local expert made hot sends far more: the row-list kernel refuses to write past the
