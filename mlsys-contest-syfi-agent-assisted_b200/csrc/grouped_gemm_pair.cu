@@ -45,7 +45,8 @@
 // Barriers another CTA signals: full[] lives in the first CTA and counts the bytes of both CTAs' loads;
 // empty[] and tfull[] exist in both CTAs and are signalled by one tcgen05.commit each; tempty[] lives
 // in the first CTA and collects the arrivals of both CTAs' epilogue warps.
-// Every wait is bounded; a CTA that gives up also raises the abort flag of its partner.
+// Every wait is bounded; a CTA that gives up also raises the abort flag of its partner, and the pair leaves together, with
+// nothing on its way into the memory of either (see the end of the kernel).
 #include <cuda_fp16.h>
 
 #include "moe_internal.h"
@@ -76,7 +77,7 @@ template <int MODE> struct PairCfg {
   // mode 1: the activation scales of a whole item, [56][128], in two buffers; mode 2: an item's scale products, [16][128], twice
   static constexpr int kScaleFloats = (MODE == 1 ? kHBlocks : 2 * kIBlocks) * kScaleEntry;
   static constexpr int kScaleBufs = 2;
-  static constexpr int kBarriers = kStages + kStages / 2 + 2 * kMaxSlots + 2 * kScaleBufs + 4;
+  static constexpr int kBarriers = kStages + kStages / 2 + 2 * kMaxSlots + 2 * kScaleBufs + 6;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleFloats * 4 +
                                     (MODE == 1 ? 2 * 4 * 128 * 4 + 2 * 128 * 4 : 0) + 8 * kBarriers +
                                     kMaxLocalExperts * static_cast<int>(sizeof(ExpertWork)) + 64;
@@ -179,11 +180,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   uint64_t* sempty = sfull + C::kScaleBufs;                                    // [2]   per CTA
   uint64_t* wfull = sempty + C::kScaleBufs;                                       // [2]   mode 1: an item's weight scales are there
   uint64_t* wempty = wfull + 2;                                                // [2]
-  ExpertWork* s_work = reinterpret_cast<ExpertWork*>(wempty + 2);
+  uint64_t* idle = wempty + 2;                                                 // [2]   a pair that gave up: an issuer's MMAs are over
+  ExpertWork* s_work = reinterpret_cast<ExpertWork*>(idle + 2);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_work + kMaxLocalExperts);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   int* s_done = reinterpret_cast<int*>(s_tmem + 2);   // mode 1: epilogue warps done with an item (running total); mode 2: items cleared
   int* s_meta = reinterpret_cast<int*>(s_tmem + 3);   // [2] token tiles, active experts
+  int* s_armed = reinterpret_cast<int*>(s_tmem + 5);  // [3] what the producer has asked for: stage pairs, (mode 1) buffers of activation scales and of weight scales
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -196,7 +199,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     for (int i = 0; i < G / 2; ++i) mbar_init(&empty[i], kIssuers);   // one commit per MMA issuer
     for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], (MODE == 1 ? 1 : 2) * kEpiWarps); }
     for (int i = 0; i < C::kScaleBufs; ++i) { mbar_init(&sfull[i], 1); mbar_init(&sempty[i], kEpiWarps); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&wfull[i], 1); mbar_init(&wempty[i], kEpiWarps); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&wfull[i], 1); mbar_init(&wempty[i], kEpiWarps); mbar_init(&idle[i], 1); }
+    for (int i = 0; i < 3; ++i) s_armed[i] = 0;
     *s_abort = 0;
     *s_done = 0;
     fence_barrier_init();
@@ -327,6 +331,57 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     ST_WRITE(4, true);
   };
 
+  // What this CTA loads of an item, and the loads of one stage pair (stages g and g + 1, K blocks kb and kb + 1).  Only the
+  // first CTA arms the barriers, for both CTAs' bytes.
+  struct Side {
+    const CUtensorMap* mb;
+    int my_row, wrow, boxes, box_pitch, box_rows;
+    uint32_t stage_tx;
+  };
+  auto side_of = [&](const PItem& im) {
+    Side sd;
+    int my_rows;
+    if (MODE == 1) {
+      // token tile on the M side: this CTA's rows 128 rank .. of the tile (none when the tile is short)
+      const int cnt0 = min(im.n, 128), cnt1 = im.n - cnt0;
+      my_rows = rank == 0 ? cnt0 : cnt1;
+      sd.my_row = im.row_start + 128 * static_cast<int>(rank);
+      sd.wrow = im.expert * 2 * kInter + static_cast<int>(rank) * kInter + im.ft * 128;
+      sd.mb = my_rows > 64 ? &tm_b0w : &tm_b0;
+      sd.stage_tx = static_cast<uint32_t>(2 * kTile + box_bytes(cnt0) + box_bytes(cnt1));
+    } else {
+      my_rows = im.n;                                      // all rows of one term
+      sd.my_row = im.row_start;
+      sd.wrow = im.expert * kHidden + (2 * im.ft + static_cast<int>(rank)) * 128;
+      sd.mb = my_rows > 64 ? &tm_b0w : rank == 0 ? &tm_b0 : &tm_b1;
+      if (my_rows > 64 && rank == 1) sd.my_row += p.row_cap;   // (tm_b0w has the lo term's rows behind the hi term's)
+      sd.stage_tx = 2u * static_cast<uint32_t>(kTile + box_bytes(im.n));
+    }
+    // more than 64 rows: one 128-row box (fewer TMA instructions); else 32-row boxes
+    sd.boxes = my_rows > 64 ? 1 : (my_rows + 31) >> 5;
+    sd.box_pitch = my_rows > 64 ? kTile : kBox;
+    sd.box_rows = my_rows > 64 ? 128 : 32;
+    return sd;
+  };
+  auto load_stage_pair = [&](const Side& sd, uint32_t g, int kb, uint32_t full0, uint64_t pol_w, uint64_t pol_b) {
+    constexpr int kTokOff = MODE == 1 ? 0 : kTile, kWOff = MODE == 1 ? kTile : 0;
+    if (rank == 0) {
+      mbar_arrive_expect_tx(&full[g], sd.stage_tx);
+      mbar_arrive_expect_tx(&full[g + 1], sd.stage_tx);
+    }
+    // boxes that continue each other along K are issued back to back (a row's 256 contiguous
+    // bytes are served by L2 far faster than two separate 128-byte visits)
+    uint8_t* st0 = smem + g * kStageBytes;
+    uint8_t* st1 = st0 + kStageBytes;
+    const int x0 = kb * 128;
+    tma_load_2d_pair(st0 + kWOff, &tm_w, full0 + 8u * g, x0, sd.wrow, pol_w);
+    tma_load_2d_pair(st1 + kWOff, &tm_w, full0 + 8u * g + 8u, x0 + 128, sd.wrow, pol_w);
+    for (int b = 0; b < sd.boxes; ++b) {
+      tma_load_2d_pair(st0 + kTokOff + b * sd.box_pitch, sd.mb, full0 + 8u * g, x0, sd.my_row + sd.box_rows * b, pol_b);
+      tma_load_2d_pair(st1 + kTokOff + b * sd.box_pitch, sd.mb, full0 + 8u * g + 8u, x0 + 128, sd.my_row + sd.box_rows * b, pol_b);
+    }
+  };
+
   if (warp < 4) {
     if (warp == 0) {
       // ------------------------------------------------------------ TMA producer (one thread per CTA)
@@ -336,7 +391,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         const uint32_t full0 = mapa_u32(smem_u32(&full[0]), 0);   // the first CTA's full[0]; the others follow at 8 bytes each
         uint32_t it = 0, g = 0, ph = 0;        // stage pairs armed, next stage, phase of its empty barrier
         uint32_t wp = 0;                       // phase bits of wempty[0..1] (mode 1)
-        uint32_t n_items = 0;
+        uint32_t n_items = 0, n_scales = 0, n_weight_scales = 0;
         int e_hint = 0;
         bool alive = true;
         ST_DECL;
@@ -344,30 +399,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         (void)st_start; (void)wp;
         for (int i = 0; i < my_items && alive; ++i) {
           const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
-          int my_rows, my_row, wrow, tok_off, w_off;
-          uint32_t stage_tx;
-          const CUtensorMap* mb;
-          if (MODE == 1) {
-            // token tile on the M side: this CTA's rows 128 rank .. of the tile (none when the tile is short)
-            const int cnt0 = min(im.n, 128), cnt1 = im.n - cnt0;
-            my_rows = rank == 0 ? cnt0 : cnt1;
-            my_row = im.row_start + 128 * static_cast<int>(rank);
-            wrow = im.expert * 2 * kInter + static_cast<int>(rank) * kInter + im.ft * 128;
-            mb = my_rows > 64 ? &tm_b0w : &tm_b0;
-            tok_off = 0;
-            w_off = kTile;
-            stage_tx = static_cast<uint32_t>(2 * kTile + box_bytes(cnt0) + box_bytes(cnt1));
-          } else {
-            my_rows = im.n;                                      // all rows of one term
-            my_row = im.row_start;
-            wrow = im.expert * kHidden + (2 * im.ft + static_cast<int>(rank)) * 128;
-            mb = my_rows > 64 ? &tm_b0w : rank == 0 ? &tm_b0 : &tm_b1;
-            if (my_rows > 64 && rank == 1) my_row += p.row_cap;   // (tm_b0w has the lo term's rows behind the hi term's)
-            tok_off = kTile;
-            w_off = 0;
-            stage_tx = 2u * static_cast<uint32_t>(kTile + box_bytes(im.n));
-          }
-          // more than 64 rows: one 128-row box (fewer TMA instructions); else 32-row boxes
+          const Side sd = side_of(im);
           if (MODE == 1) {
             // weight scales of the item, [0..55] up block and [64..119] gate block, into the buffer the
             // epilogue released two items ago
@@ -375,15 +407,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             if (!mbar_wait_bounded_tell(smem_u32(&wempty[par]), ((wp >> par) & 1u) ^ 1u, abort_flag, peer_abort,
                                         kStatusWaitTimeoutProducer, p.wait_limit)) { alive = false; break; }
             wp ^= 1u << par;
+            ++n_weight_scales;
             mbar_arrive_expect_tx(&wfull[par], 2u * kHBlocks * 4u);
             bulk_load(s_ws + par * 128, p.w_scale + (static_cast<size_t>(im.expert) * 32 + im.ft) * kHBlocks,
                       kHBlocks * 4, &wfull[par], pol_b);
             bulk_load(s_ws + par * 128 + 64, p.w_scale + (static_cast<size_t>(im.expert) * 32 + 16 + im.ft) * kHBlocks,
                       kHBlocks * 4, &wfull[par], pol_b);
           }
-          const int boxes = my_rows > 64 ? 1 : (my_rows + 31) >> 5;
-          const int box_pitch = my_rows > 64 ? kTile : kBox;
-          const int box_rows = my_rows > 64 ? 128 : 32;
           if (MODE == 2) {
             // the item's expert must have left GEMM1 (the helper warp checks and counts cleared items)
             if (*reinterpret_cast<volatile int*>(s_done) <= static_cast<int>(n_items)) {
@@ -407,6 +437,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           auto load_scales = [&](const PItem& of, int buf, int phase) {
             if (!mbar_wait_bounded_tell(smem_u32(&sempty[buf]), static_cast<uint32_t>(phase) ^ 1u, abort_flag, peer_abort,
                                         kStatusWaitTimeoutProducer, p.wait_limit)) return false;
+            ++n_scales;
             mbar_arrive_expect_tx(&sfull[buf], kScaleChunk * 128 * 4);
             tma_load_2d(s_scale + buf * kScaleChunk * 128, &tm_sc, &sfull[buf], of.row_start + 128 * static_cast<int>(rank),
                         buf * kScaleChunk, pol_b);
@@ -423,21 +454,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             if (!mbar_wait_bounded_tell(smem_u32(&empty[g >> 1]), ph ^ 1u, abort_flag, peer_abort, kStatusWaitTimeoutProducer,
                                         p.wait_limit)) { alive = false; break; }
             ST_END(0);
-            if (rank == 0) {
-              mbar_arrive_expect_tx(&full[g], stage_tx);
-              mbar_arrive_expect_tx(&full[g + 1], stage_tx);
-            }
-            // boxes that continue each other along K are issued back to back (a row's 256 contiguous
-            // bytes are served by L2 far faster than two separate 128-byte visits)
-            uint8_t* st0 = smem + g * kStageBytes;
-            uint8_t* st1 = st0 + kStageBytes;
-            const int x0 = kb * 128;
-            tma_load_2d_pair(st0 + w_off, &tm_w, full0 + 8u * g, x0, wrow, pol_w);
-            tma_load_2d_pair(st1 + w_off, &tm_w, full0 + 8u * g + 8u, x0 + 128, wrow, pol_w);
-            for (int b = 0; b < boxes; ++b) {
-              tma_load_2d_pair(st0 + tok_off + b * box_pitch, mb, full0 + 8u * g, x0, my_row + box_rows * b, pol_b);
-              tma_load_2d_pair(st1 + tok_off + b * box_pitch, mb, full0 + 8u * g + 8u, x0 + 128, my_row + box_rows * b, pol_b);
-            }
+            load_stage_pair(sd, g, kb, full0, pol_w, pol_b);
             ++it;
             g += 2;
             if (g == G) { g = 0; ph ^= 1u; }
@@ -447,14 +464,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         st_acc[1] = clock64() - st_start;
 #endif
         ST_WRITE(0, true);
-        // drain: the first CTA's full barriers count both CTAs' bytes, and no CTA of the pair leaves
-        // before the final cluster barrier, so waiting there covers the partner's loads as well
-        if (rank == 0) {
-          const uint32_t armed = 2 * it;
-          const uint32_t first = armed > static_cast<uint32_t>(G) ? armed - G : 0;
-          for (uint32_t i = first; i < armed; ++i)
-            mbar_wait_bounded_tell(smem_u32(&full[i % G]), (i / G) & 1, abort_flag, peer_abort, kStatusWaitTimeoutProducer, 1ll << 28);
-        }
+        // The epilogue waits for all that was loaded and multiplied, but nobody else for the last signals of empty[], which
+        // the first CTA's issuers send into both CTAs.
+        for (uint32_t k = it > G / 2 ? it - G / 2 : 0; k < it && alive; ++k)
+          alive = mbar_wait_bounded_tell(smem_u32(&empty[k % (G / 2)]), (k / (G / 2)) & 1, abort_flag, peer_abort, kStatusWaitTimeoutProducer,
+                                         p.wait_limit);
+        s_armed[0] = static_cast<int>(it);
+        s_armed[1] = static_cast<int>(n_scales);
+        s_armed[2] = static_cast<int>(n_weight_scales);
       }
       __syncwarp();
     } else if (warp == 1) {
@@ -780,6 +797,31 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
+  if (*s_abort != 0) {
+    // A role of the pair gave up (both CTAs know it: whoever gives up tells the partner before this barrier).  Copies and MMAs
+    // may still be on their way.  A stage pair's barriers count the bytes of both CTAs, and one producer may have come
+    // further: the other asks for the missing ones now, whose stages are free, because the first saw them released for both.
+    if (threadIdx.x == 0) {
+      const int mine = s_armed[0], theirs = static_cast<int>(ld_cluster_u32(mapa_u32(smem_u32(&s_armed[0]), peer)));
+      const uint32_t full0 = mapa_u32(smem_u32(&full[0]), 0);
+      const uint64_t pol = l2_policy_evict_normal();
+      int e_hint = 0;
+      for (int k = mine; k < theirs; ++k)
+        load_stage_pair(side_of(decode_pair_item<FI, NT>(s_work, p.e_local, item_of(k / (KB / 2)), e_hint)),
+                        2 * (k % (G / 2)), 2 * (k % (KB / 2)), full0, pol, pol);
+      const int pairs = max(mine, theirs);
+      if (rank == 0)
+        for (int k = 2 * max(pairs - G / 2, 0); k < 2 * pairs; ++k) mbar_wait_landed(&full[k % G], (k / G) & 1);
+      for (int k = max(s_armed[1] - 2, 0); k < s_armed[1]; ++k) mbar_wait_landed(&sfull[k & 1], (k >> 1) & 1);
+      for (int k = max(s_armed[2] - 2, 0); k < s_armed[2]; ++k) mbar_wait_landed(&wfull[k & 1], (k >> 1) & 1);
+    }
+    if (rank == 0 && lane == 0 && (warp == 1 || (kIssuers == 2 && warp == 2))) {   // the threads that issued MMAs
+      umma_commit_pair(&idle[warp - 1], 1);
+      mbar_wait_landed(&idle[warp - 1], 0);
+    }
+    __syncthreads();
+    cluster_sync_all();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kPairTmemCols);

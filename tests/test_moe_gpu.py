@@ -868,7 +868,7 @@ def test_waits_that_run_out_at_once_leave_whole_warps(T, E, tile, pkg, monkeypat
         assert torch.equal(before, after), limit
 
 
-@pytest.mark.parametrize("T,E,tile", [(12, 5, None), (40, 3, None), (200, 8, None), (300, 4, 64), (300, 4, 128)])
+@pytest.mark.parametrize("T,E,tile", [(12, 5, None), (40, 3, None), (200, 8, None), (300, 4, 64), (300, 4, 128), (700, 4, 256), (3000, 4, 256)])
 def test_calls_that_give_up_halfway_leave_nothing_on_its_way(T, E, tile, pkg, monkeypatch):
     """Limits between the latency of one load and the length of the call: CTAs give up with copies and MMAs under way and
     must see those land before they hand their shared and tensor memory on.  The call reports a status (a long limit may
