@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(kScoreThreads)
 dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const uint8_t* __restrict__ cache, const float* __restrict__ weights,
                  const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ block_table, int max_pages,
-                 float* __restrict__ scores, int max_ls, int tiles_per_cta, uint2* __restrict__ ranges, int* __restrict__ status) {
+                 float* __restrict__ scores, int max_ls, int tiles_per_cta, uint2* __restrict__ ranges, int* __restrict__ status,
+                 long long wait_limit) {
   const int b = blockIdx.y, t_begin = blockIdx.x * tiles_per_cta * kTokTile;
   pdl_wait();                                  // the selection of the call before reads the scores written here
   pdl_trigger();
@@ -73,7 +74,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* s_k = smem;                                     // [2 stages][128 tokens][128 B], 128-byte swizzle
   uint8_t* s_q = smem + kScoreStages * kTokTile * kDim;    // [64 heads][128 B]
-  __shared__ uint64_t full[kScoreStages], empty[kScoreStages], tfull[kScoreStages], tempty[kScoreStages], qfull;
+  __shared__ uint64_t full[kScoreStages], empty[kScoreStages], tfull[kScoreStages], tempty[kScoreStages], qfull, idle;
   __shared__ uint32_t s_tmem;
   __shared__ float s_w[kHeads];
   __shared__ int s_page[2 * kMaxTilesPerCta];
@@ -92,6 +93,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_init(&tempty[i], 4);                // one arrival per epilogue warp
     }
     mbar_init(&qfull, 1);
+    mbar_init(&idle, 1);
     s_abort = 0;
     fence_barrier_init();
   }
@@ -104,6 +106,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = s_tmem;
 
+  int loaded = 0;                              // key tiles that the producer has asked for
   if (warp == 4) {
     if (lane == 0) {
       // ---------------------------------------------------------- producer and MMA issuer (one thread)
@@ -114,19 +117,20 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         mbar_arrive_expect_tx(&full[st], pages * kPage * kDim);
         for (int p = 0; p < pages; ++p)
           tma_load_2d(s_k + st * kTokTile * kDim + p * kPage * kDim, &tm_k, &full[st], 0, s_page[2 * i + p] * kPageRows, pol);
+        loaded = i + 1;
       };
       mbar_arrive_expect_tx(&qfull, kHeads * kDim);
       tma_load_2d(s_q, &tm_q, &qfull, 0, b * kHeads, l2_policy_evict_last());
       load_tile(0);
       if (tiles > 1) load_tile(1);
-      bool alive = mbar_wait_bounded(&qfull, 0, &s_abort, kStatusScoreTimeout, kWaitLimit);
+      bool alive = mbar_wait_bounded(&qfull, 0, &s_abort, kStatusScoreTimeout, wait_limit);
       const uint64_t b0 = umma_smem_desc_sw128(smem_u32(s_q));
       const uint32_t idesc = umma_idesc_e4m3_m128(kHeads);
       for (int i = 0; i < tiles && alive; ++i) {
         const int st = i % kScoreStages;
         const uint32_t ph = (i / kScoreStages) & 1u;
-        if (!mbar_wait_bounded(&full[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit)) break;
-        if (!mbar_wait_bounded(&tempty[st], ph ^ 1u, &s_abort, kStatusScoreTimeout, kWaitLimit)) break;
+        if (!mbar_wait_bounded(&full[st], ph, &s_abort, kStatusScoreTimeout, wait_limit)) break;
+        if (!mbar_wait_bounded(&tempty[st], ph ^ 1u, &s_abort, kStatusScoreTimeout, wait_limit)) break;
         tc_fence_after();
         const uint64_t a0 = umma_smem_desc_sw128(smem_u32(s_k + st * kTokTile * kDim));
 #pragma unroll
@@ -134,7 +138,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         umma_commit(&empty[st]);               // the key tile may be overwritten once these MMAs have read it
         umma_commit(&tfull[st]);
         if (i + kScoreStages < tiles) {
-          if (!mbar_wait_bounded(&empty[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit)) break;
+          if (!mbar_wait_bounded(&empty[st], ph, &s_abort, kStatusScoreTimeout, wait_limit)) break;
           load_tile(i + kScoreStages);
         }
       }
@@ -156,7 +160,7 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float scale = valid ? __ldg(reinterpret_cast<const float*>(cache + static_cast<size_t>(page) * kPageBytes +
                                                                        kPage * kDim + (tl & (kPage - 1)) * 4))
                                 : 0.0f;
-      mbar_wait_or_clear(alive, &tfull[st], ph, &s_abort, kStatusScoreTimeout, kWaitLimit);   // (failed: the rest of the run has no scores)
+      mbar_wait_or_clear(alive, &tfull[st], ph, &s_abort, kStatusScoreTimeout, wait_limit);   // (failed: the rest of the run has no scores)
       tc_fence_after();
       float acc = 0.0f;
 #pragma unroll
@@ -190,6 +194,16 @@ dsa_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     uint2 r = s_range[0];
     for (int w = 1; w < 4; ++w) r = make_uint2(min(r.x, s_range[w].x), max(r.y, s_range[w].y));
     ranges[static_cast<size_t>(b) * gridDim.x + blockIdx.x] = r;
+  }
+  if (s_abort != 0) {
+    // A role gave up: copies and MMAs may still be on their way, which otherwise the epilogue has waited for.
+    if (tid == 4 * 32) {
+      mbar_wait_landed(&qfull, 0);
+      for (int i = max(loaded - kScoreStages, 0); i < loaded; ++i) mbar_wait_landed(&full[i % kScoreStages], (i / kScoreStages) & 1);
+      umma_commit(&idle);
+      mbar_wait_landed(&idle, 0);
+    }
+    __syncthreads();
   }
   if (warp == 4) {
     tc_fence_after();
@@ -670,6 +684,7 @@ struct Device {
   Scratch scratch[kMaxScratch];
   uint64_t calls = 0;
   int* status = nullptr;
+  long long next_wait_limit = 0;   // syfi_dsa_debug_wait_limit: applies to the next call, then clears itself
   bool checked = false;
   int num_sms = 0;
 };
@@ -798,6 +813,8 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
         !raise(dsa_select_kernel<16, false>, kSelectSmem) || !raise(dsa_select_kernel<0, true>, kSelectSmem))
       return fail(SYFI_DSA_ERR_CUDA, "cannot raise the shared-memory limit of the indexer's kernels");
   }
+  const long long wait_limit = d.next_wait_limit > 0 ? d.next_wait_limit : kWaitLimit;
+  d.next_wait_limit = 0;
   CUtensorMap tm_q, tm_k;
   if (!rows128_map(&tm_q, q_index_fp8, static_cast<uint64_t>(batch) * kHeads) ||
       !rows128_map(&tm_k, k_index_cache_fp8, static_cast<uint64_t>(num_pages) * kPageRows))
@@ -812,11 +829,22 @@ extern "C" int syfi_dsa_topk_indexer(const void* q_index_fp8, const void* k_inde
   uint2* ranges = reinterpret_cast<uint2*>(s->scores + n_scores);
   if (launch_dependent(dsa_score_kernel, dim3(runs, batch), dim3(kScoreThreads), kScoreSmem, st, tm_q, tm_k,
                        static_cast<const uint8_t*>(k_index_cache_fp8), weights, seq_lens, block_table, max_pages,
-                       s->scores, max_ls, per_cta, ranges, d.status) != cudaSuccess)
+                       s->scores, max_ls, per_cta, ranges, d.status, wait_limit) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "score kernel launch failed");
   if (launch_select(s->scores, ranges, runs, per_cta * kTokTile, max_ls, seq_lens, block_table, batch, max_pages,
                     topk_indices, d.num_sms, st) != cudaSuccess)
     return fail(SYFI_DSA_ERR_CUDA, "select kernel launch failed");
+  return SYFI_DSA_OK;
+}
+
+// Test hook for the bounded waits, no part of the interface: a wait of the next call's score kernel on the current device may
+// take this many SM clocks (0: the normal limit).
+extern "C" int syfi_dsa_debug_wait_limit(int64_t clocks) {
+  if (clocks < 0) return fail(SYFI_DSA_ERR_INVALID, "a wait limit must not be negative");
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(SYFI_DSA_ERR_CUDA, "no current CUDA device");
+  std::lock_guard<std::mutex> lock(g_mu);
+  g_devices[dev].next_wait_limit = clocks;
   return SYFI_DSA_OK;
 }
 

@@ -1,4 +1,5 @@
 """Parity of the DSA top-k indexer's CUDA path (through the C ABI) against its oracle.  Needs a B200."""
+import ctypes
 import os
 
 import pytest
@@ -259,3 +260,24 @@ def test_indexer_argument_validation(pkg):
         pkg.run_dsa_topk_indexer(q.cpu(), cache, w, sl, table, out)
     pkg.run_dsa_topk_indexer(q, cache, w, sl, table, out)
     pkg.dsa_check()
+
+
+@pytest.mark.parametrize("seq_lens", [[3000], [700, 5000, 30000], [65536] * 32])
+def test_indexer_calls_that_give_up_halfway_leave_nothing_on_its_way(seq_lens, pkg):
+    """Limits around the latency of a load: score CTAs give up with copies and MMAs under way (one, two or eight key tiles
+    per CTA) and must see them land before they leave.  The call reports status 201 (a look at a barrier may itself take
+    as long as one load, so all but the shortest limit may pass), and the calls behind it give what they gave before."""
+    from oracle import dsa_oracle
+    inputs = tuple(t.to(DEV) for t in dsa_oracle.make_inputs(seq_lens, seed=14))
+    before = _run(pkg, inputs)
+    lib = pkg.load_library()
+    failed = 0
+    for limit in (1, 1, 1, 100, 400, 1000, 3000):
+        assert lib.syfi_dsa_debug_wait_limit(ctypes.c_int64(limit)) == 0
+        try:
+            _run(pkg, inputs)
+        except pkg.MoeError as err:
+            assert "status 201" in str(err), str(err)
+            failed += 1
+        assert torch.equal(_run(pkg, inputs), before), limit
+    assert failed >= 1, failed
