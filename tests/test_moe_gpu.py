@@ -294,11 +294,16 @@ def test_rows_per_expert_at_the_edges_of_the_work_split(rows, pkg, oracle, monke
         assert torch.equal(outs[0], o)
 
 
-@pytest.mark.parametrize("rows", [(1300, 16, 400), (2100,), (256, 0, 137)])
-def test_pairs_with_several_items_in_turn_equal_the_64_row_kernels(rows, pkg, monkeypatch):
-    """A pair of CTAs that walks through many work items reuses its buffers of scales (two halves of GEMM1's K blocks, two
-    items of GEMM2) and its accumulator slots across items of different height; one item per pair, where nothing is reused,
-    with a second CTA that has few rows.  The sums are those of the single-CTA kernels, bit for bit, also unrounded."""
+@pytest.mark.parametrize("rows,least", [((2560, 1424, 700, 400, 256), 4), ((1300, 16, 400), 1), ((2100,), 1), ((256, 0, 137), 0)])
+def test_pairs_with_several_items_in_turn_equal_the_64_row_kernels(rows, least, pkg, monkeypatch):
+    """A pair of CTAs that walks through many work items reuses its buffers of scales (two halves of GEMM1's K blocks, weight
+    scales and amax exchange of every other item, two items of GEMM2) and its accumulator slots, across items of different
+    height: at least four of GEMM1's items per pair, where every buffer comes round twice; two for some pairs; at most one,
+    where nothing is reused, with a second CTA that has few rows.  The sums are those of the single-CTA kernels, bit for
+    bit, also unrounded."""
+    pad = [(n + 15) // 16 * 16 for n in rows]
+    items = 16 * sum((n - (n % 256 if n % 256 <= 128 else 0) + 255) // 256 for n in pad)      # GEMM1's, without remainders
+    assert items // (torch.cuda.get_device_properties(0).multi_processor_count // 2) >= least
     E, T = len(rows), max(rows) + 5
     inp = pkg.make_inputs(num_tokens=T, seed=23, e_local=E, device=DEV)
     g = torch.Generator(device=DEV).manual_seed(4)
@@ -316,6 +321,27 @@ def test_pairs_with_several_items_in_turn_equal_the_64_row_kernels(rows, pkg, mo
         assert tuple(pkg.get_context(0).debug_read("counts", torch.int32)[0][:E].tolist()) == rows
         outs.append(out)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("T,E,pairs", [(3583, 32, False), (3584, 32, True), (4778, 24, False), (4779, 24, True), (4999, 8, False),
+                                        (5000, 8, True), (5600, 16, True), (5000, 7, False), (6143, 7, False), (6144, 7, True)])
+def test_token_counts_around_the_lines_of_the_pairs(T, E, pairs, pkg, monkeypatch):
+    """No tile is forced: both sides of each line between 64-row tiles and CTA pairs.  The call's launches say which it took
+    (the pairs have one more, for GEMM1's remainders); the result is that of forced 64-row tiles, bit for bit.  Pre-packed
+    weights never take the pairs."""
+    inp = pkg.make_inputs(num_tokens=T, seed=T + E, e_local=E, device=DEV)
+    out, _ = _run(pkg, inp)
+    ctx = pkg.get_context(0)
+    assert ctx.launch_count() == (7 if pairs else 6)
+    packed = pkg.prepack_weights(inp.gemm1_weights, inp.gemm2_weights)
+    out_p = torch.full_like(out, float("nan"))
+    pkg.run_moe_prepacked(*inp.args()[:4], packed, inp.gemm1_weights_scale, inp.gemm2_weights_scale, 0, inp.routed_scaling_factor, out_p)
+    assert ctx.launch_count() == 6
+    ctx.check()
+    monkeypatch.setenv("SYFI_MOE_TOKEN_TILE", "64")
+    want, _ = _run(pkg, inp)
+    assert ctx.launch_count() == 6
+    assert torch.equal(out, want) and torch.equal(out_p, want)
 
 
 @pytest.mark.parametrize("T,E,off", [(1, 1, 255), (2, 32, 64), (15, 3, 32), (16, 32, 0), (17, 32, 0)])
@@ -627,13 +653,13 @@ def test_argument_validation(pkg):
     pkg.get_context(0).check()
 
 
-@pytest.mark.parametrize("T,E,seed", [(8, 2, 3), (77, 8, 4), (1500, 32, 5), (6200, 6, 9)])
+@pytest.mark.parametrize("T,E,seed", [(8, 2, 3), (77, 8, 4), (1500, 32, 5), (5000, 8, 6), (6200, 6, 9)])
 def test_token_dispatch_on_one_rank_equals_the_plain_layer(T, E, seed, pkg):
     """The token-dispatch entry point with a world of one rank: route, publish, pull the routed rows from
     the rank's own region, the layer from the row lists on, push and final sum.  Everything but the link is
     exercised, and the result must equal the plain layer bit for bit — over several steps on different
     tokens (alternating buffer sets) and interleaved with the all-gather layout on the same region.  The
-    largest case runs the CTA-pair kernels, whose GEMM2 epilogue then stores through the row targets."""
+    largest two run the CTA-pair kernels, whose GEMM2 epilogue then stores through the row targets."""
     nbytes = pkg.ep_region_bytes(1, T)
     region = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
     desc = pkg.EpDesc()
