@@ -334,7 +334,7 @@ int run_layer(syfi_moe_ctx* ctx, const void* logits, const void* bias, const voi
   if (!ctx->ws_maps) {
     if (pair) {
       MAP_TRY(make_map(&p1.tm_b0, ws.a_perm, ws.row_cap, kHidden, 32));
-      p1.tm_b1 = p1.tm_b0;
+      p1.tm_b1 = p1.tm_b0;       // (not read by GEMM1, as tm_sc by GEMM2: one signature for both)
       MAP_TRY(make_map(&p2.tm_b0, ws.c_hi, ws.row_cap, kInter, 32));
       MAP_TRY(make_map(&p2.tm_b1, ws.c_lo, ws.row_cap, kInter, 32));
       MAP_TRY(make_map(&p1.tm_b0w, ws.a_perm, ws.row_cap, kHidden, 128));

@@ -163,7 +163,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   constexpr int FI = C::kFeatItems;
   constexpr int NT = C::kTokTile;
   constexpr int SE = C::kScaleEntry;
-  constexpr int kSlots = C::kSlots;
   constexpr int kSlotCols = C::kSlotCols;
   constexpr int kIssuers = MODE == 1 ? 2 : 1;   // MMA-issuing threads
 
@@ -274,11 +273,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
       for (int j = 0; j < G / 2; ++j) {
         if (n == total) break;
+        ST_BEGIN();
         if (!mbar_wait_bounded_tell(smem_u32(&full[2 * j + par]), ph, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
+        ST_END(0);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const uint32_t slot = 2 * par + h;
+          ST_BEGIN();
           if (!mbar_wait_bounded_tell(smem_u32(&tempty[slot]), sph, abort_flag, peer_abort, kStatusWaitTimeoutMma, p.wait_limit)) return;
+          ST_END(1);
           tc_fence_after();
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)
@@ -291,6 +294,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       }
       ph ^= 1u;
     }
+#ifdef SYFI_PAIR_STATS
+    st_acc[2] = clock64() - st_start;
+#endif
     ST_WRITE(4, par == 0);
   };
 
@@ -594,14 +600,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t mapa_tempty = mapa_u32(smem_u32(&tempty[0]), 0);   // the first CTA's tempty[0]; the others follow at 8 bytes each
     const int half = grp >> 1;                    // mode 1: which half of the features
-    uint32_t sl = 0, sph = 0;                     // accumulator slot (mode 1: of this half) and its phase
+    uint32_t sl = 0, sph = 0;                     // mode 1: accumulator slot of this half; phase of the slots
     uint32_t wp = 0;                              // phase bits of wfull[0..1] (mode 1)
     bool ok = true;
     int e_hint = 0;
     const uint64_t inv_ratio = f32x2_pack(1.0f / kLoRatio, 1.0f / kLoRatio);
     ST_DECL;
     const long long st_start = clock64();
-    (void)st_start; (void)inv_ratio; (void)wp;
+    (void)st_start; (void)inv_ratio; (void)wp; (void)sl;
 
     for (int i = 0; i < my_items; ++i) {
       const PItem im = decode_pair_item<FI, NT>(s_work, p.e_local, item_of(i), e_hint);
@@ -727,21 +733,21 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         const float* sc = s_scale + (i & 1) * KB * SE + c0;
         if (ok) for (int kb2 = 0; kb2 < KB; kb2 += 2, sph ^= 1u, sc += 2 * SE) {
 #pragma unroll
-          for (int sl = 0; sl < 2; ++sl) {
+          for (int slot = 0; slot < 2; ++slot) {
             ST_BEGIN();
-            mbar_wait_or_clear_tell(ok, smem_u32(&tfull[sl]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
+            mbar_wait_or_clear_tell(ok, smem_u32(&tfull[slot]), sph, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
             ST_END(0);
             tc_fence_after();
 #ifdef SYFI_PAIR_STATS
             const long long st_p0 = clock64();
 #endif
-            const uint32_t t0 = lane_addr + sl * kSlotCols + c0;
+            const uint32_t t0 = lane_addr + slot * kSlotCols + c0;
             // (handing the slot back before the arithmetic of the last chunk, as mode 1 does, costs registers
             // here and was slower: 400 us against 359 us)
 #pragma unroll
             for (int ch = 0; ch < CN / 16; ++ch) {
               if (c0 + ch * 16 < n) {
-                const ulonglong2* sp4 = reinterpret_cast<const ulonglong2*>(sc + sl * SE + ch * 16);
+                const ulonglong2* sp4 = reinterpret_cast<const ulonglong2*>(sc + slot * SE + ch * 16);
                 uint32_t r[16], l[16];
                 tmem_ld16(t0 + ch * 16, r);                 // hi products
                 tmem_ld16(t0 + im.n + ch * 16, l);          // lo products of the same token columns
@@ -758,7 +764,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(mapa_tempty + 8u * sl);
+            if (lane == 0) mbar_arrive_cluster_relaxed(mapa_tempty + 8u * slot);
 #ifdef SYFI_PAIR_STATS
             st_acc[2] += clock64() - st_p0;
 #endif
