@@ -234,11 +234,17 @@ const void* mapped_alias(const void* host) {
 // 529 / 473, 339 / 347, 443 / 414, 240 / 262; 3600 tokens 528 / 495, 345 / 363, 453 / 420, 267 / 265; 4000 tokens 554 / 533,
 // 382 / 381, 494 / 464, 278 / 268; 5000 tokens 655 / 597, 523 / 456, 631 / 595, 512 / 437: below the line one load gains
 // what another loses.
-// With fewer experts there are fewer tiles, and pairs pay off later.  64-row tiles / pairs, us per call, four loads: 16 experts,
-// 4000 tokens 255 / 241, 363 / 317, 240 / 258, 174 / 182; 5000 tokens 365 / 318, 631 / 530, 292 / 276, 425 / 348; 8 experts, 4500
-// tokens 192 / 174, 203 / 185, 157 / 164, 87 / 96; 5000 tokens 241 / 202, 476 / 412, 178 / 175, 261 / 242; 5600 tokens 261 / 235,
-// 537 / 439, 191 / 195, 301 / 258; 4 experts, 5000 tokens 179 / 157, 448 / 351, 107 / 112, 248 / 195; 1 expert 147 / 127, 79 / 85,
-// 70 / 77, 36 / 42 (one kernel more, and few rows to gain on).
+// With fewer experts there are fewer tiles, and pairs pay off later.  64-row tiles / pairs, us per call, six loads with the rows
+// that they route here (the second and fourth with hot experts; one side's runs differ by 5 to 8 %): 16 experts, 5000 tokens
+// 2843 rows 385 / 338, 5322 620 / 514, 1739 281 / 265, 3360 426 / 351, 2952 391 / 353, 1987 319 / 278; 12 experts, 5000 tokens
+// 2007 rows 272 / 257, 4959 544 / 454, 1449 232 / 241, 2518 312 / 268, 2589 361 / 313, 1714 260 / 237; 8 experts, 5000 tokens
+// 1601 rows 239 / 199, 4403 454 / 367, 829 163 / 165, 2220 251 / 233, 2493 314 / 264, 965 163 / 165; 5600 tokens 1810 rows 251 / 222,
+// 4940 530 / 443, 914 176 / 178, 2459 286 / 242, 2793 362 / 308, 1097 196 / 174; 6000 tokens all six gain.  What the lightest of the
+// loads of 8 and 12 experts lose here, 1 to 4 %, is a matter of their rows (about 110 an expert fill two 64-row tiles), which
+// the host does not know; at 4500 tokens it is 4 to 10 % (157 / 164, 87 / 96), against gains of 9 %.
+// With fewer than 8 experts the light loads lose more, one kernel more for few rows, and still do from 6144 tokens on: 4 experts
+// 1347 rows 202 / 181, 5324 551 / 454, 341 113 / 115, 215 100 / 100; 2 experts 1285 rows 190 / 168, 387 103 / 108, 183 94 / 95, 113 90 / 95, 57 80 /
+// 86; 1 expert 1283 rows 184 / 168, 109 84 / 89, 44 79 / 84, 4 75 / 81, 0 42 / 47.
 constexpr int64_t kPairMinTokens = 3584;
 constexpr int64_t kPairMinTokens8Experts = 5000;
 constexpr int64_t kPairMinTokensAnyExperts = 6144;

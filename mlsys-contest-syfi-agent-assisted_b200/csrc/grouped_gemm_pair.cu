@@ -5,15 +5,16 @@
 // of the reference, moe/solution/cuda/moe.cu:2194-2350, 1461-1627, 1631-1714; GEMM2 replaces
 // gemm_fp8_fp8_fused_acc_grouped_kernel, moe.cu:1718-1887), with a work split made for experts that own
 // hundreds of rows: the kernel is launched as clusters of two CTAs and every MMA spans the pair
-// (M = 256, N = 256), so one instruction issue feeds both tensor cores for 128 cycles and a K block
-// costs each CTA 32 KB of operand traffic per 4.2 M MACs (the single-CTA kernel with 64-row token tiles
-// moves 40 KB per 2.1 M MACs and is bound by the L2-to-SM rate).  Each CTA loads only its own operand
+// (M = 256; a K block is two groups of N = 128 in mode 1, one of N = 256 in mode 2), so one instruction issue feeds both
+// tensor cores and a K block costs each CTA 32 KB of operand traffic per 4.2 M MACs (the single-CTA kernel with 64-row
+// token tiles moves 40 KB per 2.1 M MACs and is bound by the L2-to-SM rate).  Each CTA loads only its own operand
 // halves; nothing is multicast.
 //
 //   mode 1 (GEMM1), work item = (expert, 128 intermediate features, up to 256 token rows), TOKEN-MAJOR:
 //     the token rows are the M operand (CTA r holds rows 128 r .. 128 r + 127 of the tile), the weights
 //     the N operand (CTA 0 loads the 128 up rows of W13, CTA 1 the 128 gate rows of the same features).
-//     A tensor-memory lane is a token, columns 0..127 are its up values and 128..255 its gate values:
+//     A tensor-memory lane is a token; each of the two accumulators of a K block has the token's up values of 64 features in
+//     its columns 0..63 and the gate values of the same features in 64..127:
 //     the block scale of a lane is ONE number per K block (activation scale of the token x weight scale),
 //     SwiGLU needs no exchange, and the row's amax over the 128 features is a reduction inside four
 //     threads.  (With features on the lanes, as in grouped_gemm.cu, every thread needs the scale of each
@@ -29,11 +30,13 @@
 // in two slots of 256 columns, mode 1 in four of 128, one per half of the features (up and gate), so that a half is
 // promoted while the other's MMAs still run.
 //
-// What bounds mode 1 (clocks per K block at 8192 tokens, parts switched off): MMAs alone 531, with the loads 642, with
-// the hand-off of the slots 757, complete 879, of which the epilogue (SwiGLU, requantisation, stores) about 80.  The
-// promotion warps use two thirds of the issue slots (160 instructions per warp and K block when it took 990, 64 of them
-// the FMAs), so fewer instructions there is what counts: 32-bit barrier addresses, scales that arrive by TMA instead of
-// through the epilogue's registers, eight columns per tcgen05.ld (sixteen make the compiler keep values in local memory).
+// What bounds mode 1 (clocks per K block at 8192 tokens, in builds that left parts of the kernel out): MMAs alone 531, with the
+// loads 642, with the hand-off of the slots 757, complete 879, of which the epilogue (SwiGLU, requantisation, stores) about
+// 80.  The promotion warps use two thirds of the issue slots (160 instructions per warp and K block, 64 of them the FMAs, in
+// the kernel before, whose 256-column slots and scales through registers took 990), so fewer instructions there is what
+// counts: 32-bit barrier addresses, scales that arrive by TMA instead of through the epilogue's registers, eight columns per
+// tcgen05.ld (with sixteen the compiler kept 30 values in local memory, with eight none).  These came as one step, 2 to 3 %
+// per call (4096 tokens 509.5 / 496.2 and 577 / 565 us); each one's share was not measured.
 //
 // Roles per CTA: warp 0 = TMA producer (one thread; mode 1: the activation and weight scales too), warp 1 = tensor memory
 // owner and, in the pair's first CTA, MMA issuer (mode 1: of the even K blocks), warp 2 = issuer of the odd K blocks
@@ -257,8 +260,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   // stage pair: empty[] counts two arrivals.)  Two groups of N = 128 take the tensor core as long as one of N = 256 (528 and
   // 531 clocks per K block, MMAs alone), and a half's eight promotion warps start while the other half's MMAs run.  An
   // issuer has no more instructions between a slot's release and the next MMAs than it must: it shares its scheduler with
-  // four promotion warps.  Clocks per K block of the whole kernel at 8192 tokens, slots of 256 / of 128 columns with an
-  // issuer per half / per parity: 950 / 985 / 940.
+  // four promotion warps.  Clocks per K block of the whole kernel at 8192 tokens (one build, whose scales still went through
+  // registers), slots of 256 / of 128 columns with an issuer per half / per parity: 950 / 985 / 940.
   auto mma_halves = [&](const uint32_t par) {
     const uint32_t sb = smem_u32(smem) + par * kStageBytes;
     const uint64_t a0 = umma_smem_desc_sw128(sb), b0 = umma_smem_desc_sw128(sb + kTile);
@@ -639,7 +642,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             const long long st_p0 = clock64();
 #endif
             const uint32_t t0 = lane_addr + (2 * sl + half) * kSlotCols + (grp & 1) * 32;
-            // eight columns at a time: with sixteen the compiler keeps 30 values in local memory
+            // eight columns at a time: with sixteen the compiler kept 30 values in local memory
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
               uint32_t r[8];
@@ -726,7 +729,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         for (int j = 0; j < CN / 2; ++j) acc[j] = 0ull;
         // One wait for the scales per item, and two K blocks per trip with their slots as constants: with a ring of scales per
         // K block and a running slot the promotion, which bounds this mode, had two waits and more address arithmetic per K
-        // block (us per call 4096 tokens 512 / 501 and 586 / 573, 8192 tokens 864 / 843, 16384 with hot experts 2886 / 2842).
+        // block (us per call 4096 tokens 512 / 503 and 586 / 575, 8192 tokens 864 / 843, 16384 with hot experts 2886 / 2842).
         mbar_wait_or_clear_tell(ok, smem_u32(&sfull[i & 1]), (i >> 1) & 1, abort_flag, peer_abort, kStatusWaitTimeoutEpilogue, p.wait_limit);
         ok = __all_sync(0xffffffffu, ok);
         const int n = ok ? im.n : 0;

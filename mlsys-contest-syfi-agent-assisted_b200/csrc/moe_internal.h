@@ -111,11 +111,13 @@ struct GemmLaunch {
 // How a call with CTA pairs splits an expert's padded rows between GEMM1's two kernels: the pair kernel takes tiles of
 // 256 rows, and a remainder of more than kTailRows; a smaller remainder goes to the single-CTA kernel (kTailTile-row
 // tiles), because in the pair kernel the rows are the M operand, whose height is fixed, and in the other one the N
-// operand, which is as wide as there are rows.  A K block of a tile takes a pair about 2500 SM clocks however few rows
-// there are, the single-CTA kernel about 950 per 64 rows: the line lies between two and three of its tiles.  Measured, us
-// per call, pairs alone / lines at 64, 128 and 192 rows: 4096 tokens 566 / 540, 537, 532 and 496 / 450, 442, 453 (another
-// seed); 8192 tokens 916 / 874, 885, 883 and 852 / 823, 830, 848; 16384 tokens 908 / 879, 863, 863.  The remainders come
-// second: in front of the pairs they cost 1 to 3 % more, as the pairs' long last round then ends the GEMM.
+// operand, which is as wide as there are rows.  A K block of a tile takes a pair's two SMs about 880 clocks however few rows
+// there are, the single-CTA kernel's one SM about 950 per 64 rows: by that the line would lie near two of its tiles.
+// Measured, us per call, lines at 64 / 128 / 192 rows, three expert loads each (the second with hot experts): 4096 tokens
+// 501 / 493 / 496, 572 / 562 / 590, 427 / 426 / 433; 8192 tokens 834 / 837 / 840, 1382 / 1345 / 1423, 707 / 719 / 718; 16384 tokens
+// 1586 / 1518 / 1564, 2775 / 2814 / 2816, 1192 / 1184 / 1186 (the runs of one build differ by 0.2 % at 4096 and up to 5 % at the larger
+// sizes).  All rows on the pairs were slower at each of these sizes, by 3 to 11 %, on the kernels before these.  The
+// remainders come second: in front of the pairs they cost 1 to 3 % more, as the pairs' long last round then ends the GEMM.
 constexpr int kPairTile = 256;
 constexpr int kTailRows = 128;
 constexpr int kTailTile = 64;
